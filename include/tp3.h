@@ -114,7 +114,9 @@ int tp3_get_mode(const tp3_ctx* ctx, int* mode);
  * coupling, warps owning folded pairs of k1 rows, at 8, 7 and 13 warps per CTA with the
  * largest per-warp D buffer that fits 225 KB; 8: the same at 14 warps in pairs, the two
  * warps of a pair sharing one unit and one D buffer (7 buffers); in BF16 mode it writes
- * T order-major and the angular kernel reads it MN-major) -- selects
+ * T order-major and the angular kernel reads it MN-major; 9: lane-owned coupling, each lane
+ * holding one shell pair's D and T in registers, the default where its staged coefficients
+ * and 3j values fit an SM's shared memory; it gives the bits of form 0) -- selects
  * the fastest for this context and records it for the shape (L, LMAX, N, K, lambda,
  * dq) in the process, where TP3_MODE_AUTO finds it.  Every variant is timed with the
  * persistent angular schedule; the fastest tensor-core variant is then timed again
@@ -122,7 +124,7 @@ int tp3_get_mode(const tp3_ctx* ctx, int* mode);
  * up to *nreport rows of four values (mode, coupling form, angular schedule, ms per
  * proposal); *nreport returns the number of rows.  Synchronises. */
 int tp3_autotune(tp3_ctx* ctx, int n, double* report, int* nreport);
-/* Force a coupling form of the tensor-core path (0 to 8 as above). */
+/* Force a coupling form of the tensor-core path (0 to 9 as above). */
 int tp3_set_coupling(tp3_ctx* ctx, int form);
 /* Angular-stage schedule of the tensor-core path (no reference counterpart).
  * TP3_ANGULAR_PERSISTENT (default): one CTA per SM walks (proposal, 128-triple tile,

@@ -1,0 +1,88 @@
+"""The lane-owned coupling against the one-kernel pair coupling: both add every triple product
+in the same order, so T, c3 and the energies are equal bit for bit, at shapes on either side
+of the lane form's tiles: 32 shell pairs a unit, blocks of 8 and 16 shells k3, three orders a
+task, 32 shells a coefficient row, quads of four m3, real-function and general coefficients."""
+import numpy as np
+import pytest
+
+import tp3
+
+pytestmark = pytest.mark.gpu
+
+LANE, PAIR = 9, 0
+
+
+def _coefficients(L, LMAX, K, n, real, seed):
+    """n coefficient sets; c[l,-m] = (-1)^m conj c[l,m] when real."""
+    from tp3.structure import seanindex0
+    rng = np.random.default_rng(seed)
+    c = np.zeros((n, K, LMAX * LMAX), dtype=np.complex128)
+    for l in range(L + 1):
+        for m in range(l + 1):
+            v = (rng.normal(size=(n, K)) + 1j * rng.normal(size=(n, K)) * (m > 0)) / (1.0 + l)
+            c[:, :, seanindex0(l, m, LMAX)] = v
+            if m:
+                c[:, :, seanindex0(l, -m, LMAX)] = (-1) ** m * np.conj(v)
+    c[:, :, seanindex0(0, 0, LMAX)] += 4.0
+    if not real:
+        c += 0.1 * (rng.normal(size=c.shape) + 1j * rng.normal(size=c.shape))
+    return c
+
+
+@pytest.mark.parametrize("L,LMAX,N,K", [(0, 1, 2, 1), (2, 3, 4, 7), (4, 6, 6, 8), (6, 7, 8, 9), (10, 11, 8, 16),
+                                        (8, 9, 8, 17), (12, 13, 10, 32), (6, 8, 6, 33), (4, 5, 4, 64), (18, 20, 8, 5),
+                                        (30, 31, 4, 3)])
+@pytest.mark.parametrize("real", [True, False])
+def test_lane_form_equals_pair_form(L, LMAX, N, K, real):
+    b = tp3.calculate_basis(L, LMAX, N, K)
+    rng = np.random.default_rng(K)
+    b.set_histogram(rng.uniform(0.5, 1.5, size=(N, 2 * N, K, K, K)))
+    c = _coefficients(L, LMAX, K, 3, real, 10 * L + K)
+    got = {}
+    for form in (PAIR, LANE):
+        b.set_mode(tp3.TP3_MODE_TC_BF16X3)
+        b.set_coupling(form)
+        T, c3, E = b.triple_products(c[0]), b.c3_raw(c[0]), b.energy_batch(c)
+        b.set_mode(tp3.TP3_MODE_TC_TF32X3)
+        got[form] = (T, c3, E, b.triple_products(c[1]), b.c3_raw(c[1]), b.energy_batch(c))
+    for x, y in zip(got[PAIR], got[LANE]):
+        assert np.isfinite(x).all() and np.array_equal(x, y)
+    b.close()
+
+
+def test_lane_form_mixed_and_ragged_batches():
+    """One batch with real-function and general proposals; ragged limits with absent orders and
+    shells: energies equal the pair form's."""
+    import torch
+    L, LMAX, N, K = 14, 15, 12, 21
+    b = tp3.calculate_basis(L, LMAX, N, K)
+    rng = np.random.default_rng(3)
+    Ks = [K, 13, 16, 17]
+    hists = [rng.uniform(0.5, 1.5, size=(N, 2 * N, k, k, k)) for k in Ks]
+    b.set_histogram(hists[0])
+    b.set_histograms(hists, Ks)
+    c = _coefficients(L, LMAX, K, 6, True, 5)
+    c[1::2] = _coefficients(L, LMAX, K, 3, False, 6)
+    lkh = np.array([(14, 21, 0), (6, 13, 1), (12, 16, 2), (0, 1, 3), (8, 17, 3), (2, 9, 1)], dtype=np.int32)
+    d_c = torch.from_numpy(c.view(np.float64).copy()).cuda()
+    d_l = torch.from_numpy(lkh).cuda()
+    got = {}
+    for form in (PAIR, LANE):
+        b.set_coupling(form)
+        E, R = (torch.empty(6, dtype=torch.float64, device="cuda") for _ in range(2))
+        b.energy_batch_device(6, d_c.data_ptr(), E.data_ptr())
+        b.energy_batch_ragged_device(6, d_c.data_ptr(), d_l.data_ptr(), R.data_ptr())
+        b.sync()
+        got[form] = (E.cpu().numpy(), R.cpu().numpy())
+    for x, y in zip(got[PAIR], got[LANE]):
+        assert np.isfinite(x).all() and np.array_equal(x, y)
+    b.close()
+
+
+def test_lane_form_is_the_default():
+    b = tp3.calculate_basis(8, 9, 8, 8)
+    c = _coefficients(8, 9, 8, 1, True, 1)[0]
+    T = b.triple_products(c)
+    b.set_coupling(LANE)
+    assert np.array_equal(T, b.triple_products(c))
+    b.close()

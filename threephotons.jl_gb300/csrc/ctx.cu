@@ -74,7 +74,7 @@ cudaError_t upload(tp3_ctx* c, const std::vector<T>& h, const T** out) {
 }
 
 // ---- tensor-core path tables -------------------------------------------------
-std::string build_tc_tables(const Basis& b, std::vector<PairBlock>& pbs, std::vector<int>& eofs,
+std::string build_tc_tables(const Basis& b, const tp3::Wigner3jTable& w3j, std::vector<PairBlock>& pbs, std::vector<int>& eofs,
                             std::vector<float>& wtab, int& maxs, int& SDmax) {
   std::map<std::tuple<int, int, int>, int> ltidx;
   for (int t = 0; t < b.n_lt(); ++t) ltidx[{b.lt_l1[t], b.lt_l2[t], b.lt_l3[t]}] = t;
@@ -108,7 +108,7 @@ std::string build_tc_tables(const Basis& b, std::vector<PairBlock>& pbs, std::ve
           const int m2 = -m3 - m1;
           for (int s = 0; s < pb.nl3p; ++s) {
             const int l3 = l3min + 2 * s;
-            it.w.push_back(s < pb.nl3 && std::abs(m3) <= l3 ? (float)tp3::wigner3j(l1, l2, l3, m1, m2, m3) : 0.f);
+            it.w.push_back(s < pb.nl3 && std::abs(m3) <= l3 ? (float)w3j(l1, l2, l3, m1, m2, m3) : 0.f);
           }
           run += pb.nl3p;
         }
@@ -175,7 +175,9 @@ std::string setup_tc(tp3_ctx* c) {
   std::vector<int> eofs;
   std::vector<float> wtab;
   int maxs = 0, SDmax = 0;
-  std::string m = build_tc_tables(b, pbs, eofs, wtab, maxs, SDmax);
+  if (b.L > 30) return "more than 16 l3 values per pair block (L > 30)";
+  const tp3::Wigner3jTable w3j(b);
+  std::string m = build_tc_tables(b, w3j, pbs, eofs, wtab, maxs, SDmax);
   if (!m.empty()) return m;
   if (maxs > 16) return "more than 16 l3 values per pair block (L > 30)";
   for (const auto& pb : pbs)
@@ -417,14 +419,14 @@ std::string setup_tc(tp3_ctx* c) {
       std::vector<float> fw;
       std::vector<int2> fch;
       int wmx = 0, cmx = 0;
-      if (!tp3::build_fold_tables(pbs, rows_gen, fbl, frows, fw, fch, wmx, cmx).empty()) continue;
+      if (!tp3::build_fold_tables(pbs, w3j, rows_gen, fbl, frows, fw, fch, wmx, cmx).empty()) continue;
       const int stage = (1 + b.K * (b.K + 1) / 2 + 3) / 4 * 4;
       const int ngroups = fvs[v].nw / fvs[v].grp;
       const size_t fixed = tp3::fold_smem_bytes(ngroups, ps, 0, wmx, cmx, stage);
       const size_t per_row = (size_t)(1 + ngroups) * ps * sizeof(float2);
       if (fixed + per_row > fvs[v].budget) continue;
       const int drows = (int)std::min<size_t>((size_t)rows_gen, (fvs[v].budget - fixed) / per_row);
-      if (!tp3::build_fold_tables(pbs, drows, fbl, frows, fw, fch, wmx, cmx).empty()) continue;
+      if (!tp3::build_fold_tables(pbs, w3j, drows, fbl, frows, fw, fch, wmx, cmx).empty()) continue;
       if ((e = upload(c, fbl, &fv.blks)) != cudaSuccess || (e = upload(c, frows, &fv.rows)) != cudaSuccess ||
           (e = upload(c, fw, &fv.w)) != cudaSuccess || (e = upload(c, fch, &fv.chunks)) != cudaSuccess)
         return std::string("fold coupling tables: ") + cudaGetErrorString(e);
@@ -441,6 +443,30 @@ std::string setup_tc(tp3_ctx* c) {
       fv.ok = fv.smem <= fvs[v].budget;
     }
   }
+  // lane-owned coupling: the default form where its staged rows fit
+  {
+    tp3::LaneTables& ln = tc.lane;
+    std::vector<tp3::LaneBlock> lbl;
+    std::vector<tp3::LaneQuad> lq;
+    std::vector<int4> lg;
+    std::vector<float4> lw;
+    if (b.K <= 64 && tp3::build_lane_tables(pbs, b.coff, w3j, lbl, lq, lg, lw, ln.crows, ln.wmax, ln.c3rows).empty()) {
+      ln.ps = b.K <= 32 ? 32 : 64;
+      ln.c3row = ln.ps / 2;
+      std::vector<uint32_t> ut, sl;
+      std::vector<int2> ko;
+      tp3::build_lane_units(b.K, ut, sl, ko, ln.stage);
+      tp3::lane_pick_warps(ln);
+      if (ln.ok) ln.maxz = std::max(1, tp3::lane_tasks(ko[b.K].y, maxs) / ln.nw);
+      if (ln.ok && ((e = upload(c, lbl, &ln.blks)) != cudaSuccess || (e = upload(c, lq, &ln.quads)) != cudaSuccess ||
+                    (e = upload(c, lg, &ln.gcols)) != cudaSuccess || (e = upload(c, lw, &ln.w)) != cudaSuccess ||
+                    (e = upload(c, ut, &ln.utab)) != cudaSuccess || (e = upload(c, sl, &ln.slots)) != cudaSuccess ||
+                    (e = upload(c, ko, &ln.kofs)) != cudaSuccess ||
+                    (e = tp3::lane_configure()) != cudaSuccess))
+        return std::string("lane coupling: ") + cudaGetErrorString(e);
+    }
+    tc.use_lane = ln.ok;
+  }
   // the split coupling is kept for the autotuner and for shapes the fused kernel cannot hold
   tc.split_ok = tp3::couple_split_smem_d(t, tc) <= (size_t)tp3::kCoupleMaxDynSmem &&
              tp3::couple_split_smem_t(t, tc) <= (size_t)tp3::kCoupleMaxDynSmem &&
@@ -453,7 +479,7 @@ std::string setup_tc(tp3_ctx* c) {
     return "tensor map encoding of F failed";
   cudaGetLastError();
   if (!tc.fused_ok && !tc.split_ok) return "coupling tile exceeds shared memory";
-  tc.split = !tc.fused_ok;
+  tc.split = !tc.fused_ok && !tc.use_lane;
   (void)t;
   return "";
 }
@@ -462,7 +488,9 @@ std::string setup_tc(tp3_ctx* c) {
 void free_scratch(tp3_ctx* c) {
   cudaFree(c->d_coeff); cudaFree(c->d_cc); cudaFree(c->d_T); cudaFree(c->d_part); cudaFree(c->d_E);
   cudaFree(c->d_Thi); cudaFree(c->d_Tlo); cudaFree(c->d_Eslab); cudaFree(c->d_sym); cudaFree(c->d_D);
-  cudaFree(c->d_H);
+  cudaFree(c->d_H); cudaFree(c->d_ct); cudaFree(c->d_c3p);
+  c->d_ct = nullptr;
+  c->d_c3p = nullptr;
   c->d_D = nullptr;
   c->d_H = nullptr;
   cudaFreeHost(c->h_coeff); cudaFreeHost(c->h_E);
@@ -498,6 +526,9 @@ int ensure_cap(tp3_ctx* c, int n) {
       (c->tc_ok && (e = cudaMalloc(&c->d_Eslab, ((size_t)n * (t.klength + 2 * (size_t)c->tc.nhalf * t.klp) + 1) *
                                                     sizeof(double))) != cudaSuccess) ||
       (e = cudaMalloc(&c->d_sym, (size_t)n * sizeof(int))) != cudaSuccess ||
+      (c->tc_ok && c->tc.lane.ok &&
+       ((e = cudaMalloc(&c->d_ct, (size_t)n * t.nc * c->tc.lane.ps * sizeof(float2))) != cudaSuccess ||
+        (e = cudaMalloc(&c->d_c3p, (size_t)n * t.nc * c->tc.lane.c3row * sizeof(float4))) != cudaSuccess)) ||
       (t.nqp > 0 && (e = cudaMalloc(&c->d_H, (size_t)n * t.klp * t.nqp * sizeof(float))) != cudaSuccess) ||
       (c->tc_ok && c->tc.split_ok &&
        (e = cudaMalloc(&c->d_D, (size_t)c->tc.dsub * c->tc.dstride * sizeof(float2))) != cudaSuccess) ||
@@ -555,11 +586,19 @@ int run_coupling(tp3_ctx* c, int n, const double2* d_coeff, bool want_T32, bool 
   if (is_tc(c->mode)) {
     // lambda != 0: the coupling also writes FP32 T, from which H (the angular operand) is built
     if (c->tc.hform) want_T32 = true;
-    if ((e = tp3::launch_gather_sym(t, c->tc, n, d_coeff, lay, c->d_cc, c->d_sym, c->stream, rag)) != cudaSuccess)
+    if (c->tc.use_lane) {
+      if ((e = tp3::launch_gather_lane(t, c->tc, n, d_coeff, lay, c->d_ct, c->d_c3p, c->d_sym, c->stream, rag)) !=
+          cudaSuccess)
+        return cuda_fail(c, e, "gather_lane");
+    } else if ((e = tp3::launch_gather_sym(t, c->tc, n, d_coeff, lay, c->d_cc, c->d_sym, c->stream, rag)) != cudaSuccess)
       return cuda_fail(c, e, "gather_sym");
     cudaEvent_t ca, cb;
     const int pc = prof_begin_in(c, c->ev_c, c->ev_c_used, &ca, &cb);
-    if (rag)  // ragged batches use the one-kernel coupling (it skips absent blocks and shells)
+    if (c->tc.use_lane)
+      e = tp3::launch_couple_lane(t, c->tc, n, c->d_ct, c->d_c3p, c->d_sym, c->d_Thi, c->d_Tlo,
+                                  c->mode == TP3_MODE_TC_TF32X3, want_T32 ? c->d_T : nullptr, false, c->d_T, c->stream,
+                                  rag);
+    else if (rag)  // ragged batches use the one-kernel coupling (it skips absent blocks and shells)
       e = tp3::launch_couple_pair(t, c->tc, n, c->d_cc, c->d_sym, c->d_Thi, c->d_Tlo, c->mode == TP3_MODE_TC_TF32X3,
                                   want_T32 ? c->d_T : nullptr, c->stream, rag);
     else if (c->tc.split)
@@ -659,16 +698,17 @@ int check_ctx(tp3_ctx* c) {
 }
 
 // Coupling form of the tensor-core path: 0 one-kernel, 1 split, 2 one-kernel small
-// tiling, 3 warp-local (512 threads), 4 warp-local (256 threads, two CTAs per SM); a
-// form this shape cannot run falls back to one that it can.
+// tiling, 3 warp-local (512 threads), 4 warp-local (256 threads, two CTAs per SM), 5 to 8
+// folded-row, 9 lane-owned; a form this shape cannot run falls back to one that it can.
 void apply_coupling(tp3_ctx* c, int form) {
   TcTables& tc = c->tc;
+  tc.use_lane = form == 9 && tc.lane.ok;
   tc.use_fold = (form == 5 && tc.fold[0].ok) ? 0 : (form == 6 && tc.fold[1].ok) ? 1
                  : (form == 7 && tc.fold[2].ok) ? 2 : (form == 8 && tc.fold[3].ok) ? 3 : -1;
   tc.use_small = form == 2 && tc.small_ok;
   tc.use_warp = form == 3 && tc.warp_ok;
   tc.use_warp2 = form == 4 && tc.warp2_ok;
-  tc.split = (form == 1 && tc.split_ok) || (!tc.fused_ok && !tc.use_warp && !tc.use_warp2 && tc.use_fold < 0);
+  tc.split = (form == 1 && tc.split_ok) || (!tc.fused_ok && !tc.use_warp && !tc.use_warp2 && tc.use_fold < 0 && !tc.use_lane);
   if (tc.split) tc.use_small = tc.use_warp = tc.use_warp2 = false, tc.use_fold = -1;
 }
 
@@ -1031,6 +1071,7 @@ int tp3_autotune(tp3_ctx* c, int n, double* report, int* nreport) {
       if (c->tc.fold[1].ok) vars.push_back({m, 6, true});
       if (c->tc.fold[2].ok) vars.push_back({m, 7, true});
       if (c->tc.fold[3].ok) vars.push_back({m, 8, true});
+      if (c->tc.lane.ok) vars.push_back({m, 9, true});
     }
   // synthetic real-function coefficients (c[l,-m] = (-1)^m conj c[l,m]), n sets
   const size_t nco = (size_t)b.K * b.LMAX * b.LMAX;
@@ -1071,6 +1112,7 @@ int tp3_autotune(tp3_ctx* c, int n, double* report, int* nreport) {
   const bool warp0 = c->tc_ok ? c->tc.use_warp : false;
   const bool warp20 = c->tc_ok ? c->tc.use_warp2 : false;
   const int fold0 = c->tc_ok ? c->tc.use_fold : -1;
+  const bool lane0 = c->tc_ok ? c->tc.use_lane : false;
   const bool persist0 = c->tc_ok ? c->tc.persist : true;
   const bool prof0 = c->prof;
   c->prof = false;
@@ -1125,7 +1167,8 @@ int tp3_autotune(tp3_ctx* c, int n, double* report, int* nreport) {
     c->mode = mode0;
     if (c->tc_ok) {
       c->tc.split = split0; c->tc.use_small = small0; c->tc.use_warp = warp0;
-      c->tc.use_warp2 = warp20; c->tc.use_fold = fold0; c->tc.persist = persist0;
+      c->tc.use_warp2 = warp20; c->tc.use_fold = fold0; c->tc.use_lane = lane0;
+      c->tc.persist = persist0;
     }
     return rc != TP3_OK ? rc : fail(c, TP3_ERR_UNSUPPORTED, "no variant ran");
   }
@@ -1164,8 +1207,8 @@ int tp3_set_coupling(tp3_ctx* c, int form) {
   const bool ok = (form == 0 && c->tc.fused_ok) || (form == 1 && c->tc.split_ok) || (form == 2 && c->tc.small_ok) ||
                   (form == 3 && c->tc.warp_ok) || (form == 4 && c->tc.warp2_ok) || (form == 5 && c->tc.fold[0].ok) ||
                   (form == 6 && c->tc.fold[1].ok) || (form == 7 && c->tc.fold[2].ok) ||
-                  (form == 8 && c->tc.fold[3].ok);
-  if (!ok) return fail(c, form < 0 || form > 8 ? TP3_ERR_ARG : TP3_ERR_UNSUPPORTED, "coupling form not available");
+                  (form == 8 && c->tc.fold[3].ok) || (form == 9 && c->tc.lane.ok);
+  if (!ok) return fail(c, form < 0 || form > 9 ? TP3_ERR_ARG : TP3_ERR_UNSUPPORTED, "coupling form not available");
   apply_coupling(c, form);
   return TP3_OK;
 }

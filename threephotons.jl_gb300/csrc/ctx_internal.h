@@ -57,6 +57,8 @@ struct tp3_ctx {
   float* d_c3 = nullptr;       // [klength][G] (one proposal)
   int* d_err = nullptr;        // device error flag (timeouts)
   int* d_sym = nullptr;        // [cap] real-function symmetry flag per proposal
+  float2* d_ct = nullptr;      // [cap][nc][ps] coefficients, shells contiguous (lane-owned coupling)
+  float* d_c3p = nullptr;      // [cap][nc][4 c3row] the same, real and imaginary parts of four shells apart
   float2* d_D = nullptr;       // [dsub][dstride] pair-coupled D of the split coupling
   float* d_H = nullptr;        // [cap][klp][nqp] Fourier-pair operand (lambda != 0)
   double* h_coeff = nullptr;   // pinned [cap][K][LMAX^2][2]

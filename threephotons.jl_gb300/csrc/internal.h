@@ -9,6 +9,8 @@
 
 namespace tp3 {
 
+struct Wigner3jTable;  // tables.h
+
 // TP3_DEBUG builds (TP3_DEBUG=1 python threephotons.jl_gb300/build.py --force) check the
 // indices that the gather and folded-row coupling kernels compute before each shared- or
 // global-memory access; a failed check sets TP3_ERR_BOUNDS in the context's error flag
@@ -125,8 +127,44 @@ struct FoldVariant {
   const int2* chunks = nullptr;
 };
 
+// Lane-owned coupling (kernels_lane.cu): per pair block, quads of consecutive m3 with the 3j
+// values of their four m3 side by side.
+constexpr int kLaneMaxQuads = 20;
+struct LaneQuad {
+  int m3;      // m3 .. m3 + 3
+  int n;       // steps (m of the shorter coefficient row)
+  int x0, vb;  // first row of the stepped operand, first window row of the sliding one
+  int c0, rs;  // first stored order and orders per step
+  int wofs;    // float4 offset in the staged 3j values
+  int pad;
+};
+struct LaneBlock {
+  int l1, l2, l3min, nl3, lt_base;
+  int swap;    // l1 > l2: steps run over m2 and c_k1 slides
+  int c1, c2;  // first coefficient rows of l1 and l2
+  int q0, nq;  // quads of the real-function path (m3 >= 0, all orders)
+  int w0, wn;  // its 3j values (float4)
+};
+struct LaneTables {
+  bool ok = false;
+  int nw = 0, ctas = 0;  // warps per CTA, CTAs per SM
+  int ps = 0, c3row = 0; // shells per coefficient row (32 or 64), float4 per c_k3 row
+  int crows = 0, wmax = 0, c3rows = 0, stage = 0;
+  int maxz = 1;          // CTAs over which one block's tasks can spread
+  size_t smem = 0;
+  const LaneBlock* blks = nullptr;
+  const LaneQuad* quads = nullptr;
+  const int4* gcols = nullptr;  // [n_pb][16] general path, per order: first quad, quads, first 3j float4, count
+  const float4* w = nullptr;
+  const uint32_t* utab = nullptr;   // units (build_lane_units)
+  const uint32_t* slots = nullptr;
+  const int2* kofs = nullptr;       // [K + 1]
+};
+
 // Device tables of the tensor-core path.
 struct TcTables {
+  LaneTables lane;
+  bool use_lane = false;
   // folded-row coupling tilings: [0] 8 warps, [1] 7 warps, [2] 13 warps (smaller D
   // buffers, more l3 chunks), [3] 14 warps in pairs sharing 7 D buffers; one CTA per SM
   FoldVariant fold[4];
@@ -230,16 +268,32 @@ cudaError_t launch_finalize_parts(const DevTables& t, const TcTables& tc, int n,
 size_t couple_split_smem_d(const DevTables& t, const TcTables& tc);
 size_t couple_split_smem_t(const DevTables& t, const TcTables& tc);
 cudaError_t couple_split_configure(const DevTables& t, const TcTables& tc);
-std::string build_fold_tables(const std::vector<PairBlock>& pbs, int drows, std::vector<FoldBlock>& blks,
+std::string build_fold_tables(const std::vector<PairBlock>& pbs, const Wigner3jTable& w3j, int drows, std::vector<FoldBlock>& blks,
                               std::vector<FoldRow>& rows, std::vector<float>& w, std::vector<int2>& chunks,
                               int& wmax, int& cmax);
 // ngroups: D buffers and staging rows (warps per CTA / warps per unit)
 size_t fold_smem_bytes(int ngroups, int ps, int drows, int wmax, int cmax, int stage);
-// Layout of the T operand: the folded-row coupling in BF16 mode writes it order-major,
+// Lane-owned coupling (kernels_lane.cu).
+std::string build_lane_tables(const std::vector<PairBlock>& pbs, const std::vector<int>& coff, const Wigner3jTable& w3j,
+                              std::vector<LaneBlock>& blks, std::vector<LaneQuad>& quads, std::vector<int4>& gcols,
+                              std::vector<float4>& w, int& crows, int& wmax, int& c3rows);
+void build_lane_units(int K, std::vector<uint32_t>& utab, std::vector<uint32_t>& slots, std::vector<int2>& kofs,
+                      int& stage);
+int lane_tasks(int nu, int nl3);
+void lane_pick_warps(LaneTables& lt);
+cudaError_t lane_configure();
+cudaError_t launch_gather_lane(const DevTables& t, const TcTables& tc, int n, const double2* coeff, CoeffLayout lay,
+                               float2* ct, float* c3p, int* sym, cudaStream_t s, const RagInfo* rag = nullptr);
+// T32 (nullable): FP32 T as [ki][n_ltp] rows, or [lt][klp] when t32maj; Thi null: T32 only.
+// scratch: klp x n_ltp floats a proposal (TF32 without T32).
+cudaError_t launch_couple_lane(const DevTables& t, const TcTables& tc, int n, const float2* ct, const float* c3p,
+                               const int* sym, void* Thi, void* Tlo, bool tf32, float* T32, bool t32maj, float* scratch,
+                               cudaStream_t s, const RagInfo* rag = nullptr);
+// Layout of the T operand: the lane-owned and folded-row couplings in BF16 mode write it order-major,
 // [lt][ki] (shell triples contiguous), read by the angular kernel as an MN-major operand;
 // every other coupling form and the TF32 mode use [ki][lt].
 inline bool t_order_major(const TcTables& tc, bool tf32) {
-  return !tf32 && !tc.hform && tc.use_fold >= 0 && tc.fold[tc.use_fold].ok;
+  return !tf32 && !tc.hform && (tc.use_lane || (tc.use_fold >= 0 && tc.fold[tc.use_fold].ok));
 }
 cudaError_t fold_configure();
 cudaError_t launch_couple_fold(const DevTables& t, const TcTables& tc, const FoldVariant& fv, int n, const float2* cc,

@@ -483,7 +483,7 @@ __global__ void __launch_bounds__(NW * 32, 1) k_couple_fold(
 
 // ---- host side ----------------------------------------------------------------
 
-std::string build_fold_tables(const std::vector<PairBlock>& pbs, int drows, std::vector<FoldBlock>& blks,
+std::string build_fold_tables(const std::vector<PairBlock>& pbs, const Wigner3jTable& w3j, int drows, std::vector<FoldBlock>& blks,
                               std::vector<FoldRow>& rows, std::vector<float>& w, std::vector<int2>& chunks,
                               int& wmax, int& cmax) {
   blks.clear();
@@ -536,7 +536,7 @@ std::string build_fold_tables(const std::vector<PairBlock>& pbs, int drows, std:
               const int m3 = q == 0 ? m3a : m3b;
               const int s0 = q == 0 ? fr.s0a : fr.s0b;
               const bool in = (q == 0 || hasb) && s >= s0 && s < pb.nl3 && m1 >= m1lo_of(m3) && m1 <= m1hi_of(m3);
-              w.push_back(in ? (float)tp3::wigner3j(pb.l1, pb.l2, l3, m1, -m3 - m1, m3) : 0.f);
+              w.push_back(in ? (float)w3j(pb.l1, pb.l2, l3, m1, -m3 - m1, m3) : 0.f);
             }
           }
           run += 2 * fr.rs;

@@ -1,0 +1,845 @@
+// Stage (a) coupling, lane-owned form: the reference's triple products
+//   T[(k1,k2,k3)][(l1,l2,l3)] = sum_j w_j Re(c_k1[l1,m1] c_k2[l2,m2] c_k3[l3,m3])
+// (src/correlations.jl:157-176; src/cuda_kernel.cu:31-37), pair-factorised as
+//   D[k1,k2][l3][m3] = sum_m1 w(l1 m1 l2 m2 l3 m3) c_k1[l1,m1] c_k2[l2,m2],  m2 = -m3 - m1
+//   T[(k1,k2,k3)][lt] = Re sum_m3 D[k1,k2][l3][m3] c_k3[l3,m3]
+// with D and T held in the registers of the lane that owns the shell pair (k1, k2).
+//
+// Units: the shell pairs with k3 in one block of 16 shells, sorted by k2 downwards, 32
+// consecutive pairs a warp, one a lane, so the lanes of a warp need nearly the same k3 <= k2.
+// A task is one unit and a run of up to NC orders l3 of one (l1, l2) block; its T accumulators
+// (NC orders x 16 shells k3) stay in registers while the warp walks quads of four consecutive m3:
+//   Phase 1: D of the quad's four m3 and the task's orders.  One of the two coefficient rows
+//     of a product is the same for all four m3, the other slides by one m, so a step loads two
+//     coefficients, forms four complex products and feeds one 16-byte 3j broadcast (the four
+//     m3) per order into four packed FMAs.
+//   Phase 2: T += Re(D c_k3) for the quad, packed over pairs of k3; c_k3 comes as 16-byte
+//     broadcasts (all lanes read the same four shells).
+// A warp needs no other warp, so warps take tasks from a counter, heaviest first.
+//
+// What bounds it: issue slots.  At L = 18, K = 26 a proposal is 12.2 M warp instructions (the
+// folded rows 15.5 M) at 65 % issue and 47 % of the FMA pipe; 6.1 us of FMA pipe time on 152
+// SMs (phase 1 4.5, phase 2 1.5) in 14.8 us.  Only coefficients and 3j values are shared, 75 KB
+// a CTA with no D buffer, which lets 16 warps run with no barrier after the staging.
+//
+// Every accumulation runs in the order of the one-kernel pair coupling (k_couple_pair), so
+// both give the same bits: m1 upwards in phase 1, m3 = 1 .. l3 then the doubled sum plus the
+// m3 = 0 term in phase 2 (real functions), or m3 = -l3 .. l3 (general coefficients).
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cmath>
+#include <cstdint>
+#include <string>
+#include <type_traits>
+#include <vector>
+
+#include "../../include/tp3.h"
+#include "internal.h"
+#include "tables.h"
+#include "tc_prims.cuh"
+
+
+namespace tp3 {
+namespace {
+
+// Orders per task: 16 kLaneNC accumulator registers for T and 8 kLaneNC for D, 128 a thread in
+// all, so 16 warps per SM.  All kLaneNC columns are always computed (columns outside the task
+// are not used): with a loop per column count, or more instances for more shells k3, the code
+// of an SM's warps left its instruction cache (29 of 34 stall cycles per issue with one
+// instance per width of k3).  64 proposals at L = 18, K = 26: 0.95 ms at 3 orders and 16 warps,
+// 1.02 at 4 and 12, 1.44 at 5 and 12 (spills), 1.30 at 5 with a loop per column count; the
+// one-kernel pair coupling takes 2.51 ms and the folded rows at 13 warps 1.58.
+constexpr int kLaneNC = 3;
+constexpr int kLaneMaxWarps = 16;
+
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                   smem_u32(dst)),
+               "l"((uint64_t)__cvta_generic_to_global(src)), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
+
+__device__ __forceinline__ float2 lds2(uint32_t a) {
+  float2 v;
+  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
+  return v;
+}
+
+__device__ __forceinline__ float4 lds4(uint32_t a) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+  return v;
+}
+
+// Shared-memory addresses of one (proposal, block).
+struct LaneView {
+  uint32_t X;         // float2 rows, operand with one row per step
+  uint32_t V;         // float2 rows, operand that slides by one row per m3
+  uint32_t W;         // 3j values, float4 per (step, order): the quad's four m3
+  uint32_t C3;        // c_k3 rows: (re x 4, im x 4) per quad of shells
+  const LaneQuad* quads;
+  int nq;
+};
+
+// One step of phase 1: the products of x with the window rows of the quad's four m3, each into
+// its half of the packed accumulators.  SW: x is c_k2 and the window c_k1 (in the imaginary
+// part the product with c_k1's imaginary part is the fused one).  FIRST: sets the accumulators.
+template <int NC, bool SW, bool FIRST>
+__device__ __forceinline__ void lane_step(const float2 x, const float2 v0, const float2 v1, const float2 v2,
+                                          const float2 v3, uint32_t w, float2 (&R0)[NC], float2 (&I0)[NC],
+                                          float2 (&R1)[NC], float2 (&I1)[NC]) {
+  auto re = [&](const float2 v) { return fmaf(x.x, v.x, -(x.y * v.y)); };
+  auto im = [&](const float2 v) { return SW ? fmaf(v.y, x.x, v.x * x.y) : fmaf(x.y, v.x, x.x * v.y); };
+  const float2 xr0 = make_float2(re(v0), re(v1)), xr1 = make_float2(re(v2), re(v3));
+  const float2 xi0 = make_float2(im(v0), im(v1)), xi1 = make_float2(im(v2), im(v3));
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const float4 wv = lds4(w + 16 * c);
+    const float2 w0 = make_float2(wv.x, wv.y), w1 = make_float2(wv.z, wv.w);
+    if (FIRST) {
+      R0[c] = __fmul2_rn(w0, xr0);
+      I0[c] = __fmul2_rn(w0, xi0);
+      R1[c] = __fmul2_rn(w1, xr1);
+      I1[c] = __fmul2_rn(w1, xi1);
+    } else {
+      R0[c] = __ffma2_rn(w0, xr0, R0[c]);
+      I0[c] = __ffma2_rn(w0, xi0, I0[c]);
+      R1[c] = __ffma2_rn(w1, xr1, R1[c]);
+      I1[c] = __ffma2_rn(w1, xi1, I1[c]);
+    }
+  }
+}
+
+// Phase 1 of one quad: n steps (odd) over all NC columns; PS shells per coefficient row, rs
+// bytes of 3j values per step.  The window rows run with the steps (SW: against m3).
+template <int NC, int PS, bool SW>
+__device__ __forceinline__ void lane_p1(uint32_t x, uint32_t v, int n, uint32_t w, uint32_t rs, float2 (&R0)[NC],
+                                        float2 (&I0)[NC], float2 (&R1)[NC], float2 (&I1)[NC]) {
+  constexpr int xs = 8 * (SW ? -PS : PS), vs = -xs;
+  auto step = [&](const float2 xv, const float2 a, const float2 b, const float2 c, const float2 d, uint32_t wa, auto first) {
+    if (SW)
+      lane_step<NC, SW, decltype(first)::value>(xv, d, c, b, a, wa, R0, I0, R1, I1);
+    else
+      lane_step<NC, SW, decltype(first)::value>(xv, a, b, c, d, wa, R0, I0, R1, I1);
+  };
+  float2 a = lds2(v + vs), b = lds2(v + 2 * vs), c = lds2(v + 3 * vs);
+  step(lds2(x), lds2(v), a, b, c, w, std::true_type());
+  x += xs;
+  v += 4 * vs;
+  w += rs;
+  int i = n - 1;
+#pragma unroll 1
+  for (; i >= 4; i -= 4) {
+    const float2 d = lds2(v), e = lds2(v + vs), f = lds2(v + 2 * vs), g = lds2(v + 3 * vs);
+    step(lds2(x), a, b, c, d, w, std::false_type());
+    step(lds2(x + xs), b, c, d, e, w + rs, std::false_type());
+    step(lds2(x + 2 * xs), c, d, e, f, w + 2 * rs, std::false_type());
+    step(lds2(x + 3 * xs), d, e, f, g, w + 3 * rs, std::false_type());
+    a = e; b = f; c = g;
+    v += 4 * vs;
+    x += 4 * xs;
+    w += 4 * rs;
+  }
+#pragma unroll 1
+  for (; i > 0; --i) {
+    const float2 d = lds2(v);
+    step(lds2(x), a, b, c, d, w, std::false_type());
+    a = b; b = c; c = d;
+    v += vs;
+    x += xs;
+    w += rs;
+  }
+}
+
+// T of one order: acc (pairs of k3) += Re(D c_k3) for one m3 and the unit's 8 or 16 shells k3.
+__device__ __forceinline__ void lane_p2(uint32_t row, float dr, float di, bool wide, float2 (&acc)[8]) {
+  const float2 a = make_float2(dr, dr), b = make_float2(-di, -di);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    if (j == 2 && !wide) break;
+    const float4 r = lds4(row + 32 * j), s = lds4(row + 32 * j + 16);
+    acc[2 * j] = __ffma2_rn(a, make_float2(r.x, r.y), __ffma2_rn(b, make_float2(s.x, s.y), acc[2 * j]));
+    acc[2 * j + 1] = __ffma2_rn(a, make_float2(r.z, r.w), __ffma2_rn(b, make_float2(s.z, s.w), acc[2 * j + 1]));
+  }
+}
+
+// Where a task's T goes.
+struct LaneOut {
+  void *hi, *lo;       // split operand of the proposal (null: not written)
+  float* T32;          // FP32 T of the proposal (null: not written)
+  int KP, klp, ldT32;
+  bool tf32, ltmaj, t32maj;
+};
+
+// One task: orders s_lo .. s_lo + w - 1 of the block for the 32 shell pairs of a unit; CR bytes
+// per c_k3 row, slots / nslot: the unit's staging slots (build_lane_units).
+template <int NC, int PS, int CR>
+__device__ __forceinline__ void lane_task(const LaneView& V, bool swap, bool sym, int l3min, int s_lo, int w, int lt_base,
+                                          bool wide, int k1, int k2, int len, int off, int nslot, float* stage,
+                                          const uint32_t* __restrict__ slots, const LaneOut& o) {
+  const int lane = threadIdx.x & 31;
+  float2 acc[NC][8];
+#pragma unroll
+  for (int c = 0; c < NC; ++c)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[c][j] = make_float2(0.f, 0.f);
+  float2 R0[NC], I0[NC], R1[NC], I1[NC];
+  // column c is order s_lo + c - (NC - w); it takes the m3 with (unsigned)(m3 - m_lo) < cnt[c]
+  // (none for the NC - w columns before the task's orders).  row[c]: address of its c_k3 row of
+  // the quad's first m3: after the rows of the orders below (real functions, m3 = 0 .. l3), or
+  // of the only order staged (general coefficients, m3 = -l3 .. l3)
+  const int s_hi = s_lo + w, s_off = s_lo - (NC - w);
+  int m_lo = sym ? 1 : -(l3min + 2 * s_lo);  // the m3 = 0 term of real functions is added last
+  uint32_t row[NC];
+  int cnt[NC];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const int s = s_off + c, l3 = l3min + 2 * s;
+    cnt[c] = s < s_lo ? 0 : l3 - m_lo + 1;
+    row[c] = V.C3 + CR * (sym ? s * (l3min + s) : V.quads[0].m3 + l3);
+  }
+  const uint32_t xk = V.X + 8 * (swap ? k2 : k1), vk = V.V + 8 * (swap ? k1 : k2);
+  float2* D0 = reinterpret_cast<float2*>(stage);  // real functions: D of m3 = 0, [NC][32]
+#pragma unroll 1
+  for (int qi = 0; qi <= V.nq; ++qi) {
+    int m = 0;
+    if (qi < V.nq) {
+      const LaneQuad q = V.quads[qi];
+      if (q.c0 >= s_hi) continue;
+      m = q.m3;
+      // all NC columns; those outside the task or below the quad's orders are not used
+      const uint32_t x = xk + 8 * PS * q.x0, v = vk + 8 * PS * q.vb, wt = V.W + 16 * (q.wofs + s_hi - NC - q.c0);
+      if (swap)
+        lane_p1<NC, PS, true>(x, v, q.n, wt, 16 * q.rs, R0, I0, R1, I1);
+      else
+        lane_p1<NC, PS, false>(x, v, q.n, wt, 16 * q.rs, R0, I0, R1, I1);
+      if (sym && m == 0) {
+#pragma unroll
+        for (int c = 0; c < NC; ++c) D0[c * 32 + lane] = make_float2(R0[c].x, I0[c].x);
+      }
+    } else {
+      if (!sym) break;
+      // T = 2 sum_{m3 > 0} Re(D c) + Re(D[0] c[0])
+      m_lo = 0;
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        const int s = s_off + c;
+        cnt[c] = s < s_lo ? 0 : 1;
+        row[c] = V.C3 + CR * (s * (l3min + s));
+        const float2 d = D0[c * 32 + lane];
+        R0[c].x = d.x;
+        I0[c].x = d.y;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          acc[c][j].x *= 2.f;
+          acc[c][j].y *= 2.f;
+        }
+      }
+    }
+    // phase 2, two m3 at a time
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int t = m + 2 * h - m_lo;
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        if ((unsigned)t < (unsigned)cnt[c]) lane_p2(row[c], h ? R1[c].x : R0[c].x, h ? I1[c].x : I0[c].x, wide, acc[c]);
+        if ((unsigned)(t + 1) < (unsigned)cnt[c])
+          lane_p2(row[c] + CR, h ? R1[c].y : R0[c].y, h ? I1[c].y : I0[c].y, wide, acc[c]);
+        row[c] += 2 * CR;
+      }
+    }
+  }
+  __syncwarp();
+  // T leaves order by order through the warp's staging row, in which the unit's shell triples
+  // are sorted by their index, an even one on an even position: a lane takes slots of two
+#pragma unroll 1
+  for (int c = NC - w; c < NC; ++c) {
+    const int lt = lt_base + s_off + c;
+#define TP3_LANE_PUT(C)                                                                               \
+  case C:                                                                                             \
+    _Pragma("unroll") for (int j = 0; j < 16; ++j) if (j < len) stage[off + j] =                      \
+        (j & 1) ? acc[C][j >> 1].y : acc[C][j >> 1].x;                                                \
+    break;
+    switch (c) {
+      TP3_LANE_PUT(0) TP3_LANE_PUT(1) TP3_LANE_PUT(2)
+      default: break;
+    }
+#undef TP3_LANE_PUT
+    __syncwarp();
+    if (o.hi && o.ltmaj) {
+      __nv_bfloat16* hrow = reinterpret_cast<__nv_bfloat16*>(o.hi) + (size_t)lt * o.klp;
+      __nv_bfloat16* lrow = reinterpret_cast<__nv_bfloat16*>(o.lo) + (size_t)lt * o.klp;
+      auto put = [&](const uint32_t sl, const float2 t) {
+        const uint32_t at = (sl >> 2) * 2;
+        const __nv_bfloat162 h = __floats2bfloat162_rn(t.x, t.y);
+        const float2 hf = __bfloat1622float2(h);
+        const __nv_bfloat162 l = __floats2bfloat162_rn(t.x - hf.x, t.y - hf.y);
+        if ((sl & 3) == 3) {
+          *reinterpret_cast<__nv_bfloat162*>(hrow + at) = h;
+          *reinterpret_cast<__nv_bfloat162*>(lrow + at) = l;
+        } else if (sl & 1) {
+          hrow[at] = h.x;
+          lrow[at] = l.x;
+        } else if (sl & 2) {
+          hrow[at + 1] = h.y;
+          lrow[at + 1] = l.y;
+        }
+      };
+      const float2* st = reinterpret_cast<const float2*>(stage);
+#pragma unroll 1
+      for (int i = lane; i < nslot; i += 64) {
+        const bool two = i + 32 < nslot;
+        const uint32_t sa = __ldg(slots + i), sb = two ? __ldg(slots + i + 32) : 0u;
+        const float2 ta = st[i], tb = st[two ? i + 32 : i];
+        put(sa, ta);
+        put(sb, tb);
+      }
+    }
+    if (!o.ltmaj || o.T32) {
+#pragma unroll 1
+      for (int i = lane; i < 2 * nslot; i += 32) {
+        const uint32_t sl = __ldg(slots + (i >> 1));
+        if (!((sl >> (i & 1)) & 1)) continue;
+        const int ki = 2 * (int)(sl >> 2) + (i & 1);
+        const float t = stage[i];
+        if (o.hi && !o.ltmaj) {
+          const size_t at = (size_t)ki * o.KP + lt;
+          if (o.tf32) {
+            uint32_t h;
+            asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h) : "f"(t));
+            reinterpret_cast<float*>(o.hi)[at] = __uint_as_float(h);
+            reinterpret_cast<float*>(o.lo)[at] = t - __uint_as_float(h);
+          } else {
+            const __nv_bfloat16 h = __float2bfloat16_rn(t);
+            reinterpret_cast<__nv_bfloat16*>(o.hi)[at] = h;
+            reinterpret_cast<__nv_bfloat16*>(o.lo)[at] = __float2bfloat16_rn(t - __bfloat162float(h));
+          }
+        }
+        if (o.T32) o.T32[o.t32maj ? (size_t)lt * o.klp + ki : (size_t)ki * o.ldT32 + lt] = t;
+      }
+    }
+    __syncwarp();
+  }
+}
+
+// grid: (n, n_pb, Z); block 32 x warps; dynamic shared memory LaneTables::smem.
+// CTA (p, b, z) takes the tasks z, z + Z, .. of block b of proposal p: Z > 1 spreads the
+// tasks of a small batch over the SMs.  Proposals run fastest, so an SM's CTAs are mostly on
+// one block and their warps in the same code.
+template <int PS>
+__global__ void __launch_bounds__(32 * kLaneMaxWarps, 1) k_couple_lane(
+    const float2* __restrict__ ct, const float4* __restrict__ c3p, int K, int nc, const int* __restrict__ coff, const LaneBlock* __restrict__ blks, const LaneQuad* __restrict__ quads,
+    const int4* __restrict__ gcols, const float4* __restrict__ wtab, const uint32_t* __restrict__ utab,
+    const uint32_t* __restrict__ slots, const int2* __restrict__ kofs, int crows, int wmax, int c3rows, int stage_len,
+    const int* __restrict__ symflags, LaneOut out, const RagInfo* __restrict__ rag, int* __restrict__ err) {
+  constexpr int ps = PS, c3row = PS / 2;
+  extern __shared__ __align__(16) unsigned char lane_smem[];
+  __shared__ LaneQuad s_quads[kLaneMaxQuads];
+  __shared__ uint64_t s_bar;
+  __shared__ int s_next[17];
+  __shared__ int s_abort;
+  const int prop = blockIdx.x;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const LaneBlock fb = blks[blockIdx.y];
+  int Kp = K;
+  bool skip = false;
+  int klen = 0;
+  if (rag) {
+    const RagInfo ri = rag[prop];
+    Kp = ri.K;
+    klen = ri.klen;
+    skip = fb.l1 > ri.L || fb.l2 > ri.L;
+  }
+  const size_t pbase = (size_t)prop * out.klp * out.KP;
+  if (out.hi) {
+    out.hi = out.tf32 ? (void*)((float*)out.hi + pbase) : (void*)((__nv_bfloat16*)out.hi + pbase);
+    out.lo = out.tf32 ? (void*)((float*)out.lo + pbase) : (void*)((__nv_bfloat16*)out.lo + pbase);
+  }
+  if (out.T32) out.T32 += (size_t)prop * out.klp * out.ldT32;
+  if (skip) {
+    // absent orders: the block's l-triples are zero for this proposal's scored rows
+    for (int i = threadIdx.x + blockIdx.z * blockDim.x; i < klen * fb.nl3; i += blockDim.x * gridDim.z) {
+      const int s = i / klen, ki = i - s * klen, lt = fb.lt_base + s;
+      if (out.hi) {
+        const size_t at = out.ltmaj ? (size_t)lt * out.klp + ki : (size_t)ki * out.KP + lt;
+        if (out.tf32) {
+          reinterpret_cast<float*>(out.hi)[at] = 0.f;
+          reinterpret_cast<float*>(out.lo)[at] = 0.f;
+        } else {
+          reinterpret_cast<__nv_bfloat16*>(out.hi)[at] = __float2bfloat16_rn(0.f);
+          reinterpret_cast<__nv_bfloat16*>(out.lo)[at] = __float2bfloat16_rn(0.f);
+        }
+      }
+      if (out.T32) out.T32[out.t32maj ? (size_t)lt * out.klp + ki : (size_t)ki * out.ldT32 + lt] = 0.f;
+    }
+    return;
+  }
+  const bool sym = symflags[prop] != 0;
+  const int2 ko = kofs[Kp];
+  const int nu = ko.y;
+  if ((int)blockIdx.z >= (sym ? nu * fb.nl3 : nu)) return;  // more CTAs than tasks
+  float2* C1 = reinterpret_cast<float2*>(lane_smem);
+  float2* C2 = C1 + (size_t)crows * ps;
+  float4* W = reinterpret_cast<float4*>(C2 + (size_t)crows * ps) + 8;  // a rounded-up run may start before its row
+  float4* C3 = W + wmax;
+  float* stage = reinterpret_cast<float*>(C3 + (size_t)c3rows * c3row) + (size_t)warp * stage_len;
+  const float2* ctp = ct + (size_t)prop * nc * ps;
+  const float4* c3g = c3p + (size_t)prop * nc * c3row;
+  const int n1r = 2 * fb.l1 + 1, n2r = 2 * fb.l2 + 1;
+  const int passes = sym ? 1 : fb.nl3;  // general coefficients: one order at a time
+  // three zero rows at either end of C1 and C2: the union m range of a quad reaches up to
+  // three rows past an end, where its 3j value is zero
+  for (int i = threadIdx.x; i < 6 * ps; i += blockDim.x) {
+    const int r = i / ps, k = i - r * ps;
+    C1[(r < 3 ? r : n1r + r) * ps + k] = make_float2(0.f, 0.f);
+    C2[(r < 3 ? r : n2r + r) * ps + k] = make_float2(0.f, 0.f);
+  }
+  if (threadIdx.x == 0) {
+    mbar_init(&s_bar, 1);
+    s_abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (threadIdx.x < 17) s_next[threadIdx.x] = 0;
+  __syncthreads();
+  LaneView V;
+  V.X = smem_u32(fb.swap ? C2 : C1);
+  V.V = smem_u32(fb.swap ? C1 : C2);
+  V.W = smem_u32(W);
+  V.C3 = smem_u32(C3);
+  V.quads = s_quads;
+  for (int pass = 0; pass < passes; ++pass) {
+    int4 g = make_int4(fb.q0, fb.nq, fb.w0, fb.wn);
+    if (!sym) g = gcols[blockIdx.y * 16 + pass];
+    if (pass > 0) {
+      __syncthreads();  // the previous order's reads are done
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (threadIdx.x == 0) {
+      uint32_t bytes = (uint32_t)g.w * 16u;
+      if (pass == 0) bytes += (uint32_t)(n1r + n2r) * ps * 8u;
+      int r = 0;
+      for (int s = sym ? 0 : pass; s < (sym ? fb.nl3 : pass + 1); ++s) {
+        const int l3 = fb.l3min + 2 * s;
+        r += sym ? l3 + 1 : 2 * l3 + 1;
+      }
+      bytes += (uint32_t)r * c3row * 16u;
+      mbar_expect_tx(&s_bar, bytes);
+      if (pass == 0) {
+        bulk_load(C1 + 3 * ps, ctp + (size_t)fb.c1 * ps, (uint32_t)n1r * ps * 8u, &s_bar);
+        bulk_load(C2 + 3 * ps, ctp + (size_t)fb.c2 * ps, (uint32_t)n2r * ps * 8u, &s_bar);
+      }
+      bulk_load(W, wtab + g.z, (uint32_t)g.w * 16u, &s_bar);
+      r = 0;
+      for (int s = sym ? 0 : pass; s < (sym ? fb.nl3 : pass + 1); ++s) {
+        const int l3 = fb.l3min + 2 * s, cnt = sym ? l3 + 1 : 2 * l3 + 1;
+        const int c0 = coff[l3 >> 1] + (sym ? l3 : 0);
+        bulk_load(C3 + (size_t)r * c3row, c3g + (size_t)c0 * c3row, (uint32_t)cnt * c3row * 16u, &s_bar);
+        r += cnt;
+      }
+    }
+    for (int i = threadIdx.x; i < g.y; i += blockDim.x) s_quads[i] = quads[g.x + i];
+    __syncthreads();
+    V.nq = g.y;
+    if (!mbar_wait(&s_bar, pass & 1, &s_abort, err)) {
+      mbar_wait_limit(&s_bar, pass & 1, kTimeoutCycles, err);  // copies still in flight land before the exit
+      return;
+    }
+    const int nrun = sym ? (fb.nl3 + kLaneNC - 1) / kLaneNC : 1;
+    for (;;) {
+      int t = 0;
+      if (lane == 0) t = atomicAdd(&s_next[pass], 1);
+      t = __shfl_sync(0xffffffffu, t, 0) * gridDim.z + blockIdx.z;
+      const int u = t / nrun;
+      if (u >= nu) break;
+      int s_lo = pass, w = 1;
+      if (sym) {  // balanced runs of orders
+        const int lo = fb.nl3 / nrun, ex = fb.nl3 - lo * nrun;
+        t -= u * nrun;
+        s_lo = t * lo + min(t, ex);
+        w = lo + (t < ex ? 1 : 0);
+      }
+      const uint32_t e = utab[ko.x + u * 34 + lane];  // the lane's shell pair, see build_lane_units
+      const uint32_t s0 = utab[ko.x + u * 34 + 32], s1 = utab[ko.x + u * 34 + 33];
+      V.C3 = smem_u32(C3 + 8 * (s1 >> 17));
+      lane_task<kLaneNC, PS, 8 * PS>(V, fb.swap, sym, fb.l3min, s_lo, w, fb.lt_base, (s1 >> 16) & 1, (int)e & 63,
+                                     (int)(e >> 6) & 63, (int)(e >> 24), (int)(e >> 12) & 0xfff, (int)(s1 & 0xffff), stage,
+                                     slots + s0, out);
+      __syncwarp();
+    }
+  }
+}
+
+// (float)x by integer arithmetic: FP64 conversions, like all FP64 arithmetic, run at a few
+// lanes per clock and SM.  Round to nearest even; subnormal and non-finite results go through
+// the conversion.
+__device__ __forceinline__ float narrow(const double x) {
+  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+  const int e = (int)((hi >> 20) & 0x7ff) - 1023 + 127;
+  if (e >= 1 && e <= 254) {
+    const uint32_t m = ((hi & 0xfffff) << 3) | (lo >> 29), rem = lo & 0x1fffffff;
+    const uint32_t up = rem > 0x10000000u || (rem == 0x10000000u && (m & 1)) ? 1u : 0u;
+    return __uint_as_float((hi & 0x80000000u) | (((uint32_t)e << 23) + m + up));
+  }
+  return ((hi << 1) | lo) == 0 ? __uint_as_float(hi & 0x80000000u) : (float)x;
+}
+
+__device__ __forceinline__ double flip(const double x, bool neg) {
+  return neg ? __hiloint2double(__double2hiint(x) ^ (int)0x80000000, __double2loint(x)) : x;
+}
+
+// Coefficients for the lane-owned coupling: one CTA per proposal reads the FP64 values once
+// (each warp one shell at a time, all of its loads in flight together), checks the
+// real-function relation c[l,-m] = (-1)^m conj c[l,m] to 1e-10 of the shell's largest
+// coefficient, and writes two FP32 layouts with the shells contiguous: ct [nc][ps] (c_k1 and
+// c_k2) and c3p [nc][c3row] (c_k3: four real parts, four imaginary parts per quad of shells).
+// sym = 1 when every shell satisfies the relation; m < 0 is then rebuilt from m >= 0 so that
+// it holds exactly in FP32.  keep: all shells stay in shared memory between the check and the
+// conversion (else they are read again).  grid: n; block 1024.
+// Bound by the latency of one round of loads and the stores of one SM.  FP64 arithmetic is
+// kept for shells that hold the relation only approximately: with it everywhere (as in
+// k_gather_sym) a proposal of K = 26, L = 18 took 33 us.
+__global__ void __launch_bounds__(1024, 1) k_gather_lane(int K, int nc, int ncoef, const int* __restrict__ csean,
+                                                         const int* __restrict__ cm, const int* __restrict__ cmir,
+                                                         const int* __restrict__ cl, const double2* __restrict__ coeff,
+                                                         float2* __restrict__ ct, float* __restrict__ c3p, int ps,
+                                                         int c3row, int* __restrict__ sym, int keep,
+                                                         const RagInfo* __restrict__ rag) {
+  extern __shared__ __align__(16) double2 gl_smem[];
+  const int prop = blockIdx.x;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const int ld = nc | 1;
+  const double2* cp = coeff + (size_t)prop * K * ncoef;
+  int ok = 1;
+  for (int k = warp; k < K; k += nw) {
+    double2* row = gl_smem + (size_t)(keep ? k : warp) * ld;
+    const double2* ck = cp + (size_t)k * ncoef;
+#pragma unroll 8
+    for (int c = lane; c < nc; c += 32) row[c] = ck[csean[c]];
+    __syncwarp();
+    // exact, finite mirror images need no tolerance
+    bool exact = true;
+    for (int c = lane; c < nc; c += 32) {
+      const int m = cm[c];
+      if (m < 0) continue;
+      const double2 a = row[c];
+      if (m == 0) {
+        exact &= ((__double_as_longlong(a.y) << 1) == 0);
+      } else {
+        const double2 b = row[cmir[c]];
+        const bool odd = m & 1;
+        exact &= __double_as_longlong(b.x) == __double_as_longlong(flip(a.x, odd)) &&
+                 __double_as_longlong(b.y) == __double_as_longlong(flip(a.y, !odd)) &&
+                 (__double2hiint(a.x) & 0x7ff00000) != 0x7ff00000 && (__double2hiint(a.y) & 0x7ff00000) != 0x7ff00000;
+      }
+    }
+    if (!__all_sync(0xffffffffu, exact)) {
+      double amax = 0.0;
+      for (int c = lane; c < nc; c += 32) amax = fmax(amax, fabs(row[c].x) + fabs(row[c].y));
+      for (int o = 16; o > 0; o >>= 1) amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+      const double tol = 1e-10 * amax;
+      for (int c = lane; c < nc; c += 32) {
+        const int m = cm[c];
+        if (m < 0) continue;
+        const double2 a = row[c];
+        if (m == 0) {
+          ok &= fabs(a.y) <= tol;
+        } else {
+          const double2 b = row[cmir[c]];
+          const double sg = (m & 1) ? -1.0 : 1.0;
+          ok &= fabs(b.x - sg * a.x) + fabs(b.y + sg * a.y) <= tol;
+        }
+      }
+    }
+    __syncwarp();
+  }
+  const int s = __syncthreads_and(ok);
+  if (threadIdx.x == 0) sym[prop] = s;
+  int Lp = 1 << 30, Kp = K;
+  if (rag) { Lp = rag[prop].L; Kp = rag[prop].K; }
+  float2* ctp = ct + (size_t)prop * nc * ps;
+  float* c3o = c3p + (size_t)prop * nc * (4 * c3row);
+  for (int c = warp; c < nc; c += nw) {
+    const int m = cm[c];
+    const bool mir = s && m < 0, odd = m & 1;
+    const int cs = mir ? cmir[c] : c;
+    const bool absent = cl[c] > Lp;
+    for (int k = lane; k < ps; k += 32) {
+      float2 v = make_float2(0.f, 0.f);  // absent orders / shells
+      if (!absent && k < Kp) {
+        const double2 a = keep ? gl_smem[(size_t)k * ld + cs] : cp[(size_t)k * ncoef + csean[cs]];
+        v = make_float2(narrow(flip(a.x, mir && odd)), (s && m == 0) ? 0.f : narrow(flip(a.y, mir && !odd)));
+      }
+      ctp[(size_t)c * ps + k] = v;
+      if (m >= 0 || !s) {
+        float* o = c3o + (size_t)c * (4 * c3row) + 8 * (k >> 2) + (k & 3);
+        o[0] = v.x;
+        o[4] = v.y;
+      }
+    }
+  }
+}
+
+// FP32 T [lt][ki] of a proposal -> the TF32 split operand's rows [ki][lt] (hi, lo), 32 x 32
+// tiles through shared memory.  grid: (klp / 32, lt tiles, n); block (32, 8).
+// Memory-bound: 6.6 MB read (mostly L2) and 13.6 MB written a proposal at L = 18, K = 26.
+// Writing these rows from the coupling itself costs a sector per value and array.
+__global__ void __launch_bounds__(256) k_split_rows(const float* __restrict__ T, int n_lt, int klp, int KP, int ldT32,
+                                                    float* __restrict__ hi, float* __restrict__ lo) {
+  __shared__ float tile[32][33];
+  const int ki0 = blockIdx.x * 32, lt0 = blockIdx.y * 32;
+  const float* src = T + (size_t)blockIdx.z * klp * ldT32;
+  for (int r = threadIdx.y; r < 32; r += 8)
+    if (lt0 + r < n_lt) tile[r][threadIdx.x] = src[(size_t)(lt0 + r) * klp + ki0 + threadIdx.x];
+  __syncthreads();
+  const int lt = lt0 + threadIdx.x;
+  if (lt >= n_lt) return;
+  for (int r = threadIdx.y; r < 32; r += 8) {
+    const float t = tile[threadIdx.x][r];
+    uint32_t h;
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h) : "f"(t));
+    const size_t at = ((size_t)blockIdx.z * klp + ki0 + r) * KP + lt;
+    hi[at] = __uint_as_float(h);
+    lo[at] = t - __uint_as_float(h);
+  }
+}
+
+constexpr int kGatherMaxSmem = 200 * 1024;
+
+}  // namespace
+
+// ---- host side ----------------------------------------------------------------
+
+std::string build_lane_tables(const std::vector<PairBlock>& pbs, const std::vector<int>& coff, const Wigner3jTable& w3j,
+                              std::vector<LaneBlock>& blks, std::vector<LaneQuad>& quads, std::vector<int4>& gcols,
+                              std::vector<float4>& w, int& crows, int& wmax, int& c3rows) {
+  blks.clear(); quads.clear(); gcols.clear(); w.clear();
+  crows = wmax = c3rows = 0;
+  // blocks of one loop form together (c_k2 stepped, then c_k1), each heaviest first as given
+  std::vector<PairBlock> ord;
+  for (int pass = 0; pass < 2; ++pass)
+    for (const PairBlock& pb : pbs)
+      if ((pb.l1 > pb.l2) == (pass == 0)) ord.push_back(pb);
+  for (const PairBlock& pb : ord) {
+    const int l1 = pb.l1, l2 = pb.l2;
+    LaneBlock fb{};
+    fb.l1 = l1; fb.l2 = l2; fb.l3min = pb.l3min; fb.nl3 = pb.nl3; fb.lt_base = pb.lt_base;
+    fb.c1 = coff[l1 >> 1]; fb.c2 = coff[l2 >> 1];
+    // steps run over the m of the shorter row, the other row slides with m3
+    fb.swap = l1 > l2;
+    const int a = std::min(l1, l2), b = std::max(l1, l2);
+    // one quad (m3 .. m3 + 3), orders s0 .. nl3 - 1 (or only s0): rows and 3j values
+    auto add = [&](int m3, int s0, int s1) {
+      LaneQuad q{};
+      q.m3 = m3;
+      q.c0 = s0;
+      q.rs = s1 - s0;
+      int lo = std::max(-a, -b - m3 - 3), hi = std::min(a, b - m3);
+      if ((hi - lo) & 1) ++hi;  // an odd number of steps (the form of the loop); the extra one is zero
+      q.n = hi - lo + 1;
+      // without swap: m1 = lo .. hi, window row k holds c_k2[-(m3 + k) - m1]; with swap: m2 =
+      // hi .. lo, window row k holds c_k1[-(m3 + 3 - k) - m2].  Arrays start at row 3.
+      q.x0 = (fb.swap ? hi + l2 : lo + l1) + 3;
+      q.vb = (fb.swap ? -(m3 + 3) - hi + l1 : -m3 - lo + l2) + 3;
+      q.wofs = 0;
+      for (int i = 0; i < q.n; ++i)
+        for (int s = s0; s < s1; ++s) {
+          const int l3 = pb.l3min + 2 * s;
+          float v[4];
+          for (int k = 0; k < 4; ++k) {
+            const int mm3 = m3 + k;
+            const int m1 = fb.swap ? -mm3 - (hi - i) : lo + i, m2 = -mm3 - m1;
+            const bool in = std::abs(mm3) <= l3 && std::abs(m1) <= l1 && std::abs(m2) <= l2;
+            v[k] = in ? (float)w3j(l1, l2, l3, m1, m2, mm3) : 0.f;
+          }
+          w.push_back(make_float4(v[0], v[1], v[2], v[3]));
+        }
+      quads.push_back(q);
+      return q.n * q.rs;
+    };
+    auto fits = [&](const LaneQuad& q) {
+      const int xl = fb.swap ? 2 * l2 + 7 : 2 * l1 + 7, vl = fb.swap ? 2 * l1 + 7 : 2 * l2 + 7;
+      const int sx = fb.swap ? -1 : 1, sv = -sx;
+      const int x1 = q.x0 + sx * (q.n - 1), v1 = q.vb + sv * (q.n + 2);
+      return q.n >= 1 && std::min(q.x0, x1) >= 0 && std::max(q.x0, x1) < xl && std::min(q.vb, v1) >= 0 &&
+             std::max(q.vb, v1) < vl;
+    };
+    const int l3max = pb.l3min + 2 * (pb.nl3 - 1);
+    fb.q0 = (int)quads.size();
+    fb.w0 = (int)w.size();
+    int run = 0, rows = 0;
+    for (int m3 = 0; m3 <= l3max; m3 += 4) {
+      int s0 = 0;
+      while (pb.l3min + 2 * s0 < m3) ++s0;
+      const int len = add(m3, s0, pb.nl3);
+      quads.back().wofs = run;
+      run += len;
+      if (!fits(quads.back())) return "lane tables: a quad leaves the staged rows";
+    }
+    fb.nq = (int)quads.size() - fb.q0;
+    fb.wn = run;
+    wmax = std::max(wmax, run);
+    if (fb.nq > kLaneMaxQuads) return "lane tables: more quads than the kernel stages";
+    for (int s = 0; s < 16; ++s) {
+      int4 g = make_int4((int)quads.size(), 0, (int)w.size(), 0);
+      if (s < pb.nl3) {
+        const int l3 = pb.l3min + 2 * s;
+        int r = 0;
+        for (int m3 = -((l3 + 3) / 4) * 4; m3 <= l3; m3 += 4) {
+          const int len = add(m3, s, s + 1);
+          quads.back().wofs = r;
+          r += len;
+          if (!fits(quads.back())) return "lane tables: a quad leaves the staged rows";
+          ++g.y;
+        }
+        g.w = r;
+        wmax = std::max(wmax, r);
+        if (g.y > kLaneMaxQuads) return "lane tables: more quads than the kernel stages";
+        rows += l3 + 1;
+        c3rows = std::max(c3rows, 2 * l3 + 1);
+      }
+      gcols.push_back(g);
+    }
+    c3rows = std::max(c3rows, rows);
+    crows = std::max(crows, 2 * b + 7);
+    blks.push_back(fb);
+  }
+  return "";
+}
+
+// Units of every K' <= K: (offset in utab, units) in kofs[K'], 34 entries a unit: per lane
+// shells of the block | staging offset | k2 | k1 (bits 24, 12, 6, 0; no shells: no pair), then
+// the first slot and slots | (more than eight shells) << 16 | k3 block << 17.  A slot is two
+// staging positions: half the even shell triple's index << 2 | which of the two are the unit's.
+void build_lane_units(int K, std::vector<uint32_t>& utab, std::vector<uint32_t>& slots, std::vector<int2>& kofs,
+                      int& stage) {
+  utab.clear(); slots.clear();
+  kofs.assign(K + 1, make_int2(0, 0));
+  stage = kLaneNC * 64;  // the m3 = 0 values of a task
+  for (int Kp = 1; Kp <= K; ++Kp) {
+    kofs[Kp].x = (int)utab.size();
+    for (int blk = 0; 16 * blk < Kp; ++blk) {
+      std::vector<std::pair<int, int>> pr;  // (k1, k2)
+      for (int k2 = Kp - 1; k2 >= 16 * blk; --k2)
+        for (int k1 = k2; k1 < Kp; ++k1) pr.push_back({k1, k2});
+      for (int p0 = 0; p0 < (int)pr.size(); p0 += 32, ++kofs[Kp].y) {
+        const int n = std::min(32, (int)pr.size() - p0);
+        auto shells = [&](int i) { return std::min(16, pr[p0 + i].second + 1 - 16 * blk); };
+        std::vector<int> order(n), off(n);
+        for (int i = 0; i < n; ++i) order[i] = i;
+        std::sort(order.begin(), order.end(), [&](int a, int b) { return pr[p0 + a] < pr[p0 + b]; });
+        const size_t s0 = slots.size();
+        int pos = 0, next = -1, used[32] = {0};
+        for (int i : order) {
+          const int k1 = pr[p0 + i].first, k2 = pr[p0 + i].second;
+          const int ki0 = k1 * (k1 + 1) * (k1 + 2) / 6 + k2 * (k2 + 1) / 2 + 16 * blk;
+          if (ki0 != next) {
+            pos = ((pos + 1) & ~1) + (ki0 & 1);
+            int best = pos;
+            for (int d = 2; d <= 8; d += 2)
+              if (used[(pos + d) & 31] < used[best & 31]) best = pos + d;
+            while (s0 + best / 2 > slots.size()) slots.push_back(0);
+            pos = best;
+          }
+          ++used[pos & 31];
+          off[i] = pos;
+          next = ki0 + shells(i);
+          for (int ki = ki0; ki < next; ++ki, ++pos) {
+            if (s0 + pos / 2 == slots.size()) slots.push_back((uint32_t)(ki / 2) << 2);
+            slots[s0 + pos / 2] |= 1u << (ki & 1);
+          }
+        }
+        const int ns = (int)(slots.size() - s0);
+        stage = std::max(stage, 2 * ns);
+        for (int i = 0; i < 32; ++i)
+          utab.push_back(i < n ? (uint32_t)shells(i) << 24 | (uint32_t)off[i] << 12 | (uint32_t)pr[p0 + i].second << 6 |
+                                     (uint32_t)pr[p0 + i].first
+                               : 0u);
+        utab.push_back((uint32_t)s0);
+        utab.push_back((uint32_t)ns | (shells(0) > 8 ? 1u << 16 : 0u) | (uint32_t)blk << 17);
+      }
+    }
+  }
+  stage = (stage + 3) / 4 * 4;
+}
+
+size_t lane_smem_bytes(const LaneTables& lt, int nw) {
+  return (size_t)2 * lt.crows * lt.ps * 8 + ((size_t)lt.wmax + 8) * 16 + (size_t)lt.c3rows * lt.c3row * 16 +
+         (size_t)nw * lt.stage * 4;
+}
+
+// Tasks of a block of nl3 orders (real functions) and nu units.
+int lane_tasks(int nu, int nl3) { return nu * ((nl3 + kLaneNC - 1) / kLaneNC); }
+
+// Warps per CTA: registers hold 16 warps per SM (128 a thread), so the split into CTAs that
+// brings most of them together; on a tie the smaller CTA, whose idle tail and staging wait the
+// SM's other CTAs cover.
+void lane_pick_warps(LaneTables& lt) {
+  lt.nw = 0;
+  int best = 0;
+  for (int nw : {4, 8, 16}) {
+    const size_t b = lane_smem_bytes(lt, nw) + 2048;
+    if (b > (size_t)kCoupleMaxDynSmem) continue;
+    const int ctas = (int)std::min<size_t>(kLaneMaxWarps / nw, (size_t)(228 * 1024) / b);
+    if (ctas * nw > best) { best = ctas * nw; lt.nw = nw; lt.ctas = ctas; }
+  }
+  lt.ok = lt.nw > 0;
+  lt.smem = lt.ok ? lane_smem_bytes(lt, lt.nw) : 0;
+}
+
+cudaError_t lane_configure() {
+  cudaError_t e = cudaFuncSetAttribute(k_couple_lane<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCoupleMaxDynSmem);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_couple_lane<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCoupleMaxDynSmem);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_gather_lane, cudaFuncAttributeMaxDynamicSharedMemorySize, kGatherMaxSmem);
+  return e;
+}
+
+cudaError_t launch_gather_lane(const DevTables& t, const TcTables& tc, int n, const double2* coeff, CoeffLayout lay,
+                               float2* ct, float* c3p, int* sym, cudaStream_t s, const RagInfo* rag) {
+  const size_t row = (size_t)(t.nc | 1) * sizeof(double2);
+  const bool keep = row * t.K <= (size_t)kGatherMaxSmem;
+  int nw = std::min(32, t.K);
+  if (!keep) nw = (int)std::min<size_t>(nw, kGatherMaxSmem / row);
+  nw = std::max(nw, 8);
+  const size_t smem = row * (keep ? t.K : nw);
+  k_gather_lane<<<n, nw * 32, smem, s>>>(t.K, t.nc, lay.stride, lay.map, tc.cm, tc.cmir, tc.cl, coeff, ct, c3p,
+                                         tc.lane.ps, tc.lane.c3row, sym, keep ? 1 : 0, rag);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_couple_lane(const DevTables& t, const TcTables& tc, int n, const float2* ct, const float* c3p,
+                               const int* sym, void* Thi, void* Tlo, bool tf32, float* T32, bool t32maj, float* scratch,
+                               cudaStream_t s, const RagInfo* rag) {
+  const LaneTables& lt = tc.lane;
+  // a batch whose (block, proposal) CTAs do not fill the SMs twice over spreads each block's
+  // tasks over Z CTAs, down to one task per warp
+  const int slots = 2 * tc.nsm * lt.ctas;
+  int z = 1;
+  while (z < lt.maxz && (long long)tc.n_pb * n * z < slots) ++z;
+  // TF32 rows are split from order-major FP32 T by a kernel of its own
+  const bool rows = tf32 && Thi && !T32;
+  LaneOut o;
+  o.hi = rows ? nullptr : Thi;
+  o.lo = rows ? nullptr : Tlo;
+  o.T32 = rows ? scratch : T32;
+  o.KP = tc.KP; o.klp = t.klp; o.ldT32 = t.n_ltp;
+  o.tf32 = tf32; o.ltmaj = t_order_major(tc, tf32); o.t32maj = rows || t32maj;
+  auto go = [&](auto kernel) {
+    kernel<<<dim3(n, tc.n_pb, z), 32 * lt.nw, lt.smem, s>>>(
+        ct, reinterpret_cast<const float4*>(c3p), t.K, t.nc, tc.coff, lt.blks, lt.quads, lt.gcols, lt.w, lt.utab, lt.slots,
+        lt.kofs, lt.crows, lt.wmax, lt.c3rows, lt.stage, sym, o, rag, tc.err);
+  };
+  if (lt.ps == 32)
+    go(k_couple_lane<32>);
+  else
+    go(k_couple_lane<64>);
+  if (rows)
+    k_split_rows<<<dim3(t.klp / 32, (t.n_lt + 31) / 32, n), dim3(32, 8), 0, s>>>(scratch, t.n_lt, t.klp, tc.KP, t.n_ltp,
+                                                                                 (float*)Thi, (float*)Tlo);
+  return cudaGetLastError();
+}
+
+}  // namespace tp3

@@ -256,6 +256,22 @@ int seanindex0(int l, int m, int LMAX) {
   return (bigL * (bigL + 3)) / 2 + 1 + ((bigL + m) * (bigL + m + 1)) / 2 + (l - std::abs(m));
 }
 
+Wigner3jTable::Wigner3jTable(const Basis& b) : nl_(b.nl), at_((size_t)b.nl * b.nl * b.nl, -1) {
+  for (int t = 0; t < b.n_lt(); ++t) {
+    const int l1 = b.lt_l1[t], l2 = b.lt_l2[t], l3 = b.lt_l3[t], at = (int)v_.size();
+    at_[((size_t)(l1 / 2) * nl_ + l2 / 2) * nl_ + l3 / 2] = at;
+    v_.resize(v_.size() + (size_t)(2 * l1 + 1) * (2 * l2 + 1), 0.0);
+    for (int j = b.lt_jstart[t]; j < b.lt_jstart[t] + b.lt_jcount[t]; ++j)
+      v_[at + (size_t)(b.m1[j] + l1) * (2 * l2 + 1) + b.m2[j] + l2] = b.w[j];
+  }
+}
+
+double Wigner3jTable::operator()(int l1, int l2, int l3, int m1, int m2, int m3) const {
+  if (m1 + m2 + m3 != 0 || std::abs(m1) > l1 || std::abs(m2) > l2 || std::abs(m3) > l3) return 0.0;
+  const int at = at_[((size_t)(l1 / 2) * nl_ + l2 / 2) * nl_ + l3 / 2];
+  return at < 0 ? 0.0 : v_[at + (size_t)(m1 + l1) * (2 * l2 + 1) + m2 + l2];
+}
+
 std::string build_basis(Basis& b, int L, int LMAX, int N, int K, double lambda, double dq) {
   if (L < 0 || L > 64) return "L out of range (0..64)";
   if (LMAX < L + 1) return "LMAX must be >= L+1: a bandwidth-LMAX coefficient vector holds l <= LMAX-1";

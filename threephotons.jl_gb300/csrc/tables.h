@@ -72,6 +72,18 @@ struct Basis {
 // Enumerate the basis and index tables.  Returns "" on success or an error text.
 std::string build_basis(Basis& b, int L, int LMAX, int N, int K, double lambda, double dq);
 
+// 3j symbols (l1 l2 l3; m1 m2 m3) of a basis' entries by their indices, so that the tables
+// derived from a basis do not evaluate the exact sum again (absent entries are zero).
+struct Wigner3jTable {
+  explicit Wigner3jTable(const Basis& b);
+  double operator()(int l1, int l2, int l3, int m1, int m2, int m3) const;
+
+ private:
+  int nl_;
+  std::vector<int> at_;     // [nl][nl][nl] first value of an l-triple, -1 without entries
+  std::vector<double> v_;   // per l-triple [2 l1 + 1][2 l2 + 1]
+};
+
 // Decide and build the grid fold.  At lambda = 0 every Legendre factor is taken at
 // theta = pi/2, where sphPlm(l, m) vanishes for odd l + m; with even l only even
 // m survive, so c3(alpha, beta) = c3(alpha, beta + pi) = c3(pi - alpha, pi - beta).
