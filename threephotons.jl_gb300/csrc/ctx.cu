@@ -375,6 +375,13 @@ std::string setup_tc(tp3_ctx* c) {
       Fhi32[(size_t)u * tc.KP + l] = h32;
       Flo32[(size_t)u * tc.KP + l] = (float)(v64 - (double)h32);
     }
+  std::vector<tp3::SlabLog> logtab(128);
+  for (int i = 0; i < 128; ++i) {
+    const double inv = (double)(1.0L / (1.0L + (i + 0.5L) / 128.0L));
+    const long double lc = -std::log((i < 64 ? 1 : 2) * (long double)inv);
+    const double hi = (double)(std::nearbyint(lc * 0x1p42L) * 0x1p-42L);
+    logtab[i] = {inv, hi, (double)(lc - hi)};
+  }
   void* fn = nullptr;
   cudaDriverEntryPointQueryResult q;
   if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q) != cudaSuccess ||
@@ -392,7 +399,7 @@ std::string setup_tc(tp3_ctx* c) {
       (e = upload(c, units_sym, &tc.units_sym)) != cudaSuccess ||
       (e = upload(c, units_gen, &tc.units_gen)) != cudaSuccess ||
       (e = upload(c, Fhi, &tc.Fhi)) != cudaSuccess || (e = upload(c, Flo, &tc.Flo)) != cudaSuccess ||
-      (e = upload(c, Fhi32, &tc.Fhi32)) != cudaSuccess || (e = upload(c, Flo32, &tc.Flo32)) != cudaSuccess ||
+      (e = upload(c, Fhi32, &tc.Fhi32)) != cudaSuccess || (e = upload(c, logtab, &tc.logtab)) != cudaSuccess || (e = upload(c, Flo32, &tc.Flo32)) != cudaSuccess ||
       (e = tp3::tc_configure()) != cudaSuccess)
     return std::string("tensor-core table upload: ") + cudaGetErrorString(e);
   // folded-row coupling: three tilings in up to 225 KB, one CTA per SM (8 warps; 7 warps,
@@ -652,7 +659,7 @@ int run_energy(tp3_ctx* c, int n, const double2* d_coeff, double* d_E, bool comp
                                               rag)) != cudaSuccess)
         return cuda_fail(c, e, "angular_persistent");
       if (pr) cudaEventRecord(b, c->stream);
-      if ((e = tp3::launch_finalize_parts(t, c->tc, n, part, Qf, c->d_Eslab, d_E, c->stream, rag)) != cudaSuccess)
+      if ((e = tp3::launch_finalize_parts(t, c->tc, n, part, Qf, d_E, c->stream, rag)) != cudaSuccess)
         return cuda_fail(c, e, "finalize_parts");
     } else {
       if ((e = tp3::launch_angular_tc(t, c->tc, tf ? c->maps32 : c->maps, n, qt, Qf, c->d_Eslab, nullptr, c->d_err,
@@ -673,13 +680,12 @@ int run_energy(tp3_ctx* c, int n, const double2* d_coeff, double* d_E, bool comp
   return TP3_OK;
 }
 
-// After a synchronising call: report a device-side timeout, if any.
+// After a synchronising call: report a device-side timeout, if any.  The flag is host memory
+// that kernels write only on an error, so reading it costs no copy.
 int check_device_error(tp3_ctx* c) {
-  cudaError_t e = cudaMemcpy(c->h_err, c->d_err, sizeof(int), cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return cuda_fail(c, e, "error flag read");
-  if (*c->h_err != 0) {
-    const int code = *c->h_err;
-    cudaMemset(c->d_err, 0, sizeof(int));
+  const int code = *(volatile int*)c->h_err;
+  if (code != 0) {
+    *(volatile int*)c->h_err = 0;
     return fail(c, code, code == TP3_ERR_TIMEOUT ? "a bounded device wait ran out; results of this call are invalid"
                          : code == TP3_ERR_BOUNDS
                              ? "a device index check of the TP3_DEBUG build failed (the access was skipped); results "
@@ -985,12 +991,13 @@ int tp3_ctx_create(int L, int LMAX, int N, int K, double lambda, double dq, tp3_
       (e = upload(c, qstart, &t.qstart)) != cudaSuccess || (e = upload(c, qlist, &t.qlist)) != cudaSuccess ||
       (e = upload(c, qent, &t.qent)) != cudaSuccess ||
       (e = upload(c, Cq, &t.Cq)) != cudaSuccess ||
-      (e = cudaMalloc(&c->d_err, sizeof(int))) != cudaSuccess || (e = cudaMemset(c->d_err, 0, sizeof(int))) != cudaSuccess ||
-      (e = cudaMallocHost(&c->h_err, sizeof(int))) != cudaSuccess) {
+      (e = cudaHostAlloc(&c->h_err, sizeof(int), cudaHostAllocMapped)) != cudaSuccess ||
+      (e = cudaHostGetDevicePointer(&c->d_err, c->h_err, 0)) != cudaSuccess) {
     std::string msg = std::string("table upload: ") + cudaGetErrorString(e);
     tp3_ctx_destroy(c);
     return fail(nullptr, TP3_ERR_CUDA, msg);
   }
+  *c->h_err = 0;
   c->tc.err = c->d_err;  // device error flag of the TP3_DEBUG index checks
   c->tc_why = setup_tc(c);
   c->tc_ok = c->tc_why.empty();
@@ -1008,7 +1015,6 @@ void tp3_ctx_destroy(tp3_ctx* c) {
   for (void* p : c->allocs) cudaFree(p);
   cudaFree(c->d_qfull); cudaFree(c->d_Qfull); cudaFree(c->d_qt); cudaFree(c->d_Qfold); cudaFree(c->d_c3);
   cudaFree(c->d_qt_set); cudaFree(c->d_Qf_set); cudaFree(c->d_rag);
-  cudaFree(c->d_err);
   cudaFreeHost(c->h_err);
   for (auto ev : c->ev) cudaEventDestroy(ev);
   for (auto ev : c->ev_c) cudaEventDestroy(ev);
@@ -1436,12 +1442,17 @@ int tp3_energy_batch(tp3_ctx* c, int n, const double* coeffs, double* E) {
   double2* dev = c->d_coeff;
   cudaError_t e;
   if (c->host_direct) {
-    // the device reads the caller's buffer in place: no host packing and no staging copy
-    const int64_t total = (int64_t)n * t.K * t.nc;
-    const int blocks = (int)std::min<int64_t>((total + 255) / 256, 65535);
-    k_stage_coeff<<<blocks, 256, 0, c->stream>>>(src, total, t.nc, (int)ncoef, t.csean, dev);
-    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(c, e, "stage coefficients");
-    if (int r = run_energy(c, n, dev, c->d_E, true)) return r;
+    // the device reads the caller's buffer in place: no host packing and no staging copy, and
+    // none on the device either where the gather reads every value once
+    if (is_tc(c->mode) && c->tc.use_lane && tp3::gather_lane_once(t)) {
+      if (int r = run_energy(c, n, src, c->h_E)) return r;
+    } else {
+      const int64_t total = (int64_t)n * t.K * t.nc;
+      const int blocks = (int)std::min<int64_t>((total + 255) / 256, 65535);
+      k_stage_coeff<<<blocks, 256, 0, c->stream>>>(src, total, t.nc, (int)ncoef, t.csean, dev);
+      if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(c, e, "stage coefficients");
+      if (int r = run_energy(c, n, dev, c->h_E, true)) return r;
+    }
   }
   for (int p0 = 0; p0 < n && !c->host_direct; p0 += per) {
     const int m = std::min(per, n - p0);
@@ -1457,11 +1468,10 @@ int tp3_energy_batch(tp3_ctx* c, int n, const double* coeffs, double* E) {
     if ((e = cudaMemcpyAsync(dev + off, pin + off, (size_t)m * t.K * t.nc * sizeof(double2), cudaMemcpyHostToDevice,
                              c->stream)) != cudaSuccess)
       return cuda_fail(c, e, "H2D coeff");
-    if (int r = run_energy(c, m, dev + off, c->d_E + p0, true)) return r;
+    if (int r = run_energy(c, m, dev + off, c->h_E + p0, true)) return r;
   }
-  if ((e = cudaMemcpyAsync(c->h_E, c->d_E, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream)) != cudaSuccess ||
-      (e = cudaStreamSynchronize(c->stream)) != cudaSuccess)
-    return cuda_fail(c, e, "D2H energy");
+  // the last kernel wrote the energies to pinned host memory
+  if ((e = cudaStreamSynchronize(c->stream)) != cudaSuccess) return cuda_fail(c, e, "energies");
   if (int r = check_device_error(c)) return r;
   std::memcpy(E, c->h_E, n * sizeof(double));
   return TP3_OK;

@@ -55,7 +55,7 @@ struct tp3_ctx {
   double* d_Eslab = nullptr;   // [cap][klength]         tensor-core path
   double* d_E = nullptr;       // [cap]
   float* d_c3 = nullptr;       // [klength][G] (one proposal)
-  int* d_err = nullptr;        // device error flag (timeouts)
+  int* d_err = nullptr;        // error flag (timeouts), the device's address of h_err
   int* d_sym = nullptr;        // [cap] real-function symmetry flag per proposal
   float2* d_ct = nullptr;      // [cap][nc][ps] coefficients, shells contiguous (lane-owned coupling)
   float* d_c3p = nullptr;      // [cap][nc][4 c3row] the same, real and imaginary parts of four shells apart
@@ -63,7 +63,7 @@ struct tp3_ctx {
   float* d_H = nullptr;        // [cap][klp][nqp] Fourier-pair operand (lambda != 0)
   double* h_coeff = nullptr;   // pinned [cap][K][LMAX^2][2]
   double* h_E = nullptr;       // pinned [cap]
-  int* h_err = nullptr;        // pinned
+  int* h_err = nullptr;        // mapped host memory
 
   // histogram set of ragged batches: [nhist][klp/128][Gu][128] and [nhist][klength]
   int nhist = 0;

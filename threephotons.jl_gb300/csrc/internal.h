@@ -127,6 +127,11 @@ struct FoldVariant {
   const int2* chunks = nullptr;
 };
 
+// One interval of the slab terms' logarithm: 1/c and log c in two parts, hi a multiple of 2^-42.
+struct SlabLog {
+  double inv, hi, lo;
+};
+
 // Lane-owned coupling (kernels_lane.cu): per pair block, quads of consecutive m3 with the 3j
 // values of their four m3 side by side.
 constexpr int kLaneMaxQuads = 20;
@@ -224,6 +229,7 @@ struct TcTables {
   const __nv_bfloat16* Flo = nullptr;
   const float* Fhi32 = nullptr;        // [NP][KP] TF32 hi (fp32 with the low 13 bits clear)
   const float* Flo32 = nullptr;        // [NP][KP] fp32 remainder
+  const SlabLog* logtab = nullptr;     // [128]
 };
 
 // Per-proposal limits of a ragged batch (chains of different L and K scored in one
@@ -258,13 +264,13 @@ cudaError_t launch_finalize_slabs(int n, int klength, const double* Eslab, doubl
                                   const RagInfo* rag = nullptr);
 // Persistent angular stage: compensated partial sums into part ([n][klp][4 nhalf] floats),
 // or (c3out) c3 rows [n][klength][2N^2];
-// launch_finalize_parts turns them into slab terms (Eslab [n][klength]) and sums those
-// per proposal in a fixed order.
+// launch_finalize_parts turns them into slab terms and sums those per proposal in a fixed
+// order.
 cudaError_t launch_angular_persistent(const DevTables& t, const TcTables& tc, const TcMaps& maps, int n,
                                       const float* qt, float* part, int* err, bool tf32, cudaStream_t s,
                                       const RagInfo* rag = nullptr, float* c3out = nullptr);
 cudaError_t launch_finalize_parts(const DevTables& t, const TcTables& tc, int n, const float* part, const double* Qs,
-                                  double* Eslab, double* E, cudaStream_t s, const RagInfo* rag = nullptr);
+                                  double* E, cudaStream_t s, const RagInfo* rag = nullptr);
 size_t couple_split_smem_d(const DevTables& t, const TcTables& tc);
 size_t couple_split_smem_t(const DevTables& t, const TcTables& tc);
 cudaError_t couple_split_configure(const DevTables& t, const TcTables& tc);
@@ -282,6 +288,7 @@ void build_lane_units(int K, std::vector<uint32_t>& utab, std::vector<uint32_t>&
 int lane_tasks(int nu, int nl3);
 void lane_pick_warps(LaneTables& lt);
 cudaError_t lane_configure();
+bool gather_lane_once(const DevTables& t);
 cudaError_t launch_gather_lane(const DevTables& t, const TcTables& tc, int n, const double2* coeff, CoeffLayout lay,
                                float2* ct, float* c3p, int* sym, cudaStream_t s, const RagInfo* rag = nullptr);
 // T32 (nullable): FP32 T as [ki][n_ltp] rows, or [lt][klp] when t32maj; Thi null: T32 only.

@@ -797,10 +797,13 @@ cudaError_t lane_configure() {
   return e;
 }
 
+// Whether the gather holds all shells of a proposal in shared memory, reading each value once.
+bool gather_lane_once(const DevTables& t) { return (size_t)(t.nc | 1) * sizeof(double2) * t.K <= (size_t)kGatherMaxSmem; }
+
 cudaError_t launch_gather_lane(const DevTables& t, const TcTables& tc, int n, const double2* coeff, CoeffLayout lay,
                                float2* ct, float* c3p, int* sym, cudaStream_t s, const RagInfo* rag) {
   const size_t row = (size_t)(t.nc | 1) * sizeof(double2);
-  const bool keep = row * t.K <= (size_t)kGatherMaxSmem;
+  const bool keep = gather_lane_once(t);
   int nw = std::min(32, t.K);
   if (!keep) nw = (int)std::min<size_t>(nw, kGatherMaxSmem / row);
   nw = std::max(nw, 8);

@@ -1040,29 +1040,94 @@ __global__ void __launch_bounds__(256) k_finalize_slabs(const double* __restrict
   if (threadIdx.x == 0) E[prop] = ss[0] + sc[0];
 }
 
-// grid: (ceil(klength / 256), n); block 256.  Slab terms tf (Qs log(mult Sp) - Sql) in
-// FP64 from the persistent kernel's partial sums [klp][nhalf][2][2] per proposal, one
-// thread per shell triple; k_finalize_slabs then adds them in its fixed order.
-__global__ void __launch_bounds__(256) k_slab_terms(const float* __restrict__ part, int klp, int klength, int nhalf,
-                                                    const double* __restrict__ Qs, const double* __restrict__ tf,
-                                                    int mult, double* __restrict__ Eslab,
-                                                    const RagInfo* __restrict__ rag) {
-  const int prop = blockIdx.y;
-  const int ki = blockIdx.x * blockDim.x + threadIdx.x;
+// log(x) of a positive normal double, table-driven (P. T. P. Tang, "Table-driven implementation
+// of the logarithm function in IEEE floating-point arithmetic", ACM TOMS 16 (1990)): x = 2^e m
+// with 0.75 <= m < 1.5, c the centre of m's interval (1/128 of its binade), r = m (1/c) - 1 with
+// one rounding, log x = e ln 2 + log c + log1p(r), |r| < 2^-8.  14 FP64 operations, a third of log(): FP64 runs at two lanes per
+// clock and SM here.  tab: 1/c and log c, built in extended precision.
+__device__ __forceinline__ double slab_log(const double x, const SlabLog* __restrict__ tab) {
+  const int hi = __double2hiint(x);
+  const int e = ((hi >> 20) & 0x7ff) - 1023;
+  if (e < -1022 || e > 1023 || hi < 0) return log(x);  // zero, subnormal, infinite, NaN, negative
+  const double m = __hiloint2double((hi & 0xfffff) | 0x3ff00000, __double2loint(x));
+  const int i = (hi >> 13) & 127;
+  const double inv = tab[i].inv, chi = tab[i].hi, clo = tab[i].lo;
+  const double r = fma(m, inv, -1.0), r2 = r * r;
+  double p = fma(r, 1.0 / 7.0, -1.0 / 6.0);
+  p = fma(p, r, 0.2);
+  p = fma(p, r, -0.25);
+  p = fma(p, r, 1.0 / 3.0);
+  p = fma(p, r, -0.5);
+  const double ed = (double)(e + (i >> 6));
+  constexpr double ln2_hi = 0x1.62e42fefa38p-1, ln2_lo = 0x1.ef35793c7673p-45;  // ln 2 to 41 + 53 bits
+  return fma(ed, ln2_hi, chi) + (r + fma(p, r2, fma(ed, ln2_lo, clo)));  // the first sum is exact
+}
+
+// Energies from the persistent kernel's partial sums [klp][nhalf][2][2] per proposal: slab terms
+// tf (Qs log(mult Sp) - Sql) in FP64 and their deterministic compensated sum, in one cluster of
+// kFinCtas CTAs per proposal (the first rag[prop].klen terms of a ragged batch).  The sum is that
+// of 256 accumulators, accumulator t taking the terms t, t + 256, .., and a tree over them; CTA r
+// owns accumulators 32 r .. 32 r + 31 and their terms, CTA 0 gathers them through distributed
+// shared memory.  Bound by FP64 (two lanes per clock and SM), hence several SMs a proposal: at
+// K = 26 one proposal took 6.5 + 15 us as a kernel of terms and a kernel of one CTA that summed.
+constexpr int kFinCtas = 8, kFinRows = 16;
+__global__ void __cluster_dims__(kFinCtas, 1, 1) __launch_bounds__(128)
+    k_finalize_parts(const float* __restrict__ part, int klp, int klength, int nhalf, const double* __restrict__ Qs,
+                     const double* __restrict__ tf, int mult, const SlabLog* __restrict__ logtab, double* __restrict__ E,
+                     const RagInfo* __restrict__ rag) {
+  __shared__ double term[kFinRows][32], ss[256], sc[256];
+  const int prop = blockIdx.y, rank = blockIdx.x, lane = threadIdx.x & 31;
   int nk = klength;
   if (rag) {
     nk = rag[prop].klen;
     Qs += (size_t)rag[prop].hist * klength;
   }
-  if (ki >= nk) return;
-  const float4* p4 = reinterpret_cast<const float4*>(part) + ((size_t)prop * klp + ki) * nhalf;
-  double Sp = 0.0, Sq = 0.0;
-  for (int h = 0; h < nhalf; ++h) {
-    const float4 a = p4[h];  // (Sp, Sql) of column blocks 0 and 1
-    Sp += (double)a.x + (double)a.z;
-    Sq += (double)a.y + (double)a.w;
+  const float4* p4 = reinterpret_cast<const float4*>(part) + (size_t)prop * klp * nhalf;
+  const int k0 = 32 * rank + lane;
+  double s = 0.0, c = 0.0;
+  for (int j0 = 0; 256 * j0 + 32 * rank < nk; j0 += kFinRows) {
+    for (int j = threadIdx.x >> 5; j < kFinRows; j += 4) {
+      const int ki = k0 + 256 * (j0 + j);
+      if (ki >= nk) break;
+      double Sp = 0.0, Sq = 0.0;
+      for (int h = 0; h < nhalf; ++h) {
+        const float4 a = p4[(size_t)ki * nhalf + h];  // (Sp, Sql) of column blocks 0 and 1
+        Sp += (double)a.x + (double)a.z;
+        Sq += (double)a.y + (double)a.w;
+      }
+      term[j][lane] = tf[ki] * (Qs[ki] * slab_log((double)mult * Sp, logtab) - Sq);
+    }
+    __syncthreads();
+    if (threadIdx.x < 32)
+      for (int j = 0; j < kFinRows && k0 + 256 * (j0 + j) < nk; ++j) {
+        double t, err;
+        two_sum(s, term[j][lane], t, err);
+        s = t;
+        c += err;
+      }
+    __syncthreads();
   }
-  Eslab[(size_t)prop * klength + ki] = tf[ki] * (Qs[ki] * log((double)mult * Sp) - Sq);
+  if (threadIdx.x < 32) {
+    const uint32_t as = smem_u32(&ss[k0]), ac = smem_u32(&sc[k0]);
+    asm volatile(
+        "{\n\t.reg .b32 a;\n\t"
+        "mapa.shared::cluster.u32 a, %0, 0;\n\tst.shared::cluster.f64 [a], %2;\n\t"
+        "mapa.shared::cluster.u32 a, %1, 0;\n\tst.shared::cluster.f64 [a], %3;\n\t}" ::"r"(as),
+        "r"(ac), "d"(s), "d"(c)
+        : "memory");
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (rank != 0) return;
+  for (int h = 128; h > 0; h >>= 1) {
+    if (threadIdx.x < h) {
+      double t, err;
+      two_sum(ss[threadIdx.x], ss[threadIdx.x + h], t, err);
+      ss[threadIdx.x] = t;
+      sc[threadIdx.x] += sc[threadIdx.x + h] + err;
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) E[prop] = ss[0] + sc[0];
 }
 
 }  // namespace
@@ -1243,12 +1308,8 @@ cudaError_t launch_angular_persistent(const DevTables& t, const TcTables& tc, co
 }
 
 cudaError_t launch_finalize_parts(const DevTables& t, const TcTables& tc, int n, const float* part, const double* Qs,
-                                  double* Eslab, double* E, cudaStream_t s, const RagInfo* rag) {
-  k_slab_terms<<<dim3((t.klength + 255) / 256, n), 256, 0, s>>>(part, t.klp, t.klength, tc.nhalf, Qs, t.tf, t.mult,
-                                                                 Eslab, rag);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  k_finalize_slabs<<<n, 256, 0, s>>>(Eslab, t.klength, E, rag);
+                                  double* E, cudaStream_t s, const RagInfo* rag) {
+  k_finalize_parts<<<dim3(kFinCtas, n), 128, 0, s>>>(part, t.klp, t.klength, tc.nhalf, Qs, t.tf, t.mult, tc.logtab, E, rag);
   return cudaGetLastError();
 }
 
