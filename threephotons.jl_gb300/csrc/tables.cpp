@@ -296,16 +296,27 @@ std::string build_basis(Basis& b, int L, int LMAX, int N, int K, double lambda, 
   b.nc = off;
   auto cidx = [&](int l, int m) { return b.coff[l / 2] + m + l; };
   const double thr = 100.0 * 2.220446049250313e-16;
+  // the exact 3j sums of every (l1, l2), in parallel; read back below in the same order
+  std::vector<std::vector<double>> w3(b.nl * b.nl);
+#pragma omp parallel for schedule(dynamic, 1)
+  for (int q = b.nl * b.nl - 1; q >= 0; --q) {
+    const int l1 = 2 * (q / b.nl), l2 = 2 * (q % b.nl);
+    for (int l3 = 0; l3 <= L; l3 += 2)
+      for (int mm1 = -l1; mm1 <= l1; ++mm1)
+        for (int mm2 = -l2; mm2 <= l2; ++mm2)
+          if (std::abs(mm1 + mm2) <= l3) w3[q].push_back(wigner3j(l1, l2, l3, mm1, mm2, -(mm1 + mm2)));
+  }
   int j = 0;
   for (int l1 = 0; l1 <= L; l1 += 2)
-    for (int l2 = 0; l2 <= L; l2 += 2)
+    for (int l2 = 0; l2 <= L; l2 += 2) {
+      const double* next = w3[(l1 / 2) * b.nl + l2 / 2].data();
       for (int l3 = 0; l3 <= L; l3 += 2) {
         int count = 0, start = j;
         for (int mm1 = -l1; mm1 <= l1; ++mm1)
           for (int mm2 = -l2; mm2 <= l2; ++mm2) {
             int mloop3 = mm1 + mm2;  // wigner(l1,m1,l2,m2,l3,-m3) needs m3 = m1 + m2
             if (std::abs(mloop3) > l3) continue;
-            double w = wigner3j(l1, l2, l3, mm1, mm2, -mloop3);
+            double w = *next++;
             if (std::fabs(w) > thr) {
               b.w.push_back(w);
               b.l1.push_back(l1); b.m1.push_back(mm1);
@@ -323,6 +334,7 @@ std::string build_basis(Basis& b, int L, int LMAX, int N, int K, double lambda, 
           b.lt_jstart.push_back(start); b.lt_jcount.push_back(count);
         }
       }
+    }
   for (int k1 = 0; k1 < K; ++k1)
     for (int k2 = 0; k2 <= k1; ++k2)
       for (int k3 = 0; k3 <= k2; ++k3) {
