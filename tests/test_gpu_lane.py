@@ -86,3 +86,25 @@ def test_lane_form_is_the_default():
     b.set_coupling(LANE)
     assert np.array_equal(T, b.triple_products(c))
     b.close()
+
+
+@pytest.mark.parametrize("L,LMAX,N,K,n", [(0, 1, 2, 1, 1), (2, 3, 4, 5, 4), (6, 7, 6, 8, 5), (10, 12, 8, 9, 9),
+                                          (12, 13, 10, 17, 13), (24, 25, 4, 6, 14)])
+def test_fourier_pair_operand_equals_entry_sums(L, LMAX, N, K, n):
+    """lambda != 0: H from mirrored entry pairs (lane form) against the sum over all entries
+    (pair form), batches on either side of 4, 8 and 12 proposals a CTA."""
+    b = tp3.calculate_basis(L, LMAX, N, K, 1.7, 0.05)
+    rng = np.random.default_rng(L)
+    b.set_histogram(rng.uniform(0.5, 1.5, size=(N, 2 * N, K, K, K)))
+    c = _coefficients(L, LMAX, K, n, True, L + 1)
+    if n > 1:
+        c[1] = _coefficients(L, LMAX, K, 1, False, L + 2)[0]
+    for mode in (tp3.TP3_MODE_TC_BF16X3, tp3.TP3_MODE_TC_TF32X3):
+        got = {}
+        b.set_mode(mode)
+        for form in (PAIR, LANE):
+            b.set_coupling(form)
+            got[form] = (b.c3_raw(c[0]), b.energy_batch(c))
+        for x, y in zip(got[PAIR], got[LANE]):
+            assert np.isfinite(x).all() and np.array_equal(x, y)
+    b.close()

@@ -591,7 +591,9 @@ int run_coupling(tp3_ctx* c, int n, const double2* d_coeff, bool want_T32, bool 
   cudaError_t e;
   const tp3::CoeffLayout lay = compact ? tp3::CoeffLayout{t.cident, t.nc} : tp3::CoeffLayout{t.csean, t.LMAX * t.LMAX};
   if (is_tc(c->mode)) {
-    // lambda != 0: the coupling also writes FP32 T, from which H (the angular operand) is built
+    // lambda != 0: H (the angular operand) is built from FP32 T, order-major after the lane-owned
+    // coupling, which then writes nothing else
+    const bool hpairs = c->tc.hform && c->tc.use_lane && c->tc.hf.ok && !want_T32;
     if (c->tc.hform) want_T32 = true;
     if (c->tc.use_lane) {
       if ((e = tp3::launch_gather_lane(t, c->tc, n, d_coeff, lay, c->d_ct, c->d_c3p, c->d_sym, c->stream, rag)) !=
@@ -602,9 +604,9 @@ int run_coupling(tp3_ctx* c, int n, const double2* d_coeff, bool want_T32, bool 
     cudaEvent_t ca, cb;
     const int pc = prof_begin_in(c, c->ev_c, c->ev_c_used, &ca, &cb);
     if (c->tc.use_lane)
-      e = tp3::launch_couple_lane(t, c->tc, n, c->d_ct, c->d_c3p, c->d_sym, c->d_Thi, c->d_Tlo,
-                                  c->mode == TP3_MODE_TC_TF32X3, want_T32 ? c->d_T : nullptr, false, c->d_T, c->stream,
-                                  rag);
+      e = tp3::launch_couple_lane(t, c->tc, n, c->d_ct, c->d_c3p, c->d_sym, hpairs ? nullptr : c->d_Thi,
+                                  hpairs ? nullptr : c->d_Tlo, c->mode == TP3_MODE_TC_TF32X3, want_T32 ? c->d_T : nullptr,
+                                  hpairs, c->d_T, c->stream, rag);
     else if (rag)  // ragged batches use the one-kernel coupling (it skips absent blocks and shells)
       e = tp3::launch_couple_pair(t, c->tc, n, c->d_cc, c->d_sym, c->d_Thi, c->d_Tlo, c->mode == TP3_MODE_TC_TF32X3,
                                   want_T32 ? c->d_T : nullptr, c->stream, rag);
@@ -615,7 +617,11 @@ int run_coupling(tp3_ctx* c, int n, const double2* d_coeff, bool want_T32, bool 
       e = tp3::launch_couple_pair(t, c->tc, n, c->d_cc, c->d_sym, c->d_Thi, c->d_Tlo, c->mode == TP3_MODE_TC_TF32X3,
                                   want_T32 ? c->d_T : nullptr, c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "coupling");
-    if (c->tc.hform && (e = tp3::launch_build_H_split(t, c->tc.KP, n, c->d_T, c->d_Thi, c->d_Tlo,
+    if (hpairs) {
+      if ((e = tp3::launch_build_H_pairs(t, c->tc, n, c->d_T, c->d_Thi, c->d_Tlo, c->mode == TP3_MODE_TC_TF32X3,
+                                         c->stream)) != cudaSuccess)
+        return cuda_fail(c, e, "build_H_pairs");
+    } else if (c->tc.hform && (e = tp3::launch_build_H_split(t, c->tc.KP, n, c->d_T, c->d_Thi, c->d_Tlo,
                                                       c->mode == TP3_MODE_TC_TF32X3, c->stream)) != cudaSuccess)
       return cuda_fail(c, e, "build_H_split");
     if (pc) cudaEventRecord(cb, c->stream);
@@ -998,6 +1004,27 @@ int tp3_ctx_create(int L, int LMAX, int N, int K, double lambda, double dq, tp3_
     return fail(nullptr, TP3_ERR_CUDA, msg);
   }
   *c->h_err = 0;
+  if (lambda != 0.0) {
+    tp3::HformTables& hf = c->tc.hf;
+    std::vector<int4> hg;
+    std::vector<int2> hl, he;
+    std::vector<float> hw;
+    std::vector<int> hm;
+    if (K <= 64 && tp3::hform_fits(t.n_lt, t.nc) &&
+        tp3::build_hform_tables(b.coff, K, t.n_lt, b.lt_l1.data(), b.lt_l2.data(), b.lt_l3.data(), c->qpairs, qstart, qlist,
+                                lt_of_j, w32, hg, hl, he, hw, hm)
+            .empty()) {
+      if ((e = upload(c, hg, &hf.groups)) != cudaSuccess || (e = upload(c, hl, &hf.lists)) != cudaSuccess ||
+          (e = upload(c, he, &hf.entries)) != cudaSuccess || (e = upload(c, hw, &hf.wts)) != cudaSuccess ||
+          (e = upload(c, hm, &hf.slot_m)) != cudaSuccess || (e = tp3::hform_configure()) != cudaSuccess) {
+        std::string msg = std::string("pair table upload: ") + cudaGetErrorString(e);
+        tp3_ctx_destroy(c);
+        return fail(nullptr, TP3_ERR_CUDA, msg);
+      }
+      hf.ngroups = (int)hg.size();
+      hf.ok = true;
+    }
+  }
   c->tc.err = c->d_err;  // device error flag of the TP3_DEBUG index checks
   c->tc_why = setup_tc(c);
   c->tc_ok = c->tc_why.empty();

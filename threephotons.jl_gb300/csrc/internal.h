@@ -72,6 +72,15 @@ cudaError_t launch_build_H(const DevTables& t, int n, const float* T, float* H, 
 size_t build_H_split_smem(const DevTables& t, int ppl);
 cudaError_t launch_build_H_split(const DevTables& t, int KP, int n, const float* T32, void* Hhi, void* Hlo, bool tf32,
                                  cudaStream_t s);
+// The same from order-major FP32 T ([lt][klp] a proposal), bit for bit.
+std::string build_hform_tables(const std::vector<int>& coff, int K, int n_lt, const int* lt_l1, const int* lt_l2,
+                               const int* lt_l3, const std::vector<std::pair<int, int>>& pairs,
+                               const std::vector<int>& qstart, const std::vector<int>& qlist,
+                               const std::vector<int>& lt_of_j, const std::vector<float>& w, std::vector<int4>& groups,
+                               std::vector<int2>& lists, std::vector<int2>& entries, std::vector<float>& wts,
+                               std::vector<int>& slot_m);
+bool hform_fits(int n_lt, int nc);
+cudaError_t hform_configure();
 cudaError_t launch_finalize(const DevTables& t, int n, const double2* part, int ncg,
                             const double* Qs, int mult, double* E, cudaStream_t s);
 
@@ -166,8 +175,22 @@ struct LaneTables {
   const int2* kofs = nullptr;       // [K + 1]
 };
 
+// Fourier-pair operand at lambda != 0 (kernels_hform.cu): slots (pairs; two for (0, 0)) by
+// warps, each with its list of l-triples and their 3j values, and groups of up to four
+// consecutive shell triples.
+struct HformTables {
+  bool ok = false;
+  int ngroups = 0;
+  const int4* groups = nullptr;   // first shell triple, count, k1 | k2 << 8, first k3
+  const int2* lists = nullptr;    // per 32 slots: range of entries
+  const int2* entries = nullptr;  // l-triple, centres of its orders' coefficient rows (10 bits each)
+  const float* wts = nullptr;     // [entries][32]
+  const int* slot_m = nullptr;    // m1, m2, m3 of a slot (8 bits each)
+};
+
 // Device tables of the tensor-core path.
 struct TcTables {
+  HformTables hf;
   LaneTables lane;
   bool use_lane = false;
   // folded-row coupling tilings: [0] 8 warps, [1] 7 warps, [2] 13 warps (smaller D
@@ -271,6 +294,8 @@ cudaError_t launch_angular_persistent(const DevTables& t, const TcTables& tc, co
                                       const RagInfo* rag = nullptr, float* c3out = nullptr);
 cudaError_t launch_finalize_parts(const DevTables& t, const TcTables& tc, int n, const float* part, const double* Qs,
                                   double* E, cudaStream_t s, const RagInfo* rag = nullptr);
+cudaError_t launch_build_H_pairs(const DevTables& t, const TcTables& tc, int n, const float* T32, void* Hhi, void* Hlo,
+                                 bool tf32, cudaStream_t s);
 size_t couple_split_smem_d(const DevTables& t, const TcTables& tc);
 size_t couple_split_smem_t(const DevTables& t, const TcTables& tc);
 cudaError_t couple_split_configure(const DevTables& t, const TcTables& tc);
