@@ -131,7 +131,7 @@ int tp3_set_coupling(tp3_ctx* ctx, int form);
  * grid half) units with two TMEM accumulators, so the Bayes epilogue of one unit
  * overlaps the tensor-core work of the next.  TP3_ANGULAR_TILE: one CTA per
  * (tile, proposal), both grid halves in sequence.  Energies agree to FP32 rounding of
- * the partial sums; the c3 output path always uses the per-tile kernel. */
+ * the partial sums; the c3 output path always uses the persistent kernel. */
 #define TP3_ANGULAR_TILE 0
 #define TP3_ANGULAR_PERSISTENT 1
 int tp3_set_angular(tp3_ctx* ctx, int schedule);

@@ -668,8 +668,8 @@ int run_energy(tp3_ctx* c, int n, const double2* d_coeff, double* d_E, bool comp
       if ((e = tp3::launch_finalize_parts(t, c->tc, n, part, Qf, d_E, c->stream, rag)) != cudaSuccess)
         return cuda_fail(c, e, "finalize_parts");
     } else {
-      if ((e = tp3::launch_angular_tc(t, c->tc, tf ? c->maps32 : c->maps, n, qt, Qf, c->d_Eslab, nullptr, c->d_err,
-                                      tf, c->stream, rag)) != cudaSuccess)
+      if ((e = tp3::launch_angular_tc(t, c->tc, tf ? c->maps32 : c->maps, n, qt, Qf, c->d_Eslab, c->d_err, tf, c->stream,
+                                      rag)) != cudaSuccess)
         return cuda_fail(c, e, "angular_tc");
       if (pr) cudaEventRecord(b, c->stream);
       if ((e = tp3::launch_finalize_slabs(n, t.klength, c->d_Eslab, d_E, c->stream, rag)) != cudaSuccess)
@@ -1405,8 +1405,8 @@ int tp3_c3(tp3_ctx* c, const double* coeff, float* out) {
     return cuda_fail(c, e, "H2D coeff");
   if (int r = run_coupling(c, 1, c->d_coeff, false)) return r;
   if (is_tc(c->mode))
-    e = tp3::launch_angular_tc(t, c->tc, c->mode == TP3_MODE_TC_TF32X3 ? c->maps32 : c->maps, 1, nullptr, nullptr,
-                               nullptr, c->d_c3, c->d_err, c->mode == TP3_MODE_TC_TF32X3, c->stream);
+    e = tp3::launch_angular_persistent(t, c->tc, c->mode == TP3_MODE_TC_TF32X3 ? c->maps32 : c->maps, 1, nullptr, nullptr,
+                                       c->d_err, c->mode == TP3_MODE_TC_TF32X3, c->stream, nullptr, c->d_c3);
   else
     e = tp3::launch_angular_plain(t, 1, plain_A(c), nullptr, nullptr, tp3::plain_ncg(t), c->d_c3, c->stream);
   if (e != cudaSuccess) return cuda_fail(c, e, "angular store");
@@ -1425,8 +1425,8 @@ int tp3_c3_batch_device(tp3_ctx* c, int n, const void* d_coeffs, void* d_c3) {
   cudaError_t e;
   if (int r = run_coupling(c, n, (const double2*)d_coeffs, false)) return r;
   if (is_tc(c->mode))
-    e = tp3::launch_angular_tc(t, c->tc, c->mode == TP3_MODE_TC_TF32X3 ? c->maps32 : c->maps, n, nullptr, nullptr,
-                               nullptr, (float*)d_c3, c->d_err, c->mode == TP3_MODE_TC_TF32X3, c->stream);
+    e = tp3::launch_angular_persistent(t, c->tc, c->mode == TP3_MODE_TC_TF32X3 ? c->maps32 : c->maps, n, nullptr, nullptr,
+                                       c->d_err, c->mode == TP3_MODE_TC_TF32X3, c->stream, nullptr, (float*)d_c3);
   else
     e = tp3::launch_angular_plain(t, n, plain_A(c), nullptr, nullptr, tp3::plain_ncg(t), (float*)d_c3, c->stream);
   if (e != cudaSuccess) return cuda_fail(c, e, "angular store");

@@ -268,7 +268,7 @@ struct TcMaps {
   CUtensorMap a_hi_mn, a_lo_mn;  // BF16 T operand in the order-major layout [lt][ki]
 };
 
-size_t tc_smem_bytes();
+size_t tc_smem_bytes(bool store);
 // Dynamic shared memory the coupling kernel may request (the opt-in maximum of
 // 227 KB minus its static counters and slack).
 constexpr int kCoupleMaxDynSmem = 227 * 1024 - 2048;
@@ -281,7 +281,7 @@ cudaError_t launch_couple_pair(const DevTables& t, const TcTables& tc, int n, co
                                const RagInfo* rag = nullptr);
 // qt / Qs: one histogram, or (rag) the histogram set with strides klp * Gu and klength.
 cudaError_t launch_angular_tc(const DevTables& t, const TcTables& tc, const TcMaps& maps, int n, const float* qt,
-                              const double* Qs, double* Eslab, float* c3out, int* err, bool tf32, cudaStream_t s,
+                              const double* Qs, double* Eslab, int* err, bool tf32, cudaStream_t s,
                               const RagInfo* rag = nullptr);
 cudaError_t launch_finalize_slabs(int n, int klength, const double* Eslab, double* E, cudaStream_t s,
                                   const RagInfo* rag = nullptr);

@@ -570,6 +570,8 @@ __host__ __device__ constexpr uint32_t idesc_m128_n256(uint32_t fmt) {
   return (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(kBN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
 }
 
+constexpr int kStorePitch = 17;  // floats per row of a warp's 32 x 16 store tile
+
 struct TcSmemHeader {
   uint64_t full[kStages];
   uint64_t empty[kStages];
@@ -581,16 +583,15 @@ struct TcSmemHeader {
 };
 
 // grid: (klp / 128, n); block kThreads; dyn smem = 1 KB alignment slack + stages + header.
-// STORE: write c3 (all four images of every unique point) instead of the Bayes terms.
 // AMN (BF16 only): T is order-major, [prop][lt][ki]; each stage's A tile arrives as two
 // 64-shell-triple boxes (128-byte swizzle) and is read as an MN-major operand.
-template <bool STORE, bool TF32, bool AMN>
+template <bool TF32, bool AMN>
 __global__ void __launch_bounds__(kThreads, 1) k_angular_tc(
     const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant__ CUtensorMap tmA_lo,
     const __grid_constant__ CUtensorMap tmB_hi, const __grid_constant__ CUtensorMap tmB_lo, int klp, int KP,
     int Gu, int nhalf, int klength, const float* __restrict__ qt, const double* __restrict__ Qs,
-    const double* __restrict__ tf, int mult, double* __restrict__ Eslab, float* __restrict__ c3out,
-    const int* __restrict__ u_to_g, int N, int* __restrict__ err, const RagInfo* __restrict__ rag) {
+    const double* __restrict__ tf, int mult, double* __restrict__ Eslab, int* __restrict__ err,
+    const RagInfo* __restrict__ rag) {
   extern __shared__ uint8_t smem_raw[];
   if (rag) {
     // ragged batch: tiles past the proposal's scored shell triples do no work, and
@@ -711,7 +712,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_angular_tc(
     const int quarter = warp & 3;           // TMEM lane quarter this warp may access
     const int cblk = ew >> 2;               // which 128-column block of each half
     const int r = quarter * 32 + lane;      // row inside the tile
-    const int ki = mtile * kBM + r;
     // compensated (Kahan) sums: Sp and Sql are differences of large, nearly equal
     // energies once combined, so their rounding sets the precision of dE
     float sp = 0.f, sq = 0.f, csp = 0.f, csq = 0.f;
@@ -722,52 +722,30 @@ __global__ void __launch_bounds__(kThreads, 1) k_angular_tc(
         const int col = h * kBN + cblk * 128 + cc * 32;
         float v[32];
         tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)col, v);
-        if (STORE) {
-          if (ki < klength) {
-            float* o = c3out + ((size_t)prop * klength + ki) * (size_t)(2 * N * N);
-#pragma unroll 4
-            for (int j = 0; j < 32; ++j) {
-              const int u = col + j;
-              if (u < Gu) {
-                const int g = u_to_g[u];
-                const int a = g % N, b = g / N;
-                o[g] = v[j];
-                if (mult == 4) {
-                  o[a + N * (b + N)] = v[j];
-                  o[(N - 1 - a) + N * (N - 1 - b)] = v[j];
-                  o[(N - 1 - a) + N * (2 * N - 1 - b)] = v[j];
-                }
-              }
-            }
-          }
-        } else {
-          const float* qrow = qt + ((size_t)mtile * Gu) * kBM + r;
+        const float* qrow = qt + ((size_t)mtile * Gu) * kBM + r;
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const int u = col + j;
-            if (u < Gu) {
-              const float p = fmaxf(v[j], 1e-30f);
-              const float y1 = p - csp;
-              const float t1 = sp + y1;
-              csp = (t1 - sp) - y1;
-              sp = t1;
-              const float y2 = qrow[(size_t)u * kBM] * __logf(p) - csq;
-              const float t2 = sq + y2;
-              csq = (t2 - sq) - y2;
-              sq = t2;
-            }
+        for (int j = 0; j < 32; ++j) {
+          const int u = col + j;
+          if (u < Gu) {
+            const float p = fmaxf(v[j], 1e-30f);
+            const float y1 = p - csp;
+            const float t1 = sp + y1;
+            csp = (t1 - sp) - y1;
+            sp = t1;
+            const float y2 = qrow[(size_t)u * kBM] * __logf(p) - csq;
+            const float t2 = sq + y2;
+            csq = (t2 - sq) - y2;
+            sq = t2;
           }
         }
       }
     }
-    if (!STORE) {
-      hd->part_sp[cblk][r] = sp - csp;
-      hd->part_sq[cblk][r] = sq - csq;
-    }
+    hd->part_sp[cblk][r] = sp - csp;
+    hd->part_sq[cblk][r] = sq - csq;
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (!STORE && warp >= 2 && warp < 6) {
+  if (warp >= 2 && warp < 6) {
     const int r = (warp & 3) * 32 + lane;
     const int ki = mtile * kBM + r;
     if (ki < klength && !*abort_flag) {
@@ -790,15 +768,16 @@ __global__ void __launch_bounds__(kThreads, 1) k_angular_tc(
 // a buffer to the epilogue; tmem_empty[b] (one arrival per epilogue warp) hands it back.
 // The epilogue writes compensated partial sums per (row, half, column block) to
 // part [prop][klp][nhalf halves][2 blocks][Sp, Sql]; k_finalize_parts forms the slab
-// terms.  STORE: the epilogue writes c3 instead (all images of every unique point).
+// terms.  STORE: the epilogue writes c3 instead (all images of every unique point), through a
+// 32 x 16 transpose per warp so that a store instruction covers 64-byte runs of two rows (one row
+// a lane was 32 sectors per instruction: 268 us for 107 MB at L18 K26 N32).
 // Any number of halves (the unfolded 2N^2-point grid of lambda != 0 has 8 at N = 32).
 template <bool STORE, bool TF32, bool AMN>
 __global__ void __launch_bounds__(kThreads, 1) k_angular_tp(
     const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant__ CUtensorMap tmA_lo,
     const __grid_constant__ CUtensorMap tmB_hi, const __grid_constant__ CUtensorMap tmB_lo, int klp, int KP,
     int Gu, int nhalf, int nunits, const float* __restrict__ qt, float* __restrict__ part, int* __restrict__ err,
-    const RagInfo* __restrict__ rag, int klength, float* __restrict__ c3out, const int* __restrict__ u_to_g, int N,
-    int mult) {
+    const RagInfo* __restrict__ rag, int klength, float* __restrict__ c3out, int N, int mult) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t tmem_empty[2];
   uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -949,22 +928,28 @@ __global__ void __launch_bounds__(kThreads, 1) k_angular_tp(
         float v[32];
         if (STORE) {
           tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * kBN + col), v);
-          if (ki < klength) {
-            float* o = c3out + ((size_t)prop * klength + ki) * (size_t)(2 * N * N);
+          // unique points are the first N^2 / 2 grid points (folded grid) or all of them
+          float* tile = reinterpret_cast<float*>(hd + 1) + ew * (32 * kStorePitch);
+          const int N2 = N * N, ki0 = mtile * kBM + quarter * 32;
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) tile[lane * kStorePitch + j] = v[16 * half + j];
+            __syncwarp();
+            const int ul = u0 + 16 * half + (lane & 15);
 #pragma unroll 4
-            for (int j = 0; j < 32; ++j) {
-              const int u = u0 + j;
-              if (u < Gu) {
-                const int g = u_to_g[u];
-                const int a = g % N, bb = g / N;
-                o[g] = v[j];
-                if (mult == 4) {
-                  o[a + N * (bb + N)] = v[j];
-                  o[(N - 1 - a) + N * (N - 1 - bb)] = v[j];
-                  o[(N - 1 - a) + N * (2 * N - 1 - bb)] = v[j];
-                }
+            for (int rr = lane >> 4; rr < 32; rr += 2) {
+              if (ul >= Gu || ki0 + rr >= klength) continue;
+              const float x = tile[rr * kStorePitch + (lane & 15)];
+              float* o = c3out + ((size_t)prop * klength + ki0 + rr) * (size_t)(2 * N2);
+              o[ul] = x;
+              if (mult == 4) {  // (a, b + N), (N - 1 - a, N - 1 - b), (N - 1 - a, 2 N - 1 - b)
+                o[N2 + ul] = x;
+                o[N2 - 1 - ul] = x;
+                o[2 * N2 - 1 - ul] = x;
               }
             }
+            __syncwarp();
           }
           continue;
         }
@@ -1132,24 +1117,24 @@ __global__ void __cluster_dims__(kFinCtas, 1, 1) __launch_bounds__(128)
 
 }  // namespace
 
-size_t tc_smem_bytes() { return 1024 + (size_t)kStages * kStageBytes + sizeof(TcSmemHeader); }
+size_t tc_smem_bytes(bool store) {
+  return 1024 + (size_t)kStages * kStageBytes + sizeof(TcSmemHeader) +
+         (store ? (size_t)kEpiWarps * 32 * kStorePitch * sizeof(float) : 0);
+}
 
 cudaError_t tc_configure() {
   cudaError_t e;
-  const int smem = (int)tc_smem_bytes();
+  const int smem = (int)tc_smem_bytes(false), smem_st = (int)tc_smem_bytes(true);
   const cudaFuncAttribute ds = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  if ((e = cudaFuncSetAttribute(k_angular_tc<false, false, false>, ds, smem)) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(k_angular_tc<true, false, false>, ds, smem)) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(k_angular_tc<false, true, false>, ds, smem)) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(k_angular_tc<true, true, false>, ds, smem)) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(k_angular_tc<false, false, true>, ds, smem)) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(k_angular_tc<true, false, true>, ds, smem)) != cudaSuccess ||
+  if ((e = cudaFuncSetAttribute(k_angular_tc<false, false>, ds, smem)) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(k_angular_tc<true, false>, ds, smem)) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(k_angular_tc<false, true>, ds, smem)) != cudaSuccess ||
       (e = cudaFuncSetAttribute(k_angular_tp<false, false, false>, ds, smem)) != cudaSuccess ||
       (e = cudaFuncSetAttribute(k_angular_tp<false, true, false>, ds, smem)) != cudaSuccess ||
       (e = cudaFuncSetAttribute(k_angular_tp<false, false, true>, ds, smem)) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(k_angular_tp<true, false, false>, ds, smem)) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(k_angular_tp<true, true, false>, ds, smem)) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(k_angular_tp<true, false, true>, ds, smem)) != cudaSuccess)
+      (e = cudaFuncSetAttribute(k_angular_tp<true, false, false>, ds, smem_st)) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(k_angular_tp<true, true, false>, ds, smem_st)) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(k_angular_tp<true, false, true>, ds, smem_st)) != cudaSuccess)
     return e;
   const int cs = kCoupleMaxDynSmem, css = kCoupleSmallSmem;
 #define TP3_CP_ATTR(S, W)                                                                                    \
@@ -1251,28 +1236,16 @@ cudaError_t launch_couple_pair(const DevTables& t, const TcTables& tc, int n, co
 }
 
 cudaError_t launch_angular_tc(const DevTables& t, const TcTables& tc, const TcMaps& maps, int n, const float* qt,
-                              const double* Qs, double* Eslab, float* c3out, int* err, bool tf32, cudaStream_t s,
-                              const RagInfo* rag) {
-  // more than two grid halves do not fit one CTA's TMEM: the persistent kernel walks them
-  if (tc.nhalf > 2)
-    return c3out ? launch_angular_persistent(t, tc, maps, n, qt, nullptr, err, tf32, s, rag, c3out)
-                 : cudaErrorInvalidValue;
+                              const double* Qs, double* Eslab, int* err, bool tf32, cudaStream_t s, const RagInfo* rag) {
+  if (tc.nhalf > 2) return cudaErrorInvalidValue;  // more than two grid halves do not fit one CTA's TMEM
   dim3 grid(t.klp / kBM, n);
-  const size_t smem = tc_smem_bytes();
-  const bool amn = t_order_major(tc, tf32);
-#define TP3_ANG(ST, TF, MN, AH, AL)                                                                            \
-  k_angular_tc<ST, TF, MN><<<grid, kThreads, smem, s>>>(AH, AL, maps.b_hi, maps.b_lo, t.klp, tc.KP, t.Gu,        \
-                                                         tc.nhalf, t.klength, qt, Qs, t.tf, t.mult, Eslab, c3out, \
-                                                         t.u_to_g, t.N, err, rag)
-  if (c3out) {
-    if (tf32) TP3_ANG(true, true, false, maps.a_hi, maps.a_lo);
-    else if (amn) TP3_ANG(true, false, true, maps.a_hi_mn, maps.a_lo_mn);
-    else TP3_ANG(true, false, false, maps.a_hi, maps.a_lo);
-  } else {
-    if (tf32) TP3_ANG(false, true, false, maps.a_hi, maps.a_lo);
-    else if (amn) TP3_ANG(false, false, true, maps.a_hi_mn, maps.a_lo_mn);
-    else TP3_ANG(false, false, false, maps.a_hi, maps.a_lo);
-  }
+  const size_t smem = tc_smem_bytes(false);
+#define TP3_ANG(TF, MN, AH, AL)                                                                                   \
+  k_angular_tc<TF, MN><<<grid, kThreads, smem, s>>>(AH, AL, maps.b_hi, maps.b_lo, t.klp, tc.KP, t.Gu, tc.nhalf,  \
+                                                     t.klength, qt, Qs, t.tf, t.mult, Eslab, err, rag)
+  if (tf32) TP3_ANG(true, false, maps.a_hi, maps.a_lo);
+  else if (t_order_major(tc, tf32)) TP3_ANG(false, true, maps.a_hi_mn, maps.a_lo_mn);
+  else TP3_ANG(false, false, maps.a_hi, maps.a_lo);
 #undef TP3_ANG
   return cudaGetLastError();
 }
@@ -1288,12 +1261,11 @@ cudaError_t launch_angular_persistent(const DevTables& t, const TcTables& tc, co
                                       const RagInfo* rag, float* c3out) {
   const int nunits = n * (t.klp / kBM) * tc.nhalf;
   const int ctas = std::max(1, std::min(nunits, tc.nsm));
-  const size_t smem = tc_smem_bytes();
+  const size_t smem = tc_smem_bytes(c3out != nullptr);
   const bool amn = t_order_major(tc, tf32);
 #define TP3_ANGP(ST, TF, MN, AH, AL)                                                                          \
   k_angular_tp<ST, TF, MN><<<ctas, kThreads, smem, s>>>(AH, AL, maps.b_hi, maps.b_lo, t.klp, tc.KP, t.Gu, tc.nhalf, \
-                                                        nunits, qt, part, err, rag, t.klength, c3out, t.u_to_g, t.N,  \
-                                                        t.mult)
+                                                        nunits, qt, part, err, rag, t.klength, c3out, t.N, t.mult)
   if (c3out) {
     if (tf32) TP3_ANGP(true, true, false, maps.a_hi, maps.a_lo);
     else if (amn) TP3_ANGP(true, false, true, maps.a_hi_mn, maps.a_lo_mn);
