@@ -64,11 +64,8 @@ __global__ void __launch_bounds__(kHfThreads, 1) k_build_H_pairs(
 #pragma unroll
       for (int p = 0; p < NP / 2; ++p) acc[u][p] = make_float2(0.f, 0.f);
     const int2 ls = lists[slot >> 5];
-#pragma unroll 2
-    for (int e = ls.x; e < ls.y; ++e) {
-      const int2 en = __ldg(entries + e);  // l-triple, centres of the three orders' rows
-      const float w = __ldg(wts + (size_t)e * 32 + lane);
-      if (w == 0.f) continue;
+    auto term = [&](const int2 en, const float w) {
+      if (w == 0.f) return;
       const float y = w * y1[en.y & 1023] * y2[(en.y >> 10) & 1023];
       const float* yr = y3 + (en.y >> 20);
       const float4* t4 = reinterpret_cast<const float4*>(Ts + en.x * (4 * NP));
@@ -83,6 +80,18 @@ __global__ void __launch_bounds__(kHfThreads, 1) k_build_H_pairs(
           acc[u][2 * p + 1] = __ffma2_rn(P2, make_float2(t.z, t.w), acc[u][2 * p + 1]);
         }
       }
+    };
+    // l-triples (index, centres of the three orders' rows) and 3j values are fetched two ahead;
+    // the tables end with two spare entries
+    int2 ea = __ldg(entries + ls.x), eb = __ldg(entries + ls.x + 1);
+    float wa = __ldg(wts + (size_t)ls.x * 32 + lane), wb = __ldg(wts + (size_t)ls.x * 32 + 32 + lane);
+    for (int e = ls.x; e < ls.y; e += 2) {
+      const int f = min(e + 2, ls.y);
+      const int2 ec = __ldg(entries + f), ed = __ldg(entries + f + 1);
+      const float wc = __ldg(wts + (size_t)f * 32 + lane), wd = __ldg(wts + (size_t)f * 32 + 32 + lane);
+      term(ea, wa);
+      if (e + 1 < ls.y) term(eb, wb);
+      ea = ec; eb = ed; wa = wc; wb = wd;
     }
     const int q = slot - 1;  // slots 0 and 1: the even and odd entries of q = 0
 #pragma unroll
@@ -176,6 +185,8 @@ std::string build_hform_tables(const std::vector<int>& coff, int K, int n_lt, co
       }
     lists.push_back(make_int2(e0, (int)entries.size()));
   }
+  entries.resize(entries.size() + 2, make_int2(0, 0));  // fetched ahead of the last term
+  wts.resize(wts.size() + 64, 0.f);
   for (int k1 = 0; k1 < K; ++k1)
     for (int k2 = 0; k2 <= k1; ++k2)
       for (int k3 = 0; k3 <= k2; k3 += 4)

@@ -35,6 +35,10 @@ namespace {
 constexpr int kGStages = 4;
 constexpr int kGBM = 128;
 constexpr int kGBK = 32;  // bf16 per 64-byte swizzled row
+// Columns of a tile: at 256 the epilogue (four warps, 256 columns) was most of the 16 us of a
+// 3328 x 512 x 512 product on 52 CTAs; 64 is as fast there (241 against 251 us a training step)
+// and slower for the 26624 rows of a chain launch (161 against 126 us a forward pass).
+constexpr int kGBN = 128;
 constexpr int kGThreads = 192;  // TMA warp, MMA warp, 4 epilogue warps
 constexpr int kGABytes = kGBM * kGBK * 2;
 
@@ -50,7 +54,7 @@ struct GemmArgs {
   int ldt;
   float* out_f32;               // [M][ldf]
   int ldf;
-  int ksplit;                   // > 1: grid.z splits K; out_f32 accumulated with atomics (pre-zeroed)
+  int ksplit;                   // > 1: grid.z splits K; only out_f32, accumulated with atomics (pre-zeroed)
   int* err;
 };
 
@@ -64,8 +68,11 @@ struct GemmSmemHeader {
 
 template <int BN>
 __host__ __device__ constexpr int gemm_stage_bytes() { return kGABytes + BN * kGBK * 2; }
+// the header is followed by a 32 x 33 tile per epilogue warp (split-K accumulation)
 template <int BN>
-constexpr size_t gemm_smem_bytes() { return 1024 + (size_t)kGStages * gemm_stage_bytes<BN>() + sizeof(GemmSmemHeader); }
+constexpr size_t gemm_smem_bytes() {
+  return 1024 + (size_t)kGStages * gemm_stage_bytes<BN>() + sizeof(GemmSmemHeader) + 4 * 32 * 33 * sizeof(float);
+}
 
 // grid: (ceil(M / 128), ceil(N / BN)); block kGThreads.
 template <int BN>
@@ -157,6 +164,19 @@ __global__ void __launch_bounds__(kGThreads, 1) k_gemm_tn(const __grid_constant_
         float v[32];
         tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(c * 32), v);
         const int nb = n0 + c * 32;
+        if (ks > 1) {
+          // split K: the run is transposed so that a warp adds 32 consecutive columns of a row
+          // (one row a lane was 32 sectors an instruction: 53 us for 512 x 512 from 3328 rows)
+          float* tile = reinterpret_cast<float*>(hd + 1) + q * (32 * 33);
+#pragma unroll
+          for (int j = 0; j < 32; ++j) tile[lane * 33 + j] = v[j];
+          __syncwarp();
+          if (c * 32 + lane < BN && nb + lane < g.N)
+            for (int rr = 0; rr < 32 && m0 + q * 32 + rr < g.M; ++rr)
+              atomicAdd(&g.out_f32[(size_t)(m0 + q * 32 + rr) * g.ldf + nb + lane], tile[rr * 33 + lane]);
+          __syncwarp();
+          continue;
+        }
         // a whole 32-column run inside the tile and the matrix: 16-byte vector loads/stores
         const bool full = c * 32 + 32 <= BN && nb + 32 <= g.N && (!g.out_bf || g.ldo % 8 == 0) &&
                           (!g.gate || g.ldg % 8 == 0);
@@ -184,10 +204,7 @@ __global__ void __launch_bounds__(kGThreads, 1) k_gemm_tn(const __grid_constant_
           }
           if (g.out_f32) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              if (ks > 1) atomicAdd(&g.out_f32[(size_t)m * g.ldf + nb + j], x[j]);
-              else g.out_f32[(size_t)m * g.ldf + nb + j] = x[j];
-            }
+            for (int j = 0; j < 32; ++j) g.out_f32[(size_t)m * g.ldf + nb + j] = x[j];
           }
           if (g.out_bf) {
             uint4* op = reinterpret_cast<uint4*>(g.out_bf + (size_t)m * g.ldo + nb);
@@ -215,10 +232,7 @@ __global__ void __launch_bounds__(kGThreads, 1) k_gemm_tn(const __grid_constant_
             if (g.bias) x += g.bias[n];
             if (g.relu) x = fmaxf(x, 0.f);
             if (g.gate && !(__bfloat162float(g.gate[(size_t)m * g.ldg + n]) > 0.f)) x = 0.f;
-            if (g.out_f32) {
-              if (ks > 1) atomicAdd(&g.out_f32[(size_t)m * g.ldf + n], x);
-              else g.out_f32[(size_t)m * g.ldf + n] = x;
-            }
+            if (g.out_f32) g.out_f32[(size_t)m * g.ldf + n] = x;
             const __nv_bfloat16 xb = __float2bfloat16_rn(x);
             if (g.out_bf) g.out_bf[(size_t)m * g.ldo + n] = xb;
             if (g.outT_bf) g.outT_bf[(size_t)n * g.ldt + m] = xb;
@@ -254,89 +268,102 @@ __global__ void k_transpose_bf16(const __nv_bfloat16* __restrict__ X, int R, int
 // Regression of the logged energy changes on the steps: for candidate j (rows
 // jK..jK+K-1, one per shell) r_j = t_j - sum_k u_k . V_k with (t_j, lambda_j) = tw[j],
 // V = v / sigma the logged step; resid[j] = lambda_j r_j, part[block] = sum of
-// lambda_j r_j^2 / 2.  grid ceil(nc / 128), block 128.
+// lambda_j r_j^2 / 2.  One warp a candidate (a thread a candidate took 19 us for 128, on one
+// SM's FP64 units).  grid ceil(nc / 4), block 128.
 __global__ void k_reg_residual(const float* __restrict__ O, const float* __restrict__ V,
                                const float2* __restrict__ tw, int K, int nc, float* __restrict__ resid,
                                double* __restrict__ part) {
-  __shared__ double red[128];
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  __shared__ double red[4];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int j = blockIdx.x * 4 + warp;
   double l = 0.0;
   if (j < nc) {
     double p = 0.0;
-    for (int k = 0; k < K; ++k) {
+    for (int i = lane; i < 3 * K; i += 32) {
+      const int k = i / 3, d = i - 3 * k;
       const size_t r = (size_t)j * K + k;
-      for (int d = 0; d < 3; ++d) p += (double)O[r * kMlpOutPad + d] * (double)V[r * 3 + d];
+      p += (double)O[r * kMlpOutPad + d] * (double)V[r * 3 + d];
     }
+    for (int o = 16; o > 0; o >>= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
     const float2 t = tw[j];
     const double res = (double)t.x - p;
-    resid[j] = (float)((double)t.y * res);
+    if (lane == 0) resid[j] = (float)((double)t.y * res);
     l = 0.5 * (double)t.y * res * res;
   }
-  red[threadIdx.x] = l;
+  if (lane == 0) red[warp] = l;
   __syncthreads();
-  for (int h = 64; h > 0; h >>= 1) {
-    if (threadIdx.x < h) red[threadIdx.x] += red[threadIdx.x + h];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) part[blockIdx.x] = red[0];
+  if (threadIdx.x == 0) part[blockIdx.x] = (red[0] + red[1]) + (red[2] + red[3]);
 }
 
 // Gradient of the loss wrt the raw outputs: the regression term on u (resid
 // nullable: none) and the weighted zero-mean Gaussian NLL of the logged steps V on
 // the log-scales s, sum_d w [s_d + V_d^2 exp(-2 s_d) / 2 + log(2 pi) / 2].
-// grid ceil(R/128), block 128.  dO [R][16] bf16 and dOt [16][ldt] bf16 (columns /
+// Four threads a row, three of them an order each, so that the FP64 tanh and exp spread over
+// the SMs.  grid ceil(R/32), block 128.  dO [R][16] bf16 and dOt [16][ldt] bf16 (columns /
 // rows 6..15 zero); part[block] = sum of w NLL over the block.
 __global__ void k_head_loss(const float* __restrict__ O, int R, const float* __restrict__ vlog,
                             const float* __restrict__ w, const float* __restrict__ resid, int K, int nc,
                             __nv_bfloat16* __restrict__ dO, __nv_bfloat16* __restrict__ dOt, int ldt,
                             double* __restrict__ part) {
-  __shared__ double red[128];
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  __shared__ double red[32];
+  const int d = threadIdx.x & 3, lr = threadIdx.x >> 2, r = blockIdx.x * 32 + lr;
   double nll = 0.0;
-  if (r < R) {
+  float gu = 0.f, gs = 0.f;
+  double wr = 0.0;
+  if (r < R && d < 3) {
     const float* o = O + (size_t)r * kMlpOutPad;
-    const double wr = w[r];
+    wr = w[r];
     const double rj = (resid && r / K < nc) ? (double)resid[r / K] : 0.0;
-    float g[kMlpOutPad];
-    for (int j = 0; j < kMlpOutPad; ++j) g[j] = 0.f;
-    for (int d = 0; d < 3; ++d) {
-      const double ts = tanh((double)o[3 + d]);
-      const double s = kSMid + kSHalf * ts;
-      const double e = (double)vlog[(size_t)r * 3 + d];
-      const double is2 = exp(-2.0 * s);
-      nll += s + 0.5 * e * e * is2 + 0.9189385332046727;  // 0.5 log(2 pi)
-      g[d] = (float)(-rj * e);
-      g[3 + d] = (float)(wr * (1.0 - e * e * is2) * kSHalf * (1.0 - ts * ts));
-    }
-    nll *= wr;
-    for (int j = 0; j < kMlpOutPad; ++j) {
-      const __nv_bfloat16 b = __float2bfloat16_rn(g[j]);
+    const double ts = tanh((double)o[3 + d]);
+    const double s = kSMid + kSHalf * ts;
+    const double e = (double)vlog[(size_t)r * 3 + d];
+    const double is2 = exp(-2.0 * s);
+    nll = s + 0.5 * e * e * is2 + 0.9189385332046727;  // 0.5 log(2 pi)
+    gu = (float)(-rj * e);
+    gs = (float)(wr * (1.0 - e * e * is2) * kSHalf * (1.0 - ts * ts));
+  }
+  const double n1 = __shfl_down_sync(0xffffffffu, nll, 1), n2 = __shfl_down_sync(0xffffffffu, nll, 2);
+  if (r < R) {
+    // columns d and 3 + d from the row's first three threads, the ten zero columns from all four
+    auto put = [&](int j, float g) {
+      const __nv_bfloat16 b = __float2bfloat16_rn(g);
       dO[(size_t)r * kMlpOutPad + j] = b;
       dOt[(size_t)j * ldt + r] = b;
+    };
+    if (d < 3) {
+      put(d, gu);
+      put(3 + d, gs);
     }
+    for (int j = 6 + d; j < kMlpOutPad; j += 4) put(j, 0.f);
   }
-  red[threadIdx.x] = nll;
+  if (d == 0) red[lr] = (nll + n1 + n2) * wr;
   __syncthreads();
-  for (int h = 64; h > 0; h >>= 1) {
+  for (int h = 16; h > 0; h >>= 1) {
     if (threadIdx.x < h) red[threadIdx.x] += red[threadIdx.x + h];
     __syncthreads();
   }
   if (threadIdx.x == 0) part[blockIdx.x] = red[0];
 }
 
-// db[n] = sum_r Zt[n][r] (FP32 sum of BF16 values); grid N, block 256.
+// db[n] = sum_r Zt[n][r] (FP32 sum of BF16 values), R and ldt multiples of 8; grid N, block 128.
+// Bound by latency: 16-byte loads (one value at a time took 9.5 us for 512 x 3328).
 __global__ void k_rowsum_bf16(const __nv_bfloat16* __restrict__ Zt, int ldt, int R, float* __restrict__ db) {
-  __shared__ float red[256];
-  const __nv_bfloat16* z = Zt + (size_t)blockIdx.x * ldt;
+  __shared__ float red[4];
+  const uint4* z = reinterpret_cast<const uint4*>(Zt + (size_t)blockIdx.x * ldt);
   float s = 0.f;
-  for (int r = threadIdx.x; r < R; r += blockDim.x) s += __bfloat162float(z[r]);
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int h = 128; h > 0; h >>= 1) {
-    if (threadIdx.x < h) red[threadIdx.x] += red[threadIdx.x + h];
-    __syncthreads();
+#pragma unroll 4
+  for (int r = threadIdx.x; r < R / 8; r += 128) {
+    const uint4 u = z[r];
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+    float t = 0.f;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) t += __uint_as_float(w[q] << 16) + __uint_as_float(w[q] & 0xffff0000u);
+    s += t;
   }
-  if (threadIdx.x == 0) db[blockIdx.x] = red[0];
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) db[blockIdx.x] = (red[0] + red[1]) + (red[2] + red[3]);
 }
 
 __global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
@@ -404,7 +431,7 @@ struct tp3_mlp {
   float* O = nullptr;                            // [max_rows][16]
   __nv_bfloat16 *dO = nullptr, *dOt = nullptr;   // [max_rows][16], [16][max_rows]
   __nv_bfloat16 *P = nullptr, *Q = nullptr, *Tt = nullptr;  // [max_rows][H] x2, [H][max_rows]
-  double* d_part = nullptr;                      // loss partials [2][max_rows / 128] (NLL, regression)
+  double* d_part = nullptr;                      // loss partials [max_rows / 32] NLL, [max_rows / 4] regression
   float* d_resid = nullptr;                      // weighted regression residual per candidate [max_rows]
   int* d_err = nullptr;
   // tensor maps: forward F1..F4, backward B1..B7
@@ -426,7 +453,7 @@ cudaError_t enc(tp3_ctx* c, CUtensorMap* m, const void* ptr, uint64_t inner, uin
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-int pick_bn(int N) { return N <= 16 ? 16 : (N <= 128 ? 128 : 256); }
+int pick_bn(int N) { return N <= 16 ? 16 : kGBN; }
 
 cudaError_t gemm(tp3_mlp* net, const CUtensorMap& A, const CUtensorMap& B, GemmArgs g) {
   const int bn = pick_bn(g.N);
@@ -436,8 +463,7 @@ cudaError_t gemm(tp3_mlp* net, const CUtensorMap& A, const CUtensorMap& B, GemmA
   grid.z = g.ksplit;
   cudaStream_t s = net->ctx->stream;
   if (bn == 16) k_gemm_tn<16><<<grid, kGThreads, gemm_smem_bytes<16>(), s>>>(A, B, g);
-  else if (bn == 128) k_gemm_tn<128><<<grid, kGThreads, gemm_smem_bytes<128>(), s>>>(A, B, g);
-  else k_gemm_tn<256><<<grid, kGThreads, gemm_smem_bytes<256>(), s>>>(A, B, g);
+  else k_gemm_tn<kGBN><<<grid, kGThreads, gemm_smem_bytes<kGBN>(), s>>>(A, B, g);
   return cudaGetLastError();
 }
 
@@ -499,11 +525,11 @@ cudaError_t backward(tp3_mlp* n, int R, const float* v, const float* w, const fl
   k_transpose_bf16<<<tg, tb, 0, s>>>(n->X, R, n->n_in_pad, n->n_in_pad, n->Xt, MR);
   const int nc = R / K;
   if (tw) {
-    k_reg_residual<<<(nc + 127) / 128, 128, 0, s>>>(n->O, v, reinterpret_cast<const float2*>(tw), K, nc, n->d_resid,
-                                                   n->d_part + MR / 128);
+    k_reg_residual<<<(nc + 3) / 4, 128, 0, s>>>(n->O, v, reinterpret_cast<const float2*>(tw), K, nc, n->d_resid,
+                                               n->d_part + MR / 32);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
-  k_head_loss<<<R / 128, 128, 0, s>>>(n->O, R, v, w, tw ? n->d_resid : nullptr, K, nc, n->dO, n->dOt, MR, n->d_part);
+  k_head_loss<<<R / 32, 128, 0, s>>>(n->O, R, v, w, tw ? n->d_resid : nullptr, K, nc, n->dO, n->dOt, MR, n->d_part);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   float* gW[4];
   float* gb[4];
@@ -522,7 +548,7 @@ cudaError_t backward(tp3_mlp* n, int R, const float* v, const float* w, const fl
   GemmArgs g = args(kMlpOut, H, R);
   g.out_f32 = gW[3]; g.ldf = H; g.ksplit = split(kMlpOut, H);
   if ((e = gemm(n, n->bA[0], n->bB[0], g)) != cudaSuccess) return e;
-  k_rowsum_bf16<<<kMlpOut, 256, 0, s>>>(n->dOt, MR, R, gb[3]);
+  k_rowsum_bf16<<<kMlpOut, 128, 0, s>>>(n->dOt, MR, R, gb[3]);
   // B2: dZ3 = (dO W4) . [H3 > 0] -> P, Tt
   g = args(R, H, kMlpOutPad);
   g.gate = n->Hh[2]; g.ldg = H; g.out_bf = n->P; g.ldo = H; g.outT_bf = n->Tt; g.ldt = MR;
@@ -531,7 +557,7 @@ cudaError_t backward(tp3_mlp* n, int R, const float* v, const float* w, const fl
   g = args(H, H, R);
   g.out_f32 = gW[2]; g.ldf = H; g.ksplit = split(H, H);
   if ((e = gemm(n, n->bA[2], n->bB[2], g)) != cudaSuccess) return e;
-  k_rowsum_bf16<<<H, 256, 0, s>>>(n->Tt, MR, R, gb[2]);
+  k_rowsum_bf16<<<H, 128, 0, s>>>(n->Tt, MR, R, gb[2]);
   // B4: dZ2 = (dZ3 W3) . [H2 > 0] -> Q, Tt
   g = args(R, H, H);
   g.gate = n->Hh[1]; g.ldg = H; g.out_bf = n->Q; g.ldo = H; g.outT_bf = n->Tt; g.ldt = MR;
@@ -540,7 +566,7 @@ cudaError_t backward(tp3_mlp* n, int R, const float* v, const float* w, const fl
   g = args(H, H, R);
   g.out_f32 = gW[1]; g.ldf = H; g.ksplit = split(H, H);
   if ((e = gemm(n, n->bA[4], n->bB[4], g)) != cudaSuccess) return e;
-  k_rowsum_bf16<<<H, 256, 0, s>>>(n->Tt, MR, R, gb[1]);
+  k_rowsum_bf16<<<H, 128, 0, s>>>(n->Tt, MR, R, gb[1]);
   // B6: dZ1^T = ((dZ2 W2) . [H1 > 0])^T -> Tt
   g = args(R, H, H);
   g.gate = n->Hh[0]; g.ldg = H; g.outT_bf = n->Tt; g.ldt = MR;
@@ -549,7 +575,7 @@ cudaError_t backward(tp3_mlp* n, int R, const float* v, const float* w, const fl
   g = args(H, n->n_in, R);
   g.out_f32 = gW[0]; g.ldf = n->n_in; g.ksplit = split(H, n->n_in);
   if ((e = gemm(n, n->bA[6], n->bB[6], g)) != cudaSuccess) return e;
-  k_rowsum_bf16<<<H, 256, 0, s>>>(n->Tt, MR, R, gb[0]);
+  k_rowsum_bf16<<<H, 128, 0, s>>>(n->Tt, MR, R, gb[0]);
   return cudaGetLastError();
 }
 
@@ -559,10 +585,8 @@ cudaError_t mlp_configure() {
   cudaError_t e;
   if ((e = cudaFuncSetAttribute(k_gemm_tn<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)gemm_smem_bytes<16>())) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(k_gemm_tn<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)gemm_smem_bytes<128>())) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(k_gemm_tn<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)gemm_smem_bytes<256>())) != cudaSuccess)
+      (e = cudaFuncSetAttribute(k_gemm_tn<kGBN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)gemm_smem_bytes<kGBN>())) != cudaSuccess)
     return e;
   return cudaSuccess;
 }
@@ -625,7 +649,7 @@ int tp3_mlp_create(tp3_ctx* c, int n_in, int hidden, int max_rows, uint64_t seed
   A((void**)&n->O, (size_t)MR * tp3::kMlpOutPad * 4);
   A((void**)&n->dO, (size_t)MR * tp3::kMlpOutPad * bf); A((void**)&n->dOt, (size_t)tp3::kMlpOutPad * MR * bf);
   A((void**)&n->P, (size_t)MR * H * bf); A((void**)&n->Q, (size_t)MR * H * bf); A((void**)&n->Tt, (size_t)H * MR * bf);
-  A((void**)&n->d_part, (size_t)(2 * MR / 128) * sizeof(double)); A((void**)&n->d_err, sizeof(int));
+  A((void**)&n->d_part, (size_t)(MR / 32 + MR / 4) * sizeof(double)); A((void**)&n->d_err, sizeof(int));
   A((void**)&n->d_resid, (size_t)MR * sizeof(float));
   if (e != cudaSuccess) {
     tp3::mlp_free(n);
@@ -756,12 +780,12 @@ static int mlp_loss_grad(tp3_mlp* n, int rows, const void* d_x, const float* d_v
   if (e == cudaSuccess) e = tp3::backward(n, rows, d_v, d_w, d_target, shells);
   if (e != cudaSuccess) return tp3::ctx_cuda_fail(c, e, "mlp backward");
   if (loss) {
-    const int nb = rows / 128, nr = d_target ? (rows / shells + 127) / 128 : 0;
+    const int nb = rows / 32, nr = d_target ? (rows / shells + 3) / 4 : 0;
     std::vector<double> part(nb), rpart(nr > 0 ? nr : 1);
     int err = 0;
     if ((e = cudaMemcpyAsync(part.data(), n->d_part, nb * sizeof(double), cudaMemcpyDeviceToHost, c->stream)) !=
             cudaSuccess ||
-        (nr > 0 && (e = cudaMemcpyAsync(rpart.data(), n->d_part + n->max_rows / 128, nr * sizeof(double),
+        (nr > 0 && (e = cudaMemcpyAsync(rpart.data(), n->d_part + n->max_rows / 32, nr * sizeof(double),
                                         cudaMemcpyDeviceToHost, c->stream)) != cudaSuccess) ||
         (e = cudaMemcpyAsync(&err, n->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream)) != cudaSuccess ||
         (e = cudaStreamSynchronize(c->stream)) != cudaSuccess)
