@@ -120,15 +120,21 @@ __host__ __device__ inline void philox4x32_10(uint32_t c[4], uint32_t k0, uint32
 
 __device__ inline double u01(uint32_t x) { return ((double)x + 0.5) * 2.3283064365386963e-10; }
 
-// Four standard normals (two Box-Muller pairs) for (step, chain, purpose, index).
-__device__ inline void normals4(uint64_t seed, long long step, int chain, int purpose, int index, double z[4]) {
+// Box-Muller pair h (0 or 1) of the four standard normals of (step, chain, purpose, index).
+__device__ inline double2 normals2(uint64_t seed, long long step, int chain, int purpose, int index, int h) {
   uint32_t c[4] = {(uint32_t)step, (uint32_t)chain, (uint32_t)purpose, (uint32_t)index};
   philox4x32_10(c, (uint32_t)seed, (uint32_t)(seed >> 32));
+  const double r = sqrt(-2.0 * log(u01(h ? c[2] : c[0])));
+  const double a = 6.283185307179586 * u01(h ? c[3] : c[1]);
+  return make_double2(r * cos(a), r * sin(a));
+}
+
+// All four of them.
+__device__ inline void normals4(uint64_t seed, long long step, int chain, int purpose, int index, double z[4]) {
   for (int h = 0; h < 2; ++h) {
-    const double r = sqrt(-2.0 * log(u01(c[2 * h])));
-    const double a = 6.283185307179586 * u01(c[2 * h + 1]);
-    z[2 * h] = r * cos(a);
-    z[2 * h + 1] = r * sin(a);
+    const double2 v = normals2(seed, step, chain, purpose, index, h);
+    z[2 * h] = v.x;
+    z[2 * h + 1] = v.y;
   }
 }
 
@@ -145,29 +151,48 @@ __global__ void __launch_bounds__(256) k_propose(const double2* __restrict__ sta
                                                  int nl, int B, int K, int LMAX, int L, double f, uint64_t seed,
                                                  const tp3::RagInfo* __restrict__ rag) {
   if (rag) L = rag[blockIdx.x].L;  // a ragged chain rotates its own orders only
-  __shared__ double sp[8][2 * kMaxL + 1], sq[8][2 * kMaxL + 1];
+  __shared__ double sp[8][2 * kMaxL + 1], sq[8][2 * kMaxL + 1], ssig[kMaxL / 2 + 1];
   const int cid = blockIdx.x / B, i = blockIdx.x % B;
   const int ncoef = LMAX * LMAX;
   const double2* src = state + (size_t)cid * K * ncoef;
   double2* dst = cand + (size_t)blockIdx.x * K * ncoef;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  // step sizes after i rejections, divided step by step exactly as the sequential chain does:
+  // one warp for all orders (FP64 runs at two lanes per clock and SM), the others copy
+  if (warp == 0)
+    for (int q = lane; q < nl; q += 32) {
+      double sgl = sigma[(size_t)cid * nl + q];
+      for (int t = 0; t < i; ++t) sgl /= f;
+      ssig[q] = sgl;
+    }
   for (int e = threadIdx.x; e < K * ncoef; e += blockDim.x) dst[e] = src[e];
   __syncthreads();
   const long long step = cs[cid].step + i;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   for (int l = 2 * (warp + 1); l <= L; l += 2 * nw) {
     const int d = 2 * l + 1;
     double* p = sp[warp];
     double* q = sq[warp];
-    // plane: 2d normals, four per Philox call
-    for (int j = lane; 4 * j < 2 * d; j += 32) {
-      double z[4];
-      normals4(seed, step, cid, kPurposePlane, l * 64 + j, z);
-      for (int t = 0; t < 4; ++t) {
-        const int idx = 4 * j + t;
-        if (idx < d) p[idx] = z[t];
-        else if (idx < 2 * d) q[idx - d] = z[t];
+    // plane: 2d normals, four per Philox call, a pair a lane; the last lane draws the angle's pair
+    // beside them (a draw is some 300 FP64 instructions whatever the number of lanes)
+    double za = 0.0;
+    for (int j0 = 0; j0 < d; j0 += 31) {
+      const int j = j0 + lane;  // pair j: normals 2 j and 2 j + 1
+      const bool angle = lane == 31;
+      if (angle ? j0 == 0 : j < d) {
+        const double2 z = normals2(seed, step, cid, angle ? kPurposeAngle : kPurposePlane,
+                                   angle ? l : l * 64 + (j >> 1), angle ? 0 : j & 1);
+        if (angle) {
+          za = z.x;
+        } else {
+          for (int t = 0; t < 2; ++t) {
+            const int idx = 2 * j + t;
+            if (idx < d) p[idx] = t ? z.y : z.x;
+            else q[idx - d] = t ? z.y : z.x;
+          }
+        }
       }
     }
+    za = __shfl_sync(0xffffffffu, za, 31);
     __syncwarp();
     // Gram-Schmidt (FP64, lane-parallel sums)
     double pp = 0.0;
@@ -187,12 +212,7 @@ __global__ void __launch_bounds__(256) k_propose(const double2* __restrict__ sta
     const double iq = 1.0 / sqrt(qq);
     for (int t = lane; t < d; t += 32) q[t] *= iq;
     __syncwarp();
-    double za[4];
-    normals4(seed, step, cid, kPurposeAngle, l, za);
-    // step size after i rejections, divided step by step exactly as the sequential chain does
-    double sgl = sigma[(size_t)cid * nl + l / 2];
-    for (int t = 0; t < i; ++t) sgl /= f;
-    const double beta = za[0] * sgl;
+    const double beta = za * ssig[l / 2];
     const double cb = cos(beta) - 1.0, sb = sin(beta);
     const double r2 = 0.7071067811865476;
     // one shell per lane
