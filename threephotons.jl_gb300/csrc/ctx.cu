@@ -479,10 +479,10 @@ std::string setup_tc(tp3_ctx* c) {
              tp3::couple_split_smem_t(t, tc) <= (size_t)tp3::kCoupleMaxDynSmem &&
              tp3::couple_split_configure(t, tc) == cudaSuccess;
   cudaGetLastError();
-  if ((e = encode_2d(c, &c->maps.b_hi, (void*)tc.Fhi, tc.KP, tc.NP, 256, false)) != cudaSuccess ||
-      (e = encode_2d(c, &c->maps.b_lo, (void*)tc.Flo, tc.KP, tc.NP, 256, false)) != cudaSuccess ||
-      (e = encode_2d(c, &c->maps32.b_hi, (void*)tc.Fhi32, tc.KP, tc.NP, 256, true)) != cudaSuccess ||
-      (e = encode_2d(c, &c->maps32.b_lo, (void*)tc.Flo32, tc.KP, tc.NP, 256, true)) != cudaSuccess)
+  if ((e = encode_2d(c, &c->maps.b_hi, (void*)tc.Fhi, tc.KP, tc.NP, 128, false)) != cudaSuccess ||
+      (e = encode_2d(c, &c->maps.b_lo, (void*)tc.Flo, tc.KP, tc.NP, 128, false)) != cudaSuccess ||
+      (e = encode_2d(c, &c->maps32.b_hi, (void*)tc.Fhi32, tc.KP, tc.NP, 128, true)) != cudaSuccess ||
+      (e = encode_2d(c, &c->maps32.b_lo, (void*)tc.Flo32, tc.KP, tc.NP, 128, true)) != cudaSuccess)
     return "tensor map encoding of F failed";
   cudaGetLastError();
   if (!tc.fused_ok && !tc.split_ok) return "coupling tile exceeds shared memory";

@@ -564,10 +564,11 @@ constexpr int kBBytes = kBN * kBK * 2;        // 16 KB
 constexpr int kStageBytes = 2 * kABytes + 2 * kBBytes;  // 48 KB
 constexpr int kEpiWarps = 8;
 constexpr int kThreads = 64 + 32 * kEpiWarps;  // producer warp, MMA warp, 8 epilogue warps
-// Instruction descriptor: F32 accumulator, both operands K-major, M = 128, N = 256;
+constexpr int kBNh = kBN / 2;                  // columns of a TMA box of B, and of a narrow MMA
+// Instruction descriptor: F32 accumulator, both operands K-major, M = 128, N = n;
 // operand format 1 = BF16 (kind::f16), 2 = TF32 (kind::tf32).
-__host__ __device__ constexpr uint32_t idesc_m128_n256(uint32_t fmt) {
-  return (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(kBN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+__host__ __device__ constexpr uint32_t idesc_m128(uint32_t fmt, int n) {
+  return (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
 }
 
 constexpr int kStorePitch = 17;  // floats per row of a warp's 32 x 16 store tile
@@ -648,7 +649,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_angular_tc(
           if (!mbar_wait(&hd->empty[s], ph ^ 1u, abort_flag, err)) break;
           last[s] = it;
           uint8_t* st = stages + s * kStageBytes;
-          mbar_expect_tx(&hd->full[s], kStageBytes);
+          const int nb = Gu - h * kBN > kBNh ? 2 : 1;  // boxes of 128 grid points in this half
+          mbar_expect_tx(&hd->full[s], 2 * kABytes + nb * kBBytes);
           if (AMN) {
             const int y = prop * KP + kc * kbk;  // order row of T[lt][ki]
 #pragma unroll
@@ -660,8 +662,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_angular_tc(
             tma_load_2d(st, &tmA_hi, &hd->full[s], kc * kbk, row0);
             tma_load_2d(st + kABytes, &tmA_lo, &hd->full[s], kc * kbk, row0);
           }
-          tma_load_2d(st + 2 * kABytes, &tmB_hi, &hd->full[s], kc * kbk, h * kBN);
-          tma_load_2d(st + 2 * kABytes + kBBytes, &tmB_lo, &hd->full[s], kc * kbk, h * kBN);
+          for (int g = 0; g < nb; ++g) {
+            tma_load_2d(st + 2 * kABytes + g * (kBBytes / 2), &tmB_hi, &hd->full[s], kc * kbk, h * kBN + g * kBNh);
+            tma_load_2d(st + 2 * kABytes + kBBytes + g * (kBBytes / 2), &tmB_lo, &hd->full[s], kc * kbk,
+                        h * kBN + g * kBNh);
+          }
         }
       }
       if (*abort_flag) {
@@ -678,9 +683,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_angular_tc(
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     if (lane == 0) {
-      const uint32_t idesc = idesc_m128_n256(TF32 ? 2u : 1u) | (AMN ? (1u << 15) : 0u);  // bit 15: A MN-major
       int it = 0;
       for (int h = 0; h < nhalf && !*abort_flag; ++h) {
+        const uint32_t idesc = idesc_m128(TF32 ? 2u : 1u, Gu - h * kBN > kBNh ? kBN : kBNh) |
+                               (AMN ? (1u << 15) : 0u);  // bit 15: A MN-major
         const uint32_t dt = tmem + (uint32_t)(h * kBN);
         for (int kc = 0; kc < nk; ++kc, ++it) {
           const int s = it % kStages;
@@ -720,6 +726,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_angular_tc(
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       for (int cc = 0; cc < 4; ++cc) {
         const int col = h * kBN + cblk * 128 + cc * 32;
+        if (col >= Gu) break;  // points past the grid contribute nothing
         float v[32];
         tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)col, v);
         const float* qrow = qt + ((size_t)mtile * Gu) * kBM + r;
@@ -838,7 +845,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_angular_tp(
           if (!mbar_wait(&hd->empty[s], ph ^ 1u, abort_flag, err)) break;
           last[s] = it;
           uint8_t* st = stages + s * kStageBytes;
-          mbar_expect_tx(&hd->full[s], kStageBytes);
+          const int nb = Gu - h * kBN > kBNh ? 2 : 1;  // boxes of 128 grid points in this half
+          mbar_expect_tx(&hd->full[s], 2 * kABytes + nb * kBBytes);
           if (AMN) {
             const int y = prop * KP + kc * kbk;
 #pragma unroll
@@ -850,8 +858,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_angular_tp(
             tma_load_2d(st, &tmA_hi, &hd->full[s], kc * kbk, row0);
             tma_load_2d(st + kABytes, &tmA_lo, &hd->full[s], kc * kbk, row0);
           }
-          tma_load_2d(st + 2 * kABytes, &tmB_hi, &hd->full[s], kc * kbk, h * kBN);
-          tma_load_2d(st + 2 * kABytes + kBBytes, &tmB_lo, &hd->full[s], kc * kbk, h * kBN);
+          for (int g = 0; g < nb; ++g) {
+            tma_load_2d(st + 2 * kABytes + g * (kBBytes / 2), &tmB_hi, &hd->full[s], kc * kbk, h * kBN + g * kBNh);
+            tma_load_2d(st + 2 * kABytes + kBBytes + g * (kBBytes / 2), &tmB_lo, &hd->full[s], kc * kbk,
+                        h * kBN + g * kBNh);
+          }
         }
       }
       if (*abort_flag) {
@@ -867,7 +878,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_angular_tp(
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     if (lane == 0) {
-      const uint32_t idesc = idesc_m128_n256(TF32 ? 2u : 1u) | (AMN ? (1u << 15) : 0u);
       int it = 0, i = 0;
       for (int u = blockIdx.x; u < nunits && !*abort_flag; u += gridDim.x) {
         int prop, mtile, h;
@@ -877,6 +887,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_angular_tp(
         if (!mbar_wait(&tmem_empty[b], (uint32_t)(((i >> 1) & 1) ^ 1), abort_flag, err)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t dt = tmem + (uint32_t)(b * kBN);
+        const uint32_t idesc = idesc_m128(TF32 ? 2u : 1u, Gu - h * kBN > kBNh ? kBN : kBNh) | (AMN ? (1u << 15) : 0u);
         bool ok = true;
         for (int kc = 0; kc < nk; ++kc, ++it) {
           const int s = it % kStages;
@@ -925,6 +936,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_angular_tp(
       for (int cc = 0; cc < 4; ++cc) {
         const int col = cblk * 128 + cc * 32;  // column inside the half
         const int u0 = h * kBN + col;          // unique grid point of column 0
+        if (u0 >= Gu) break;                   // points past the grid contribute nothing
         float v[32];
         if (STORE) {
           tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * kBN + col), v);
@@ -1048,61 +1060,87 @@ __device__ __forceinline__ double slab_log(const double x, const SlabLog* __rest
   return fma(ed, ln2_hi, chi) + (r + fma(p, r2, fma(ed, ln2_lo, clo)));  // the first sum is exact
 }
 
+// (double)x by integer arithmetic (exact); zeros, subnormals and non-finite values go through
+// the conversion, which runs at FP64 rate.
+__device__ __forceinline__ double widen(const float x) {
+  const uint32_t u = __float_as_uint(x);
+  const uint32_t e = (u >> 23) & 255;
+  if (e == 0 || e == 255) return (double)x;
+  return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + (896u << 20))), (int)(u << 29));
+}
+
 // Energies from the persistent kernel's partial sums [klp][nhalf][2][2] per proposal: slab terms
 // tf (Qs log(mult Sp) - Sql) in FP64 and their deterministic compensated sum, in one cluster of
-// kFinCtas CTAs per proposal (the first rag[prop].klen terms of a ragged batch).  The sum is that
+// CTAS CTAs per proposal (the first rag[prop].klen terms of a ragged batch).  The sum is that
 // of 256 accumulators, accumulator t taking the terms t, t + 256, .., and a tree over them; CTA r
-// owns accumulators 32 r .. 32 r + 31 and their terms, CTA 0 gathers them through distributed
-// shared memory.  Bound by FP64 (two lanes per clock and SM), hence several SMs a proposal: at
-// K = 26 one proposal took 6.5 + 15 us as a kernel of terms and a kernel of one CTA that summed.
-constexpr int kFinCtas = 8, kFinRows = 16;
-__global__ void __cluster_dims__(kFinCtas, 1, 1) __launch_bounds__(128)
+// owns 256 / CTAS consecutive accumulators and their terms, CTA 0 gathers them through
+// distributed shared memory.  Bound by FP64 (two lanes per clock and SM), hence eight SMs for each
+// proposal of a small batch (at K = 26 one proposal took 6.5 + 15 us as a kernel of terms and a
+// kernel of one CTA that summed); a batch that fills the SMs by itself takes one CTA each.
+constexpr int kFinRows = 16;
+template <int CTAS>
+__global__ void __launch_bounds__(128)
     k_finalize_parts(const float* __restrict__ part, int klp, int klength, int nhalf, const double* __restrict__ Qs,
                      const double* __restrict__ tf, int mult, const SlabLog* __restrict__ logtab, double* __restrict__ E,
                      const RagInfo* __restrict__ rag) {
-  __shared__ double term[kFinRows][32], ss[256], sc[256];
-  const int prop = blockIdx.y, rank = blockIdx.x, lane = threadIdx.x & 31;
+  constexpr int NA = 256 / CTAS;                   // accumulators of this CTA
+  constexpr int ROWS = kFinRows * 32 / NA < 2 ? 2 : kFinRows * 32 / NA;
+  __shared__ double term[ROWS][NA], ss[256], sc[256];
+  const int prop = blockIdx.y, rank = blockIdx.x;
   int nk = klength;
   if (rag) {
     nk = rag[prop].klen;
     Qs += (size_t)rag[prop].hist * klength;
   }
   const float4* p4 = reinterpret_cast<const float4*>(part) + (size_t)prop * klp * nhalf;
-  const int k0 = 32 * rank + lane;
-  double s = 0.0, c = 0.0;
-  for (int j0 = 0; 256 * j0 + 32 * rank < nk; j0 += kFinRows) {
-    for (int j = threadIdx.x >> 5; j < kFinRows; j += 4) {
-      const int ki = k0 + 256 * (j0 + j);
-      if (ki >= nk) break;
+  const int a0 = NA * rank;
+  double s[(NA + 127) / 128] = {}, c[(NA + 127) / 128] = {};
+  for (int j0 = 0; 256 * j0 + a0 < nk; j0 += ROWS) {
+    for (int i = threadIdx.x; i < ROWS * NA; i += 128) {
+      const int j = i / NA, ki = a0 + i % NA + 256 * (j0 + j);
+      if (ki >= nk) continue;
       double Sp = 0.0, Sq = 0.0;
       for (int h = 0; h < nhalf; ++h) {
         const float4 a = p4[(size_t)ki * nhalf + h];  // (Sp, Sql) of column blocks 0 and 1
-        Sp += (double)a.x + (double)a.z;
-        Sq += (double)a.y + (double)a.w;
+        Sp += widen(a.x) + widen(a.z);
+        Sq += widen(a.y) + widen(a.w);
       }
-      term[j][lane] = tf[ki] * (Qs[ki] * slab_log((double)mult * Sp, logtab) - Sq);
+      term[j][i % NA] = tf[ki] * (Qs[ki] * slab_log((double)mult * Sp, logtab) - Sq);
     }
     __syncthreads();
-    if (threadIdx.x < 32)
-      for (int j = 0; j < kFinRows && k0 + 256 * (j0 + j) < nk; ++j) {
-        double t, err;
-        two_sum(s, term[j][lane], t, err);
-        s = t;
-        c += err;
-      }
+#pragma unroll
+    for (int q = 0; q < (NA + 127) / 128; ++q) {
+      const int a = threadIdx.x + 128 * q;
+      if (a < NA)
+        for (int j = 0; j < ROWS && a0 + a + 256 * (j0 + j) < nk; ++j) {
+          double t, err;
+          two_sum(s[q], term[j][a], t, err);
+          s[q] = t;
+          c[q] += err;
+        }
+    }
     __syncthreads();
   }
-  if (threadIdx.x < 32) {
-    const uint32_t as = smem_u32(&ss[k0]), ac = smem_u32(&sc[k0]);
-    asm volatile(
-        "{\n\t.reg .b32 a;\n\t"
-        "mapa.shared::cluster.u32 a, %0, 0;\n\tst.shared::cluster.f64 [a], %2;\n\t"
-        "mapa.shared::cluster.u32 a, %1, 0;\n\tst.shared::cluster.f64 [a], %3;\n\t}" ::"r"(as),
-        "r"(ac), "d"(s), "d"(c)
-        : "memory");
+  if (CTAS == 1) {
+#pragma unroll
+    for (int q = 0; q < (NA + 127) / 128; ++q) {
+      ss[threadIdx.x + 128 * q] = s[q];
+      sc[threadIdx.x + 128 * q] = c[q];
+    }
+    __syncthreads();
+  } else {
+    if (threadIdx.x < NA) {
+      const uint32_t as = smem_u32(&ss[a0 + threadIdx.x]), ac = smem_u32(&sc[a0 + threadIdx.x]);
+      asm volatile(
+          "{\n\t.reg .b32 a;\n\t"
+          "mapa.shared::cluster.u32 a, %0, 0;\n\tst.shared::cluster.f64 [a], %2;\n\t"
+          "mapa.shared::cluster.u32 a, %1, 0;\n\tst.shared::cluster.f64 [a], %3;\n\t}" ::"r"(as),
+          "r"(ac), "d"(s[0]), "d"(c[0])
+          : "memory");
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (rank != 0) return;
   }
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-  if (rank != 0) return;
   for (int h = 128; h > 0; h >>= 1) {
     if (threadIdx.x < h) {
       double t, err;
@@ -1281,8 +1319,22 @@ cudaError_t launch_angular_persistent(const DevTables& t, const TcTables& tc, co
 
 cudaError_t launch_finalize_parts(const DevTables& t, const TcTables& tc, int n, const float* part, const double* Qs,
                                   double* E, cudaStream_t s, const RagInfo* rag) {
-  k_finalize_parts<<<dim3(kFinCtas, n), 128, 0, s>>>(part, t.klp, t.klength, tc.nhalf, Qs, t.tf, t.mult, tc.logtab, E, rag);
-  return cudaGetLastError();
+  // eight SMs a proposal until the batch has about one proposal per SM
+  if (n >= tc.nsm / 2) {
+    k_finalize_parts<1><<<dim3(1, n), 128, 0, s>>>(part, t.klp, t.klength, tc.nhalf, Qs, t.tf, t.mult, tc.logtab, E, rag);
+    return cudaGetLastError();
+  }
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 8;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(8, n);
+  cfg.blockDim = dim3(128);
+  cfg.stream = s;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_finalize_parts<8>, part, t.klp, t.klength, tc.nhalf, Qs, t.tf, t.mult, tc.logtab, E, rag);
 }
 
 }  // namespace tp3
