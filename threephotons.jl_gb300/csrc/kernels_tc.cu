@@ -927,19 +927,31 @@ __global__ void __launch_bounds__(kThreads, 1) k_angular_tp(
       int prop, mtile, h;
       if (!decode(u, prop, mtile, h)) continue;
       const int b = i & 1;
-      if (!mbar_wait(&hd->tmem_full[b], (uint32_t)((i >> 1) & 1), abort_flag, err)) break;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      // a half of one 128-column block is drained by the two groups of four warps in turn
+      const bool narrow = Gu - h * kBN <= kBNh;
+      const bool mine = !narrow || cblk == (i & 1);
+      const int cb = narrow ? 0 : cblk;
+      const int ub = h * kBN + cb * kBNh;  // unique grid point of the block's first column
+      const int nch = mine ? min(4, (Gu - ub + 31) / 32) : 0;
       const float* qrow =
           STORE ? nullptr : qt + (rag ? (size_t)rag[prop].hist * klp * Gu : 0) + ((size_t)mtile * Gu) * kBM + r;
       const int ki = mtile * kBM + r;
       float sp = 0.f, sq = 0.f, csp = 0.f, csq = 0.f;
-      for (int cc = 0; cc < 4; ++cc) {
-        const int col = cblk * 128 + cc * 32;  // column inside the half
-        const int u0 = h * kBN + col;          // unique grid point of column 0
-        if (u0 >= Gu) break;                   // points past the grid contribute nothing
+      // histogram values one run of 32 columns ahead, the first before the accumulator is ready
+      float qn[32];
+      auto fetch = [&](int u0) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) qn[j] = u0 + j < Gu ? qrow[(size_t)(u0 + j) * kBM] : 0.f;
+      };
+      if (!STORE && nch > 0) fetch(ub);
+      if (!mbar_wait(&hd->tmem_full[b], (uint32_t)((i >> 1) & 1), abort_flag, err)) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+      for (int cc = 0; cc < nch; ++cc) {
+        const int u0 = ub + cc * 32;
         float v[32];
+        tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * kBN + cb * kBNh + cc * 32), v);
         if (STORE) {
-          tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * kBN + col), v);
           // unique points are the first N^2 / 2 grid points (folded grid) or all of them
           float* tile = reinterpret_cast<float*>(hd + 1) + ew * (32 * kStorePitch);
           const int N2 = N * N, ki0 = mtile * kBM + quarter * 32;
@@ -967,11 +979,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_angular_tp(
         }
         float q[32];
 #pragma unroll
-        for (int j = 0; j < 32; ++j) q[j] = u0 + j < Gu ? qrow[(size_t)(u0 + j) * kBM] : 0.f;
-        tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * kBN + col), v);
+        for (int j = 0; j < 32; ++j) q[j] = qn[j];
+        if (cc + 1 < nch) fetch(u0 + 32);
+        const int left = Gu - u0;
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
-          if (u0 + j < Gu) {
+          if (j < left) {
             const float p = fmaxf(v[j], 1e-30f);
             const float y1 = p - csp;
             const float t1 = sp + y1;
@@ -987,9 +1000,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_angular_tp(
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&tmem_empty[b])) : "memory");
-      if (!STORE)
-        reinterpret_cast<float2*>(part)[(((size_t)prop * klp + ki) * nhalf + h) * 2 + cblk] =
-            make_float2(sp - csp, sq - csq);
+      if (!STORE && mine) {
+        float2* o = reinterpret_cast<float2*>(part) + (((size_t)prop * klp + ki) * nhalf + h) * 2;
+        o[cb] = make_float2(sp - csp, sq - csq);
+        if (narrow) o[1] = make_float2(0.f, 0.f);
+      }
       ++i;
     }
   }
