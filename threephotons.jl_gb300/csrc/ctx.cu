@@ -464,11 +464,18 @@ std::string setup_tc(tp3_ctx* c) {
       std::vector<int2> ko;
       tp3::build_lane_units(b.K, ut, sl, ko, ln.stage);
       tp3::lane_pick_warps(ln);
-      if (ln.ok) ln.maxz = std::max(1, tp3::lane_tasks(ko[b.K].y, maxs) / ln.nw);
+      ln.tasks = tp3::lane_tasks(ko[b.K].y, maxs);
+      std::vector<int> by_work(pbs.size()), by_form;
+      for (int i = 0; i < (int)pbs.size(); ++i) by_work[i] = i;
+      for (int form = 1; form >= 0; --form)
+        for (int i = 0; i < (int)pbs.size(); ++i)
+          if (lbl[i].swap == form) by_form.push_back(i);
       if (ln.ok && ((e = upload(c, lbl, &ln.blks)) != cudaSuccess || (e = upload(c, lq, &ln.quads)) != cudaSuccess ||
                     (e = upload(c, lg, &ln.gcols)) != cudaSuccess || (e = upload(c, lw, &ln.w)) != cudaSuccess ||
                     (e = upload(c, ut, &ln.utab)) != cudaSuccess || (e = upload(c, sl, &ln.slots)) != cudaSuccess ||
                     (e = upload(c, ko, &ln.kofs)) != cudaSuccess ||
+                    (e = upload(c, by_work, &ln.by_work)) != cudaSuccess ||
+                    (e = upload(c, by_form, &ln.by_form)) != cudaSuccess ||
                     (e = tp3::lane_configure()) != cudaSuccess))
         return std::string("lane coupling: ") + cudaGetErrorString(e);
     }
@@ -1471,7 +1478,7 @@ int tp3_energy_batch(tp3_ctx* c, int n, const double* coeffs, double* E) {
   if (c->host_direct) {
     // the device reads the caller's buffer in place: no host packing and no staging copy, and
     // none on the device either where the gather reads every value once
-    if (is_tc(c->mode) && c->tc.use_lane && tp3::gather_lane_once(t)) {
+    if (is_tc(c->mode) && c->tc.use_lane) {
       if (int r = run_energy(c, n, src, c->h_E)) return r;
     } else {
       const int64_t total = (int64_t)n * t.K * t.nc;

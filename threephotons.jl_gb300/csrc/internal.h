@@ -164,9 +164,11 @@ struct LaneTables {
   int nw = 0, ctas = 0;  // warps per CTA, CTAs per SM
   int ps = 0, c3row = 0; // shells per coefficient row (32 or 64), float4 per c_k3 row
   int crows = 0, wmax = 0, c3rows = 0, stage = 0;
-  int maxz = 1;          // CTAs over which one block's tasks can spread
+  int tasks = 1;         // tasks of the block of most orders
   size_t smem = 0;
-  const LaneBlock* blks = nullptr;
+  const LaneBlock* blks = nullptr;  // heaviest first
+  const int* by_work = nullptr;     // [n_pb] 0, 1, ..
+  const int* by_form = nullptr;     // [n_pb] blocks of one loop form (c_k2 stepped, c_k1 stepped) together
   const LaneQuad* quads = nullptr;
   const int4* gcols = nullptr;  // [n_pb][16] general path, per order: first quad, quads, first 3j float4, count
   const float4* w = nullptr;
@@ -313,7 +315,6 @@ void build_lane_units(int K, std::vector<uint32_t>& utab, std::vector<uint32_t>&
 int lane_tasks(int nu, int nl3);
 void lane_pick_warps(LaneTables& lt);
 cudaError_t lane_configure();
-bool gather_lane_once(const DevTables& t);
 cudaError_t launch_gather_lane(const DevTables& t, const TcTables& tc, int n, const double2* coeff, CoeffLayout lay,
                                float2* ct, float* c3p, int* sym, cudaStream_t s, const RagInfo* rag = nullptr);
 // T32 (nullable): FP32 T as [ki][n_ltp] rows, or [lt][klp] when t32maj; Thi null: T32 only.

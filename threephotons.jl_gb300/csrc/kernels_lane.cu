@@ -324,13 +324,14 @@ __device__ __forceinline__ void lane_task(const LaneView& V, bool swap, bool sym
   }
 }
 
-// grid: (n, n_pb, Z); block 32 x warps; dynamic shared memory LaneTables::smem.
-// CTA (p, b, z) takes the tasks z, z + Z, .. of block b of proposal p: Z > 1 spreads the
+// grid: (n, Z, n_pb); block 32 x warps; dynamic shared memory lane_smem_bytes.
+// CTA (p, z, b) takes the tasks z, z + Z, .. of block order[b] of proposal p: Z > 1 spreads the
 // tasks of a small batch over the SMs.  Proposals run fastest, so an SM's CTAs are mostly on
 // one block and their warps in the same code.
 template <int PS>
 __global__ void __launch_bounds__(32 * kLaneMaxWarps, 1) k_couple_lane(
-    const float2* __restrict__ ct, const float4* __restrict__ c3p, int K, int nc, const int* __restrict__ coff, const LaneBlock* __restrict__ blks, const LaneQuad* __restrict__ quads,
+    const float2* __restrict__ ct, const float4* __restrict__ c3p, int K, int nc, const int* __restrict__ order,
+    const int* __restrict__ coff, const LaneBlock* __restrict__ blks, const LaneQuad* __restrict__ quads,
     const int4* __restrict__ gcols, const float4* __restrict__ wtab, const uint32_t* __restrict__ utab,
     const uint32_t* __restrict__ slots, const int2* __restrict__ kofs, int crows, int wmax, int c3rows, int stage_len,
     const int* __restrict__ symflags, LaneOut out, const RagInfo* __restrict__ rag, int* __restrict__ err) {
@@ -342,7 +343,8 @@ __global__ void __launch_bounds__(32 * kLaneMaxWarps, 1) k_couple_lane(
   __shared__ int s_abort;
   const int prop = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const LaneBlock fb = blks[blockIdx.y];
+  const int blk = order[blockIdx.z];
+  const LaneBlock fb = blks[blk];
   int Kp = K;
   bool skip = false;
   int klen = 0;
@@ -360,7 +362,7 @@ __global__ void __launch_bounds__(32 * kLaneMaxWarps, 1) k_couple_lane(
   if (out.T32) out.T32 += (size_t)prop * out.klp * out.ldT32;
   if (skip) {
     // absent orders: the block's l-triples are zero for this proposal's scored rows
-    for (int i = threadIdx.x + blockIdx.z * blockDim.x; i < klen * fb.nl3; i += blockDim.x * gridDim.z) {
+    for (int i = threadIdx.x + blockIdx.y * blockDim.x; i < klen * fb.nl3; i += blockDim.x * gridDim.y) {
       const int s = i / klen, ki = i - s * klen, lt = fb.lt_base + s;
       if (out.hi) {
         const size_t at = out.ltmaj ? (size_t)lt * out.klp + ki : (size_t)ki * out.KP + lt;
@@ -379,7 +381,7 @@ __global__ void __launch_bounds__(32 * kLaneMaxWarps, 1) k_couple_lane(
   const bool sym = symflags[prop] != 0;
   const int2 ko = kofs[Kp];
   const int nu = ko.y;
-  if ((int)blockIdx.z >= (sym ? nu * fb.nl3 : nu)) return;  // more CTAs than tasks
+  if ((int)blockIdx.y >= (sym ? nu * fb.nl3 : nu)) return;  // more CTAs than tasks
   float2* C1 = reinterpret_cast<float2*>(lane_smem);
   float2* C2 = C1 + (size_t)crows * ps;
   float4* W = reinterpret_cast<float4*>(C2 + (size_t)crows * ps) + 8;  // a rounded-up run may start before its row
@@ -411,7 +413,7 @@ __global__ void __launch_bounds__(32 * kLaneMaxWarps, 1) k_couple_lane(
   V.quads = s_quads;
   for (int pass = 0; pass < passes; ++pass) {
     int4 g = make_int4(fb.q0, fb.nq, fb.w0, fb.wn);
-    if (!sym) g = gcols[blockIdx.y * 16 + pass];
+    if (!sym) g = gcols[blk * 16 + pass];
     if (pass > 0) {
       __syncthreads();  // the previous order's reads are done
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -450,7 +452,7 @@ __global__ void __launch_bounds__(32 * kLaneMaxWarps, 1) k_couple_lane(
     for (;;) {
       int t = 0;
       if (lane == 0) t = atomicAdd(&s_next[pass], 1);
-      t = __shfl_sync(0xffffffffu, t, 0) * gridDim.z + blockIdx.z;
+      t = __shfl_sync(0xffffffffu, t, 0) * gridDim.y + blockIdx.y;
       const int u = t / nrun;
       if (u >= nu) break;
       int s_lo = pass, w = 1;
@@ -489,43 +491,49 @@ __device__ __forceinline__ double flip(const double x, bool neg) {
   return neg ? __hiloint2double(__double2hiint(x) ^ (int)0x80000000, __double2loint(x)) : x;
 }
 
-// Coefficients for the lane-owned coupling: one CTA per proposal reads the FP64 values once
-// (each warp one shell at a time, all of its loads in flight together), checks the
-// real-function relation c[l,-m] = (-1)^m conj c[l,m] to 1e-10 of the shell's largest
-// coefficient, and writes two FP32 layouts with the shells contiguous: ct [nc][ps] (c_k1 and
-// c_k2) and c3p [nc][c3row] (c_k3: four real parts, four imaginary parts per quad of shells).
-// sym = 1 when every shell satisfies the relation; m < 0 is then rebuilt from m >= 0 so that
-// it holds exactly in FP32.  keep: all shells stay in shared memory between the check and the
-// conversion (else they are read again).  grid: n; block 1024.
-// Bound by the latency of one round of loads and the stores of one SM.  FP64 arithmetic is
-// kept for shells that hold the relation only approximately: with it everywhere (as in
-// k_gather_sym) a proposal of K = 26, L = 18 took 33 us.
-__global__ void __launch_bounds__(1024, 1) k_gather_lane(int K, int nc, int ncoef, const int* __restrict__ csean,
-                                                         const int* __restrict__ cm, const int* __restrict__ cmir,
-                                                         const int* __restrict__ cl, const double2* __restrict__ coeff,
-                                                         float2* __restrict__ ct, float* __restrict__ c3p, int ps,
-                                                         int c3row, int* __restrict__ sym, int keep,
-                                                         const RagInfo* __restrict__ rag) {
+// Coefficients for the lane-owned coupling: one cluster of kGatherCtas CTAs per proposal, four
+// shells (a quad) a CTA and round, reads the FP64 values once, checks the real-function relation
+// c[l,-m] = (-1)^m conj c[l,m] to 1e-10 of the shell's largest coefficient, and writes two FP32
+// layouts with the shells contiguous: ct [nc][ps] (c_k1 and c_k2) and c3p [nc][c3row] (c_k3: four
+// real parts, four imaginary parts per quad of shells).  sym = 1 when every shell satisfies the
+// relation; m < 0 is then rebuilt from m >= 0 so that it holds exactly in FP32.
+// grid: (kGatherCtas, n); block 256; dynamic shared memory ROUNDS x 4 (nc | 1) double2.
+// Bound by the latency of one round of loads (device memory or the caller's host array).  FP64
+// arithmetic is kept for shells that hold the relation only approximately: with it everywhere
+// and one CTA a proposal (as in k_gather_sym) K = 26, L = 18 took 34 us.
+constexpr int kGatherCtas = 8;
+template <int ROUNDS>
+__global__ void __cluster_dims__(kGatherCtas, 1, 1) __launch_bounds__(256)
+    k_gather_lane(int K, int nc, int ncoef, const int* __restrict__ csean, const int* __restrict__ cm,
+                  const int* __restrict__ cmir, const int* __restrict__ cl, const double2* __restrict__ coeff,
+                  float2* __restrict__ ct, float* __restrict__ c3p, int* __restrict__ sym, const RagInfo* __restrict__ rag) {
   extern __shared__ __align__(16) double2 gl_smem[];
-  const int prop = blockIdx.x;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  __shared__ int s_ok[kGatherCtas];
+  constexpr int ps = 32 * ROUNDS, c3row = ps / 2;
+  const int prop = blockIdx.y, rank = blockIdx.x;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ld = nc | 1;
   const double2* cp = coeff + (size_t)prop * K * ncoef;
-  int ok = 1;
-  for (int k = warp; k < K; k += nw) {
-    double2* row = gl_smem + (size_t)(keep ? k : warp) * ld;
-    const double2* ck = cp + (size_t)k * ncoef;
-#pragma unroll 8
-    for (int c = lane; c < nc; c += 32) row[c] = ck[csean[c]];
-    __syncwarp();
-    // exact, finite mirror images need no tolerance
-    bool exact = true;
-    for (int c = lane; c < nc; c += 32) {
-      const int m = cm[c];
+  for (int rd = 0; rd < ROUNDS; ++rd) {
+    const int k0 = 4 * (rank + kGatherCtas * rd), nk = min(4, K - k0);
+#pragma unroll 4
+    for (int i = threadIdx.x; i < nk * nc; i += 256) {
+      const int kk = i / nc, c = i - kk * nc;
+      gl_smem[(4 * rd + kk) * ld + c] = cp[(size_t)(k0 + kk) * ncoef + csean[c]];
+    }
+  }
+  __syncthreads();
+  // exact, finite mirror images need no tolerance
+  int exact = 1;
+  for (int rd = 0; rd < ROUNDS; ++rd) {
+    const int nk = min(4, K - 4 * (rank + kGatherCtas * rd));
+    for (int i = threadIdx.x; i < nk * nc; i += 256) {
+      const int kk = i / nc, c = i - kk * nc, m = cm[c];
       if (m < 0) continue;
+      const double2* row = gl_smem + (4 * rd + kk) * ld;
       const double2 a = row[c];
       if (m == 0) {
-        exact &= ((__double_as_longlong(a.y) << 1) == 0);
+        exact &= (__double_as_longlong(a.y) << 1) == 0;
       } else {
         const double2 b = row[cmir[c]];
         const bool odd = m & 1;
@@ -534,46 +542,60 @@ __global__ void __launch_bounds__(1024, 1) k_gather_lane(int K, int nc, int ncoe
                  (__double2hiint(a.x) & 0x7ff00000) != 0x7ff00000 && (__double2hiint(a.y) & 0x7ff00000) != 0x7ff00000;
       }
     }
-    if (!__all_sync(0xffffffffu, exact)) {
-      double amax = 0.0;
+  }
+  int ok = 1;
+  if (!__syncthreads_and(exact) && warp < 4 * ROUNDS) {  // one warp a shell
+    const double2* row = gl_smem + warp * ld;
+    const bool live = 4 * (rank + kGatherCtas * (warp >> 2)) + (warp & 3) < K;
+    double amax = 0.0;
+    if (live)
       for (int c = lane; c < nc; c += 32) amax = fmax(amax, fabs(row[c].x) + fabs(row[c].y));
-      for (int o = 16; o > 0; o >>= 1) amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-      const double tol = 1e-10 * amax;
-      for (int c = lane; c < nc; c += 32) {
-        const int m = cm[c];
-        if (m < 0) continue;
-        const double2 a = row[c];
-        if (m == 0) {
-          ok &= fabs(a.y) <= tol;
-        } else {
-          const double2 b = row[cmir[c]];
-          const double sg = (m & 1) ? -1.0 : 1.0;
-          ok &= fabs(b.x - sg * a.x) + fabs(b.y + sg * a.y) <= tol;
-        }
+    for (int o = 16; o > 0; o >>= 1) amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    const double tol = 1e-10 * amax;
+    for (int c = lane; live && c < nc; c += 32) {
+      const int m = cm[c];
+      if (m < 0) continue;
+      const double2 a = row[c];
+      if (m == 0) {
+        ok &= fabs(a.y) <= tol;
+      } else {
+        const double2 b = row[cmir[c]];
+        const double sg = (m & 1) ? -1.0 : 1.0;
+        ok &= fabs(b.x - sg * a.x) + fabs(b.y + sg * a.y) <= tol;
       }
     }
-    __syncwarp();
   }
-  const int s = __syncthreads_and(ok);
-  if (threadIdx.x == 0) sym[prop] = s;
+  ok = __syncthreads_and(ok);
+  if (threadIdx.x < kGatherCtas) {  // to every CTA of the cluster
+    asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\tst.shared::cluster.u32 [a], %2;\n\t}" ::"r"(
+                     smem_u32(&s_ok[rank])),
+                 "r"((uint32_t)threadIdx.x), "r"(ok)
+                 : "memory");
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  int s = 1;
+#pragma unroll
+  for (int i = 0; i < kGatherCtas; ++i) s &= s_ok[i];
+  if (rank == 0 && threadIdx.x == 0) sym[prop] = s;
   int Lp = 1 << 30, Kp = K;
   if (rag) { Lp = rag[prop].L; Kp = rag[prop].K; }
   float2* ctp = ct + (size_t)prop * nc * ps;
   float* c3o = c3p + (size_t)prop * nc * (4 * c3row);
-  for (int c = warp; c < nc; c += nw) {
-    const int m = cm[c];
-    const bool mir = s && m < 0, odd = m & 1;
-    const int cs = mir ? cmir[c] : c;
-    const bool absent = cl[c] > Lp;
-    for (int k = lane; k < ps; k += 32) {
+  for (int rd = 0; rd < ROUNDS; ++rd) {
+    const int q = rank + kGatherCtas * rd;
+#pragma unroll 2
+    for (int i = threadIdx.x; i < 4 * nc; i += 256) {
+      const int c = i >> 2, kk = i & 3, k = 4 * q + kk;
+      const int m = cm[c];
+      const bool mir = s && m < 0, odd = m & 1;
       float2 v = make_float2(0.f, 0.f);  // absent orders / shells
-      if (!absent && k < Kp) {
-        const double2 a = keep ? gl_smem[(size_t)k * ld + cs] : cp[(size_t)k * ncoef + csean[cs]];
+      if (cl[c] <= Lp && k < Kp) {
+        const double2 a = gl_smem[(4 * rd + kk) * ld + (mir ? cmir[c] : c)];
         v = make_float2(narrow(flip(a.x, mir && odd)), (s && m == 0) ? 0.f : narrow(flip(a.y, mir && !odd)));
       }
       ctp[(size_t)c * ps + k] = v;
       if (m >= 0 || !s) {
-        float* o = c3o + (size_t)c * (4 * c3row) + 8 * (k >> 2) + (k & 3);
+        float* o = c3o + (size_t)c * (4 * c3row) + 8 * q + kk;
         o[0] = v.x;
         o[4] = v.y;
       }
@@ -605,7 +627,7 @@ __global__ void __launch_bounds__(256) k_split_rows(const float* __restrict__ T,
   }
 }
 
-constexpr int kGatherMaxSmem = 200 * 1024;
+constexpr int kGatherMaxSmem = 8 * 1025 * 16;  // two rounds of four shells, nc <= 1024
 
 }  // namespace
 
@@ -616,12 +638,7 @@ std::string build_lane_tables(const std::vector<PairBlock>& pbs, const std::vect
                               std::vector<float4>& w, int& crows, int& wmax, int& c3rows) {
   blks.clear(); quads.clear(); gcols.clear(); w.clear();
   crows = wmax = c3rows = 0;
-  // blocks of one loop form together (c_k2 stepped, then c_k1), each heaviest first as given
-  std::vector<PairBlock> ord;
-  for (int pass = 0; pass < 2; ++pass)
-    for (const PairBlock& pb : pbs)
-      if ((pb.l1 > pb.l2) == (pass == 0)) ord.push_back(pb);
-  for (const PairBlock& pb : ord) {
+  for (const PairBlock& pb : pbs) {
     const int l1 = pb.l1, l2 = pb.l2;
     LaneBlock fb{};
     fb.l1 = l1; fb.l2 = l2; fb.l3min = pb.l3min; fb.nl3 = pb.nl3; fb.lt_base = pb.lt_base;
@@ -793,23 +810,23 @@ cudaError_t lane_configure() {
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_couple_lane<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCoupleMaxDynSmem);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_gather_lane, cudaFuncAttributeMaxDynamicSharedMemorySize, kGatherMaxSmem);
+    e = cudaFuncSetAttribute(k_gather_lane<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGatherMaxSmem);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_gather_lane<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGatherMaxSmem);
   return e;
 }
-
-// Whether the gather holds all shells of a proposal in shared memory, reading each value once.
-bool gather_lane_once(const DevTables& t) { return (size_t)(t.nc | 1) * sizeof(double2) * t.K <= (size_t)kGatherMaxSmem; }
 
 cudaError_t launch_gather_lane(const DevTables& t, const TcTables& tc, int n, const double2* coeff, CoeffLayout lay,
                                float2* ct, float* c3p, int* sym, cudaStream_t s, const RagInfo* rag) {
   const size_t row = (size_t)(t.nc | 1) * sizeof(double2);
-  const bool keep = gather_lane_once(t);
-  int nw = std::min(32, t.K);
-  if (!keep) nw = (int)std::min<size_t>(nw, kGatherMaxSmem / row);
-  nw = std::max(nw, 8);
-  const size_t smem = row * (keep ? t.K : nw);
-  k_gather_lane<<<n, nw * 32, smem, s>>>(t.K, t.nc, lay.stride, lay.map, tc.cm, tc.cmir, tc.cl, coeff, ct, c3p,
-                                         tc.lane.ps, tc.lane.c3row, sym, keep ? 1 : 0, rag);
+  auto go = [&](auto kernel, int rounds) {
+    kernel<<<dim3(kGatherCtas, n), 256, 4 * rounds * row, s>>>(t.K, t.nc, lay.stride, lay.map, tc.cm, tc.cmir, tc.cl, coeff,
+                                                               ct, c3p, sym, rag);
+  };
+  if (tc.lane.ps == 32)
+    go(k_gather_lane<1>, 1);
+  else
+    go(k_gather_lane<2>, 2);
   return cudaGetLastError();
 }
 
@@ -817,11 +834,18 @@ cudaError_t launch_couple_lane(const DevTables& t, const TcTables& tc, int n, co
                                const int* sym, void* Thi, void* Tlo, bool tf32, float* T32, bool t32maj, float* scratch,
                                cudaStream_t s, const RagInfo* rag) {
   const LaneTables& lt = tc.lane;
-  // a batch whose (block, proposal) CTAs do not fill the SMs twice over spreads each block's
-  // tasks over Z CTAs, down to one task per warp
+  // a batch whose (block, proposal) CTAs do not fill the SMs spreads each block's tasks over Z CTAs
+  // of four warps until they do, blocks strictly heaviest first (one proposal at L18 K26: 45 us in
+  // CTAs of eight warps over twice the slots, 35 so, 43 with four times the CTAs, which stage more)
   const int slots = 2 * tc.nsm * lt.ctas;
-  int z = 1;
-  while (z < lt.maxz && (long long)tc.n_pb * n * z < slots) ++z;
+  int z = 1, nw = lt.nw;
+  size_t smem = lt.smem;
+  if ((long long)tc.n_pb * n < slots) {
+    nw = 4;
+    smem = lane_smem_bytes(lt, nw);
+    const int maxz = std::max(1, (lt.tasks + nw - 1) / nw);
+    while (z < maxz && (long long)tc.n_pb * n * z < slots) ++z;
+  }
   // TF32 rows are split from order-major FP32 T by a kernel of its own
   const bool rows = tf32 && Thi && !T32;
   LaneOut o;
@@ -831,8 +855,8 @@ cudaError_t launch_couple_lane(const DevTables& t, const TcTables& tc, int n, co
   o.KP = tc.KP; o.klp = t.klp; o.ldT32 = t.n_ltp;
   o.tf32 = tf32; o.ltmaj = t_order_major(tc, tf32); o.t32maj = rows || t32maj;
   auto go = [&](auto kernel) {
-    kernel<<<dim3(n, tc.n_pb, z), 32 * lt.nw, lt.smem, s>>>(
-        ct, reinterpret_cast<const float4*>(c3p), t.K, t.nc, tc.coff, lt.blks, lt.quads, lt.gcols, lt.w, lt.utab, lt.slots,
+    kernel<<<dim3(n, z, tc.n_pb), 32 * nw, smem, s>>>(
+        ct, reinterpret_cast<const float4*>(c3p), t.K, t.nc, z > 1 ? lt.by_work : lt.by_form, tc.coff, lt.blks, lt.quads, lt.gcols, lt.w, lt.utab, lt.slots,
         lt.kofs, lt.crows, lt.wmax, lt.c3rows, lt.stage, sym, o, rag, tc.err);
   };
   if (lt.ps == 32)
