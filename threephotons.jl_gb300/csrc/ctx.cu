@@ -1013,22 +1013,23 @@ int tp3_ctx_create(int L, int LMAX, int N, int K, double lambda, double dq, tp3_
   *c->h_err = 0;
   if (lambda != 0.0) {
     tp3::HformTables& hf = c->tc.hf;
-    std::vector<int4> hg;
     std::vector<int2> hl, he;
     std::vector<float> hw;
-    std::vector<int> hm;
-    if (K <= 64 && tp3::hform_fits(t.n_lt, t.nc) &&
-        tp3::build_hform_tables(b.coff, K, t.n_lt, b.lt_l1.data(), b.lt_l2.data(), b.lt_l3.data(), c->qpairs, qstart, qlist,
-                                lt_of_j, w32, hg, hl, he, hw, hm)
+    std::vector<int> hm, hq;
+    const int KP = (std::max(t.nq, t.n_lt) + 31) / 32 * 32;
+    if (tp3::hform_fits(t.n_lt, t.nc, L, KP / 32 + 1) &&
+        tp3::build_hform_tables(b.coff, t.n_lt, b.lt_l1.data(), b.lt_l2.data(), b.lt_l3.data(), c->qpairs, qstart, qlist,
+                                lt_of_j, w32, KP, hl, he, hw, hm, hq)
             .empty()) {
-      if ((e = upload(c, hg, &hf.groups)) != cudaSuccess || (e = upload(c, hl, &hf.lists)) != cudaSuccess ||
-          (e = upload(c, he, &hf.entries)) != cudaSuccess || (e = upload(c, hw, &hf.wts)) != cudaSuccess ||
-          (e = upload(c, hm, &hf.slot_m)) != cudaSuccess || (e = tp3::hform_configure()) != cudaSuccess) {
+      if ((e = upload(c, hl, &hf.lists)) != cudaSuccess || (e = upload(c, he, &hf.entries)) != cudaSuccess ||
+          (e = upload(c, hw, &hf.wts)) != cudaSuccess || (e = upload(c, hm, &hf.quad_m)) != cudaSuccess ||
+          (e = upload(c, hq, &hf.quad_q)) != cudaSuccess || (e = tp3::hform_configure()) != cudaSuccess) {
         std::string msg = std::string("pair table upload: ") + cudaGetErrorString(e);
         tp3_ctx_destroy(c);
         return fail(nullptr, TP3_ERR_CUDA, msg);
       }
-      hf.ngroups = (int)hg.size();
+      hf.nunits = (int)hl.size();
+      hf.L = L;
       hf.ok = true;
     }
   }

@@ -73,13 +73,13 @@ size_t build_H_split_smem(const DevTables& t, int ppl);
 cudaError_t launch_build_H_split(const DevTables& t, int KP, int n, const float* T32, void* Hhi, void* Hlo, bool tf32,
                                  cudaStream_t s);
 // The same from order-major FP32 T ([lt][klp] a proposal), bit for bit.
-std::string build_hform_tables(const std::vector<int>& coff, int K, int n_lt, const int* lt_l1, const int* lt_l2,
+std::string build_hform_tables(const std::vector<int>& coff, int n_lt, const int* lt_l1, const int* lt_l2,
                                const int* lt_l3, const std::vector<std::pair<int, int>>& pairs,
                                const std::vector<int>& qstart, const std::vector<int>& qlist,
-                               const std::vector<int>& lt_of_j, const std::vector<float>& w, std::vector<int4>& groups,
+                               const std::vector<int>& lt_of_j, const std::vector<float>& w, int KP,
                                std::vector<int2>& lists, std::vector<int2>& entries, std::vector<float>& wts,
-                               std::vector<int>& slot_m);
-bool hform_fits(int n_lt, int nc);
+                               std::vector<int>& quad_m, std::vector<int>& quad_q);
+bool hform_fits(int n_lt, int nc, int L, int nunits);
 cudaError_t hform_configure();
 cudaError_t launch_finalize(const DevTables& t, int n, const double2* part, int ncg,
                             const double* Qs, int mult, double* E, cudaStream_t s);
@@ -182,12 +182,12 @@ struct LaneTables {
 // consecutive shell triples.
 struct HformTables {
   bool ok = false;
-  int ngroups = 0;
-  const int4* groups = nullptr;   // first shell triple, count, k1 | k2 << 8, first k3
-  const int2* lists = nullptr;    // per 32 slots: range of entries
+  int nunits = 0, L = 0;
+  const int2* lists = nullptr;    // per unit of eight quads of columns: range of entries
   const int2* entries = nullptr;  // l-triple, centres of its orders' coefficient rows (10 bits each)
-  const float* wts = nullptr;     // [entries][32]
-  const int* slot_m = nullptr;    // m1, m2, m3 of a slot (8 bits each)
+  const float* wts = nullptr;     // [entries][8 quads][4]
+  const int* quad_m = nullptr;    // [units][8][4]: m1, m2, m3 of a column (8 bits each)
+  const int* quad_q = nullptr;    // [units][8]: first column, -1 none
 };
 
 // Device tables of the tensor-core path.
