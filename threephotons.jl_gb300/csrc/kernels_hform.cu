@@ -29,6 +29,7 @@
 #include <vector>
 
 #include "internal.h"
+#include "tc_prims.cuh"
 
 namespace tp3 {
 namespace {
@@ -68,6 +69,9 @@ __global__ void __launch_bounds__(kHfThreads, 1) k_build_H_pairs(
     Ys[i] = c >= 0 && c < nc ? Ytab[(size_t)(r == 0 ? k.x : r == 1 ? k.y : k.z) * nc + c] : 0.f;
   }
   for (int i = threadIdx.x; i < nunits * 8; i += blockDim.x) Ms[i] = __ldg(quad_m + i);
+  grid_wait();
+  grid_release();
+  T32 = after_wait(T32);
   // rows of T are padded to a multiple of 16 shell triples, so a group's 16 bytes are always there
   for (int i = threadIdx.x; i < n_lt * NP; i += blockDim.x) {
     const int lt = i / NP, p = i - lt * NP;
@@ -340,18 +344,17 @@ cudaError_t launch_build_H_pairs(const DevTables& t, const TcTables& tc, int n, 
   const int threads = two ? kHfThreads / 2 : kHfThreads;
   const size_t smem = hf_smem_bytes(np, t.n_lt, t.nc, h.L, h.nunits, threads);
   auto go = [&](auto kernel) {
-    kernel<<<dim3((t.klength + 3) / 4, (n + np - 1) / np), threads, smem, s>>>(
-        T32, t.klp, (int64_t)t.klp * t.n_ltp, n, t.klength, t.n_lt, t.Ytab, t.nc, h.L, t.kl, h.lists, h.entries,
+    return launch_after(
+        kernel, dim3((t.klength + 3) / 4, (n + np - 1) / np), threads, smem, s, 1, T32, t.klp, (int64_t)t.klp * t.n_ltp, n, t.klength, t.n_lt, t.Ytab, t.nc, h.L, t.kl, h.lists, h.entries,
         reinterpret_cast<const float4*>(h.wts), reinterpret_cast<const int4*>(h.quad_m), h.quad_q, h.nunits, tc.KP,
         tf32 ? 1 : 0, Hhi, Hlo);
   };
   switch (np) {
-    case 12: go(k_build_H_pairs<12>); break;
-    case 8: go(k_build_H_pairs<8>); break;
-    case 4: go(k_build_H_pairs<4>); break;
+    case 12: return go(k_build_H_pairs<12>);
+    case 8: return go(k_build_H_pairs<8>);
+    case 4: return go(k_build_H_pairs<4>);
     default: return cudaErrorInvalidConfiguration;
   }
-  return cudaGetLastError();
 }
 
 }  // namespace tp3

@@ -341,6 +341,8 @@ __global__ void __launch_bounds__(32 * kLaneMaxWarps, 1) k_couple_lane(
   __shared__ uint64_t s_bar;
   __shared__ int s_next[17];
   __shared__ int s_abort;
+  grid_wait();
+  grid_release();
   const int prop = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int blk = order[blockIdx.z];
@@ -349,7 +351,7 @@ __global__ void __launch_bounds__(32 * kLaneMaxWarps, 1) k_couple_lane(
   bool skip = false;
   int klen = 0;
   if (rag) {
-    const RagInfo ri = rag[prop];
+    const RagInfo ri = after_wait(rag)[prop];
     Kp = ri.K;
     klen = ri.klen;
     skip = fb.l1 > ri.L || fb.l2 > ri.L;
@@ -378,7 +380,7 @@ __global__ void __launch_bounds__(32 * kLaneMaxWarps, 1) k_couple_lane(
     }
     return;
   }
-  const bool sym = symflags[prop] != 0;
+  const bool sym = after_wait(symflags)[prop] != 0;
   const int2 ko = kofs[Kp];
   const int nu = ko.y;
   if ((int)blockIdx.y >= (sym ? nu * fb.nl3 : nu)) return;  // more CTAs than tasks
@@ -507,6 +509,7 @@ __global__ void __cluster_dims__(kGatherCtas, 1, 1) __launch_bounds__(256)
     k_gather_lane(int K, int nc, int ncoef, const int* __restrict__ csean, const int* __restrict__ cm,
                   const int* __restrict__ cmir, const int* __restrict__ cl, const double2* __restrict__ coeff,
                   float2* __restrict__ ct, float* __restrict__ c3p, int* __restrict__ sym, const RagInfo* __restrict__ rag) {
+  grid_release();
   extern __shared__ __align__(16) double2 gl_smem[];
   __shared__ int s_ok[kGatherCtas];
   constexpr int ps = 32 * ROUNDS, c3row = ps / 2;
@@ -610,8 +613,10 @@ __global__ void __cluster_dims__(kGatherCtas, 1, 1) __launch_bounds__(256)
 __global__ void __launch_bounds__(256) k_split_rows(const float* __restrict__ T, int n_lt, int klp, int KP, int ldT32,
                                                     float* __restrict__ hi, float* __restrict__ lo) {
   __shared__ float tile[32][33];
+  grid_wait();
+  grid_release();
   const int ki0 = blockIdx.x * 32, lt0 = blockIdx.y * 32;
-  const float* src = T + (size_t)blockIdx.z * klp * ldT32;
+  const float* src = after_wait(T) + (size_t)blockIdx.z * klp * ldT32;
   for (int r = threadIdx.y; r < 32; r += 8)
     if (lt0 + r < n_lt) tile[r][threadIdx.x] = src[(size_t)(lt0 + r) * klp + ki0 + threadIdx.x];
   __syncthreads();
@@ -855,18 +860,14 @@ cudaError_t launch_couple_lane(const DevTables& t, const TcTables& tc, int n, co
   o.KP = tc.KP; o.klp = t.klp; o.ldT32 = t.n_ltp;
   o.tf32 = tf32; o.ltmaj = t_order_major(tc, tf32); o.t32maj = rows || t32maj;
   auto go = [&](auto kernel) {
-    kernel<<<dim3(n, z, tc.n_pb), 32 * nw, smem, s>>>(
-        ct, reinterpret_cast<const float4*>(c3p), t.K, t.nc, z > 1 ? lt.by_work : lt.by_form, tc.coff, lt.blks, lt.quads, lt.gcols, lt.w, lt.utab, lt.slots,
-        lt.kofs, lt.crows, lt.wmax, lt.c3rows, lt.stage, sym, o, rag, tc.err);
+    return launch_after(kernel, dim3(n, z, tc.n_pb), 32 * nw, smem, s, 1, ct, reinterpret_cast<const float4*>(c3p), t.K,
+                        t.nc, z > 1 ? lt.by_work : lt.by_form, tc.coff, lt.blks, lt.quads, lt.gcols, lt.w, lt.utab,
+                        lt.slots, lt.kofs, lt.crows, lt.wmax, lt.c3rows, lt.stage, sym, o, rag, tc.err);
   };
-  if (lt.ps == 32)
-    go(k_couple_lane<32>);
-  else
-    go(k_couple_lane<64>);
-  if (rows)
-    k_split_rows<<<dim3(t.klp / 32, (t.n_lt + 31) / 32, n), dim3(32, 8), 0, s>>>(scratch, t.n_lt, t.klp, tc.KP, t.n_ltp,
-                                                                                 (float*)Thi, (float*)Tlo);
-  return cudaGetLastError();
+  const cudaError_t e = lt.ps == 32 ? go(k_couple_lane<32>) : go(k_couple_lane<64>);
+  if (e != cudaSuccess || !rows) return e;
+  return launch_after(k_split_rows, dim3(t.klp / 32, (t.n_lt + 31) / 32, n), dim3(32, 8), 0, s, 1, scratch, t.n_lt, t.klp,
+                      tc.KP, t.n_ltp, (float*)Thi, (float*)Tlo);
 }
 
 }  // namespace tp3

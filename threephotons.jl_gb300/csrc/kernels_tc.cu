@@ -807,6 +807,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_angular_tp(
     hd->abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  // No grid_release: CTAs of the energies' sum that came while this kernel holds the SMs would crowd
+  // where there is room, and their FP64 work is bound per SM (256 candidates at L = 12: 50 us more).
+  grid_wait();
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&hd->tmem_base)),
                  "r"(512u)
@@ -825,7 +828,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_angular_tp(
     const int tile = u / nhalf;
     mtile = tile % nmt;
     prop = tile / nmt;
-    return !rag || mtile * kBM < rag[prop].klen;
+    return !rag || mtile * kBM < after_wait(rag)[prop].klen;
   };
 
   if (warp == 0) {
@@ -1101,6 +1104,10 @@ __global__ void __launch_bounds__(128)
   constexpr int NA = 256 / CTAS;                   // accumulators of this CTA
   constexpr int ROWS = kFinRows * 32 / NA < 2 ? 2 : kFinRows * 32 / NA;
   __shared__ double term[ROWS][NA], ss[256], sc[256];
+  grid_wait();
+  part = after_wait(part);
+  rag = after_wait(rag);
+  Qs = after_wait(Qs);
   const int prop = blockIdx.y, rank = blockIdx.x;
   int nk = klength;
   if (rag) {
@@ -1316,40 +1323,28 @@ cudaError_t launch_angular_persistent(const DevTables& t, const TcTables& tc, co
   const int ctas = std::max(1, std::min(nunits, tc.nsm));
   const size_t smem = tc_smem_bytes(c3out != nullptr);
   const bool amn = t_order_major(tc, tf32);
-#define TP3_ANGP(ST, TF, MN, AH, AL)                                                                          \
-  k_angular_tp<ST, TF, MN><<<ctas, kThreads, smem, s>>>(AH, AL, maps.b_hi, maps.b_lo, t.klp, tc.KP, t.Gu, tc.nhalf, \
-                                                        nunits, qt, part, err, rag, t.klength, c3out, t.N, t.mult)
+#define TP3_ANGP(ST, TF, MN, AH, AL)                                                                        \
+  launch_after(k_angular_tp<ST, TF, MN>, ctas, kThreads, smem, s, 1, AH, AL, maps.b_hi, maps.b_lo, t.klp, tc.KP, t.Gu, \
+               tc.nhalf, nunits, qt, part, err, rag, t.klength, c3out, t.N, t.mult)
   if (c3out) {
-    if (tf32) TP3_ANGP(true, true, false, maps.a_hi, maps.a_lo);
-    else if (amn) TP3_ANGP(true, false, true, maps.a_hi_mn, maps.a_lo_mn);
-    else TP3_ANGP(true, false, false, maps.a_hi, maps.a_lo);
-  } else {
-    if (tf32) TP3_ANGP(false, true, false, maps.a_hi, maps.a_lo);
-    else if (amn) TP3_ANGP(false, false, true, maps.a_hi_mn, maps.a_lo_mn);
-    else TP3_ANGP(false, false, false, maps.a_hi, maps.a_lo);
+    if (tf32) return TP3_ANGP(true, true, false, maps.a_hi, maps.a_lo);
+    if (amn) return TP3_ANGP(true, false, true, maps.a_hi_mn, maps.a_lo_mn);
+    return TP3_ANGP(true, false, false, maps.a_hi, maps.a_lo);
   }
+  if (tf32) return TP3_ANGP(false, true, false, maps.a_hi, maps.a_lo);
+  if (amn) return TP3_ANGP(false, false, true, maps.a_hi_mn, maps.a_lo_mn);
+  return TP3_ANGP(false, false, false, maps.a_hi, maps.a_lo);
 #undef TP3_ANGP
-  return cudaGetLastError();
 }
 
 cudaError_t launch_finalize_parts(const DevTables& t, const TcTables& tc, int n, const float* part, const double* Qs,
                                   double* E, cudaStream_t s, const RagInfo* rag) {
   // eight SMs a proposal until the batch has about one proposal per SM
-  if (n >= tc.nsm / 2) {
-    k_finalize_parts<1><<<dim3(1, n), 128, 0, s>>>(part, t.klp, t.klength, tc.nhalf, Qs, t.tf, t.mult, tc.logtab, E, rag);
-    return cudaGetLastError();
-  }
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = 8;
-  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(8, n);
-  cfg.blockDim = dim3(128);
-  cfg.stream = s;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_finalize_parts<8>, part, t.klp, t.klength, tc.nhalf, Qs, t.tf, t.mult, tc.logtab, E, rag);
+  auto go = [&](auto kernel, unsigned ctas) {
+    return launch_after(kernel, dim3(ctas, n), 128, 0, s, ctas, part, t.klp, t.klength, tc.nhalf, Qs, t.tf, t.mult,
+                        tc.logtab, E, rag);
+  };
+  return n >= tc.nsm / 2 ? go(k_finalize_parts<1>, 1) : go(k_finalize_parts<8>, 8);
 }
 
 }  // namespace tp3

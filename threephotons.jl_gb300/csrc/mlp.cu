@@ -99,6 +99,8 @@ __global__ void __launch_bounds__(kGThreads, 1) k_gemm_tn(const __grid_constant_
     hd->abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  grid_wait();
+  grid_release();
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&hd->tmem_base)),
                  "r"(kCols)
@@ -252,6 +254,9 @@ __global__ void __launch_bounds__(kGThreads, 1) k_gemm_tn(const __grid_constant_
 // X [R][ld] -> Xt [C][ldt]; grid (ceil(C/32), ceil(R/32)), block (32, 8).
 __global__ void k_transpose_bf16(const __nv_bfloat16* __restrict__ X, int R, int C, int ld, __nv_bfloat16* __restrict__ Xt,
                                  int ldt) {
+  grid_wait();
+  grid_release();
+  X = after_wait(X);
   __shared__ __nv_bfloat16 t[32][33];
   const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
   for (int i = threadIdx.y; i < 32; i += 8) {
@@ -273,6 +278,9 @@ __global__ void k_transpose_bf16(const __nv_bfloat16* __restrict__ X, int R, int
 __global__ void k_reg_residual(const float* __restrict__ O, const float* __restrict__ V,
                                const float2* __restrict__ tw, int K, int nc, float* __restrict__ resid,
                                double* __restrict__ part) {
+  grid_wait();
+  grid_release();
+  O = after_wait(O);
   __shared__ double red[4];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int j = blockIdx.x * 4 + warp;
@@ -305,6 +313,10 @@ __global__ void k_head_loss(const float* __restrict__ O, int R, const float* __r
                             const float* __restrict__ w, const float* __restrict__ resid, int K, int nc,
                             __nv_bfloat16* __restrict__ dO, __nv_bfloat16* __restrict__ dOt, int ldt,
                             double* __restrict__ part) {
+  grid_wait();
+  grid_release();
+  O = after_wait(O);
+  resid = after_wait(resid);
   __shared__ double red[32];
   const int d = threadIdx.x & 3, lr = threadIdx.x >> 2, r = blockIdx.x * 32 + lr;
   double nll = 0.0;
@@ -348,6 +360,9 @@ __global__ void k_head_loss(const float* __restrict__ O, int R, const float* __r
 // db[n] = sum_r Zt[n][r] (FP32 sum of BF16 values), R and ldt multiples of 8; grid N, block 128.
 // Bound by latency: 16-byte loads (one value at a time took 9.5 us for 512 x 3328).
 __global__ void k_rowsum_bf16(const __nv_bfloat16* __restrict__ Zt, int ldt, int R, float* __restrict__ db) {
+  grid_wait();
+  grid_release();
+  Zt = after_wait(Zt);
   __shared__ float red[4];
   const uint4* z = reinterpret_cast<const uint4*>(Zt + (size_t)blockIdx.x * ldt);
   float s = 0.f;
@@ -462,9 +477,8 @@ cudaError_t gemm(tp3_mlp* net, const CUtensorMap& A, const CUtensorMap& B, GemmA
   if (g.ksplit < 1) g.ksplit = 1;
   grid.z = g.ksplit;
   cudaStream_t s = net->ctx->stream;
-  if (bn == 16) k_gemm_tn<16><<<grid, kGThreads, gemm_smem_bytes<16>(), s>>>(A, B, g);
-  else k_gemm_tn<kGBN><<<grid, kGThreads, gemm_smem_bytes<kGBN>(), s>>>(A, B, g);
-  return cudaGetLastError();
+  return bn == 16 ? launch_after(k_gemm_tn<16>, grid, kGThreads, gemm_smem_bytes<16>(), s, 1, A, B, g)
+                  : launch_after(k_gemm_tn<kGBN>, grid, kGThreads, gemm_smem_bytes<kGBN>(), s, 1, A, B, g);
 }
 
 GemmArgs args(int M, int N, int K) {
@@ -522,20 +536,22 @@ cudaError_t backward(tp3_mlp* n, int R, const float* v, const float* w, const fl
   cudaStream_t s = n->ctx->stream;
   const int H = n->H, MR = n->max_rows;
   dim3 tg((n->n_in_pad + 31) / 32, (R + 31) / 32), tb(32, 8);
-  k_transpose_bf16<<<tg, tb, 0, s>>>(n->X, R, n->n_in_pad, n->n_in_pad, n->Xt, MR);
+  if ((e = cudaMemsetAsync(n->d_grad, 0, n->n_par * sizeof(float), s)) != cudaSuccess ||
+      (e = launch_after(k_transpose_bf16, tg, tb, 0, s, 1, n->X, R, n->n_in_pad, n->n_in_pad, n->Xt, MR)) != cudaSuccess)
+    return e;
   const int nc = R / K;
   if (tw) {
-    k_reg_residual<<<(nc + 3) / 4, 128, 0, s>>>(n->O, v, reinterpret_cast<const float2*>(tw), K, nc, n->d_resid,
-                                               n->d_part + MR / 32);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if ((e = launch_after(k_reg_residual, (nc + 3) / 4, 128, 0, s, 1, n->O, v, reinterpret_cast<const float2*>(tw), K, nc,
+                          n->d_resid, n->d_part + MR / 32)) != cudaSuccess)
+      return e;
   }
-  k_head_loss<<<R / 32, 128, 0, s>>>(n->O, R, v, w, tw ? n->d_resid : nullptr, K, nc, n->dO, n->dOt, MR, n->d_part);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  if ((e = launch_after(k_head_loss, R / 32, 128, 0, s, 1, n->O, R, v, w, tw ? n->d_resid : nullptr, K, nc, n->dO, n->dOt,
+                        MR, n->d_part)) != cudaSuccess)
+    return e;
   float* gW[4];
   float* gb[4];
   for (int l = 0; l < 4; ++l) { gW[l] = n->d_grad + n->off_W[l]; gb[l] = n->d_grad + n->off_b[l]; }
   // weight gradients reduce over the R rows: split K so that about two CTAs per SM work
-  if ((e = cudaMemsetAsync(n->d_grad, 0, n->n_par * sizeof(float), s)) != cudaSuccess) return e;
   auto split = [&](int M, int N) {
     const int tiles = ((M + kGBM - 1) / kGBM) * ((N + pick_bn(N) - 1) / pick_bn(N));
     const int nk = (R + kGBK - 1) / kGBK;
@@ -548,7 +564,7 @@ cudaError_t backward(tp3_mlp* n, int R, const float* v, const float* w, const fl
   GemmArgs g = args(kMlpOut, H, R);
   g.out_f32 = gW[3]; g.ldf = H; g.ksplit = split(kMlpOut, H);
   if ((e = gemm(n, n->bA[0], n->bB[0], g)) != cudaSuccess) return e;
-  k_rowsum_bf16<<<kMlpOut, 128, 0, s>>>(n->dOt, MR, R, gb[3]);
+  if ((e = launch_after(k_rowsum_bf16, kMlpOut, 128, 0, s, 1, n->dOt, MR, R, gb[3])) != cudaSuccess) return e;
   // B2: dZ3 = (dO W4) . [H3 > 0] -> P, Tt
   g = args(R, H, kMlpOutPad);
   g.gate = n->Hh[2]; g.ldg = H; g.out_bf = n->P; g.ldo = H; g.outT_bf = n->Tt; g.ldt = MR;
@@ -557,7 +573,7 @@ cudaError_t backward(tp3_mlp* n, int R, const float* v, const float* w, const fl
   g = args(H, H, R);
   g.out_f32 = gW[2]; g.ldf = H; g.ksplit = split(H, H);
   if ((e = gemm(n, n->bA[2], n->bB[2], g)) != cudaSuccess) return e;
-  k_rowsum_bf16<<<H, 128, 0, s>>>(n->Tt, MR, R, gb[2]);
+  if ((e = launch_after(k_rowsum_bf16, H, 128, 0, s, 1, n->Tt, MR, R, gb[2])) != cudaSuccess) return e;
   // B4: dZ2 = (dZ3 W3) . [H2 > 0] -> Q, Tt
   g = args(R, H, H);
   g.gate = n->Hh[1]; g.ldg = H; g.out_bf = n->Q; g.ldo = H; g.outT_bf = n->Tt; g.ldt = MR;
@@ -566,7 +582,7 @@ cudaError_t backward(tp3_mlp* n, int R, const float* v, const float* w, const fl
   g = args(H, H, R);
   g.out_f32 = gW[1]; g.ldf = H; g.ksplit = split(H, H);
   if ((e = gemm(n, n->bA[4], n->bB[4], g)) != cudaSuccess) return e;
-  k_rowsum_bf16<<<H, 128, 0, s>>>(n->Tt, MR, R, gb[1]);
+  if ((e = launch_after(k_rowsum_bf16, H, 128, 0, s, 1, n->Tt, MR, R, gb[1])) != cudaSuccess) return e;
   // B6: dZ1^T = ((dZ2 W2) . [H1 > 0])^T -> Tt
   g = args(R, H, H);
   g.gate = n->Hh[0]; g.ldg = H; g.outT_bf = n->Tt; g.ldt = MR;
@@ -575,7 +591,7 @@ cudaError_t backward(tp3_mlp* n, int R, const float* v, const float* w, const fl
   g = args(H, n->n_in, R);
   g.out_f32 = gW[0]; g.ldf = n->n_in; g.ksplit = split(H, n->n_in);
   if ((e = gemm(n, n->bA[6], n->bB[6], g)) != cudaSuccess) return e;
-  k_rowsum_bf16<<<H, 128, 0, s>>>(n->Tt, MR, R, gb[0]);
+  if ((e = launch_after(k_rowsum_bf16, H, 128, 0, s, 1, n->Tt, MR, R, gb[0])) != cudaSuccess) return e;
   return cudaGetLastError();
 }
 
