@@ -17,8 +17,9 @@
 //     broadcasts (all lanes read the same four shells).
 // A warp needs no other warp, so warps take tasks from a counter, heaviest first.
 //
-// What bounds it: issue slots.  At L = 18, K = 26 a proposal is 12.2 M warp instructions (the
-// folded rows 15.5 M) at 65 % issue and 47 % of the FMA pipe; 6.1 us of FMA pipe time on 152
+// What bounds it: issue slots and the shared-memory port.  At L = 18, K = 26 a proposal is 11.8 M
+// warp instructions (the folded rows 15.5 M) at 65 % issue, 64 % of the port and 47 % of the FMA
+// pipe; 6.1 us of FMA pipe time on 152
 // SMs (phase 1 4.5, phase 2 1.5) in 14.8 us.  Only coefficients and 3j values are shared, 75 KB
 // a CTA with no D buffer, which lets 16 warps run with no barrier after the staging.
 //
@@ -606,29 +607,36 @@ __global__ void __cluster_dims__(kGatherCtas, 1, 1) __launch_bounds__(256)
   }
 }
 
-// FP32 T [lt][ki] of a proposal -> the TF32 split operand's rows [ki][lt] (hi, lo), 32 x 32
-// tiles through shared memory.  grid: (klp / 32, lt tiles, n); block (32, 8).
+// FP32 T [lt][ki] of a proposal -> the TF32 split operand's rows [ki][lt] (hi, lo), 64 x 32
+// tiles through shared memory; a column past n_lt gets 0, as the padding holds.  grid: (klp / 32, lt tiles, n); block (32, 8).
 // Memory-bound: 6.6 MB read (mostly L2) and 13.6 MB written a proposal at L = 18, K = 26.
 // Writing these rows from the coupling itself costs a sector per value and array.
 __global__ void __launch_bounds__(256) k_split_rows(const float* __restrict__ T, int n_lt, int klp, int KP, int ldT32,
                                                     float* __restrict__ hi, float* __restrict__ lo) {
-  __shared__ float tile[32][33];
+  __shared__ float tile[64][33];
   grid_wait();
   grid_release();
-  const int ki0 = blockIdx.x * 32, lt0 = blockIdx.y * 32;
-  const float* src = after_wait(T) + (size_t)blockIdx.z * klp * ldT32;
-  for (int r = threadIdx.y; r < 32; r += 8)
-    if (lt0 + r < n_lt) tile[r][threadIdx.x] = src[(size_t)(lt0 + r) * klp + ki0 + threadIdx.x];
+  const int ki0 = blockIdx.x * 32, lt0 = blockIdx.y * 64;
+  const float* src = after_wait(T) + (size_t)blockIdx.z * klp * ldT32 + ki0 + threadIdx.x;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const int r = threadIdx.y + 8 * j;
+    tile[r][threadIdx.x] = lt0 + r < n_lt ? src[(size_t)(lt0 + r) * klp] : 0.f;
+  }
   __syncthreads();
-  const int lt = lt0 + threadIdx.x;
+  const int lt = lt0 + 2 * threadIdx.x;
   if (lt >= n_lt) return;
-  for (int r = threadIdx.y; r < 32; r += 8) {
-    const float t = tile[threadIdx.x][r];
-    uint32_t h;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h) : "f"(t));
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int r = threadIdx.y + 8 * j;
+    const float2 t = make_float2(tile[2 * threadIdx.x][r], tile[2 * threadIdx.x + 1][r]);
+    uint32_t h0, h1;
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h0) : "f"(t.x));
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h1) : "f"(t.y));
+    const float2 h = make_float2(__uint_as_float(h0), __uint_as_float(h1));
     const size_t at = ((size_t)blockIdx.z * klp + ki0 + r) * KP + lt;
-    hi[at] = __uint_as_float(h);
-    lo[at] = t - __uint_as_float(h);
+    *reinterpret_cast<float2*>(hi + at) = h;
+    *reinterpret_cast<float2*>(lo + at) = make_float2(t.x - h.x, t.y - h.y);
   }
 }
 
@@ -866,7 +874,7 @@ cudaError_t launch_couple_lane(const DevTables& t, const TcTables& tc, int n, co
   };
   const cudaError_t e = lt.ps == 32 ? go(k_couple_lane<32>) : go(k_couple_lane<64>);
   if (e != cudaSuccess || !rows) return e;
-  return launch_after(k_split_rows, dim3(t.klp / 32, (t.n_lt + 31) / 32, n), dim3(32, 8), 0, s, 1, scratch, t.n_lt, t.klp,
+  return launch_after(k_split_rows, dim3(t.klp / 32, (t.n_lt + 63) / 64, n), dim3(32, 8), 0, s, 1, scratch, t.n_lt, t.klp,
                       tc.KP, t.n_ltp, (float*)Thi, (float*)Tlo);
 }
 
