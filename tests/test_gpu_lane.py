@@ -108,3 +108,50 @@ def test_fourier_pair_operand_equals_entry_sums(L, LMAX, N, K, n):
         for x, y in zip(got[PAIR], got[LANE]):
             assert np.isfinite(x).all() and np.array_equal(x, y)
     b.close()
+
+
+@pytest.mark.parametrize("N", [2, 16, 18, 22, 24, 28, 32])
+def test_grid_halves_and_batch_sizes(N):
+    """Grids of Gu = N^2/2 points on either side of 128, 256 and 384, the widths of the persistent
+    schedule's products; one proposal (tasks spread over small CTAs, a cluster sums the energy)
+    against the same proposals in a batch of 160 (one CTA a sum) bit for bit, and against the
+    per-tile schedule.  Both schedules add the same FP32 c3 and keep the sums compensated, so they
+    differ by the rounding of the stored partials, 2^-24 each, of a slab's Qs log Sp and Sql with
+    Qs = 1 and |log| below 70 (c3 is clamped at 1e-30): K^3 slabs of 2^-23 x 80."""
+    L, LMAX, K, n = 6, 7, 9, 160
+    b = tp3.calculate_basis(L, LMAX, N, K)
+    rng = np.random.default_rng(N)
+    b.set_histogram(rng.uniform(0.5, 1.5, size=(N, 2 * N, K, K, K)))
+    c = _coefficients(L, LMAX, K, n, True, N)
+    for mode in (tp3.TP3_MODE_TC_BF16X3, tp3.TP3_MODE_TC_TF32X3):
+        b.set_mode(mode)
+        b.set_coupling(LANE)
+        E = b.energy_batch(c)
+        assert np.isfinite(E).all()
+        one = np.array([b.energy_batch(c[i:i + 1])[0] for i in (0, 75, n - 1)])
+        assert np.array_equal(one, E[[0, 75, n - 1]])
+        b.set_angular(tp3.TP3_ANGULAR_TILE)
+        assert np.abs(b.energy_batch(c) - E).max() <= 2.0**-23 * 80 * K**3
+        b.set_angular(tp3.TP3_ANGULAR_PERSISTENT)
+    b.close()
+
+
+@pytest.mark.parametrize("broken", [0.0, 1e-12, 1e-7])
+def test_gather_takes_the_pair_forms_branch(broken):
+    """Mirrored orders equal only to a part of the largest coefficient: below 1e-10 of it they
+    count as a real function's, above as general ones, in both forms."""
+    L, LMAX, N, K = 8, 9, 6, 11
+    b = tp3.calculate_basis(L, LMAX, N, K)
+    rng = np.random.default_rng(4)
+    b.set_histogram(rng.uniform(0.5, 1.5, size=(N, 2 * N, K, K, K)))
+    c = _coefficients(L, LMAX, K, 2, True, 9)
+    from tp3.structure import seanindex0
+    c[1, K - 1, seanindex0(4, -3, LMAX)] += broken * np.abs(c).max()
+    got = {}
+    b.set_mode(tp3.TP3_MODE_TC_BF16X3)
+    for form in (PAIR, LANE):
+        b.set_coupling(form)
+        got[form] = (b.triple_products(c[1]), b.energy_batch(c))
+    for x, y in zip(got[PAIR], got[LANE]):
+        assert np.isfinite(x).all() and np.array_equal(x, y)
+    b.close()
