@@ -767,7 +767,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_angular_tc(
   }
 }
 
-// Persistent schedule of the same contraction (Bayes terms only).  A unit is one
+// Persistent schedule of the same contraction (Bayes terms, or c3).  A unit is one
 // (proposal, 128-shell-triple tile, 256-column half of the grid), half fastest; CTA c
 // takes units c, c + gridDim.x, ...  TMEM holds two 256-column accumulators: the i-th
 // unit of a CTA accumulates into buffer i & 1, so the epilogue warps drain one unit
@@ -777,7 +777,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_angular_tc(
 // part [prop][klp][nhalf halves][2 blocks][Sp, Sql]; k_finalize_parts forms the slab
 // terms.  STORE: the epilogue writes c3 instead (all images of every unique point), through a
 // 32 x 16 transpose per warp so that a store instruction covers 64-byte runs of two rows (one row
-// a lane was 32 sectors per instruction: 268 us for 107 MB at L18 K26 N32).
+// a lane was 32 sectors per instruction: 268 us for 107 MB at L18 K26 N32, now 37).
 // Any number of halves (the unfolded 2N^2-point grid of lambda != 0 has 8 at N = 32).
 template <bool STORE, bool TF32, bool AMN>
 __global__ void __launch_bounds__(kThreads, 1) k_angular_tp(
