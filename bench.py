@@ -77,6 +77,10 @@ STAGE_TRAFFIC = {
         "coupling": (155.9e6 / 32, 0.0), "angular": (230.8e6 / 32, 0.0),
         "source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one 32-proposal launch of each stage, "
                   "scaled in proportion to the proposals (profiles/traffic_L18K26N32_b32_folded13w.md)"},
+    ("tc_bf16x3", "lane", "persistent"): {
+        "coupling": (274.6e6 / 32, 0.0), "angular": (229.1e6 / 32, 0.0),
+        "source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one 32-proposal launch of each stage, "
+                  "scaled in proportion to the proposals (profiles/traffic_L18K26N32_b32_lane.md)"},
     ("tc_bf16x3", "folded_7w", "persistent"): {
         "coupling": (154.2e6 / 32, 0.0), "angular": (231.1e6 / 32, 0.0),
         "source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one 32-proposal launch of each stage, "
@@ -408,10 +412,8 @@ def lambda_measure(reps: int = 10, lam: float = 2.5, dq: float = 0.15) -> dict:
     d_coeff = torch.from_numpy(props.view(np.float64)).cuda()
     out = {"workload": f"L{L} K{K} N{N} LMAX{LMAX}, lambda {lam}, dq {dq}, 64 proposals per step", "steps": reps}
     E = {}
-    for name, mode, form in (("tc_bf16x3", tp3.TP3_MODE_TC_BF16X3, 6), ("plain_fp32", tp3.TP3_MODE_PLAIN_FP32, None)):
+    for name, mode in (("tc_bf16x3", tp3.TP3_MODE_TC_BF16X3), ("plain_fp32", tp3.TP3_MODE_PLAIN_FP32)):
         basis.set_mode(mode)
-        if form is not None:
-            basis.set_coupling(form)
         d_E = torch.empty(64, dtype=torch.float64, device="cuda")
         with torch.cuda.stream(stream):
             n = reps if mode != tp3.TP3_MODE_PLAIN_FP32 else max(2, reps // 5)
@@ -544,7 +546,7 @@ def main():
     ap.add_argument("--mode", default="auto", choices=["auto", "tuned", "plain", "tc", "tf32"])
     ap.add_argument("--impl", default="ours", choices=["ours", "reference"])
     ap.add_argument("--workload", default="proposals", choices=["proposals", "ragged", "learned", "chains"])
-    ap.add_argument("--coupling", type=int, default=-1, choices=[-1, 0, 1, 2, 3, 4, 5, 6, 7, 8],
+    ap.add_argument("--coupling", type=int, default=-1, choices=[-1, 0, 1, 2, 3, 4, 5, 6, 7, 8, 9],
                     help="force a tensor-core coupling form (with --mode tc/tf32)")
     ap.add_argument("--angular", default="persistent", choices=["persistent", "tile"],
                     help="angular-stage schedule of the tensor-core path (with --mode tc/tf32)")
