@@ -510,6 +510,7 @@ __global__ void __cluster_dims__(kGatherCtas, 1, 1) __launch_bounds__(256)
     k_gather_lane(int K, int nc, int ncoef, const int* __restrict__ csean, const int* __restrict__ cm,
                   const int* __restrict__ cmir, const int* __restrict__ cl, const double2* __restrict__ coeff,
                   float2* __restrict__ ct, float* __restrict__ c3p, int* __restrict__ sym, const RagInfo* __restrict__ rag) {
+  cluster_started_arrive();
   grid_release();
   extern __shared__ __align__(16) double2 gl_smem[];
   __shared__ int s_ok[kGatherCtas];
@@ -570,13 +571,14 @@ __global__ void __cluster_dims__(kGatherCtas, 1, 1) __launch_bounds__(256)
     }
   }
   ok = __syncthreads_and(ok);
+  cluster_wait();  // ranks past the shells come here at once, before the others may have started
   if (threadIdx.x < kGatherCtas) {  // to every CTA of the cluster
     asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\tst.shared::cluster.u32 [a], %2;\n\t}" ::"r"(
                      smem_u32(&s_ok[rank])),
                  "r"((uint32_t)threadIdx.x), "r"(ok)
                  : "memory");
   }
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  cluster_sync();
   int s = 1;
 #pragma unroll
   for (int i = 0; i < kGatherCtas; ++i) s &= s_ok[i];

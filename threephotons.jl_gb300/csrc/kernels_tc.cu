@@ -1104,6 +1104,7 @@ __global__ void __launch_bounds__(128)
   constexpr int NA = 256 / CTAS;                   // accumulators of this CTA
   constexpr int ROWS = kFinRows * 32 / NA < 2 ? 2 : kFinRows * 32 / NA;
   __shared__ double term[ROWS][NA], ss[256], sc[256];
+  if (CTAS > 1) cluster_started_arrive();
   grid_wait();
   part = after_wait(part);
   rag = after_wait(rag);
@@ -1151,6 +1152,7 @@ __global__ void __launch_bounds__(128)
     }
     __syncthreads();
   } else {
+    cluster_wait();  // CTA 0 runs; a CTA without terms comes here at once
     if (threadIdx.x < NA) {
       const uint32_t as = smem_u32(&ss[a0 + threadIdx.x]), ac = smem_u32(&sc[a0 + threadIdx.x]);
       asm volatile(
@@ -1160,7 +1162,7 @@ __global__ void __launch_bounds__(128)
           "r"(ac), "d"(s[0]), "d"(c[0])
           : "memory");
     }
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    cluster_sync();
     if (rank != 0) return;
   }
   for (int h = 128; h > 0; h >>= 1) {

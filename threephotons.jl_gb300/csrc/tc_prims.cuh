@@ -54,6 +54,21 @@ cudaError_t launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t sme
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
+// Thread-block clusters.  Another CTA's shared memory may be accessed only once that CTA is known
+// to have started: a kernel that stores into it calls cluster_started_arrive as its first statement
+// and cluster_wait before the first such store (the work in between hides the wait), in every
+// thread; cluster_sync then makes the stores of all CTAs visible.
+__device__ __forceinline__ void cluster_started_arrive() {
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  cluster_wait();
+}
+
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }
