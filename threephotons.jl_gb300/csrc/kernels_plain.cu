@@ -80,6 +80,8 @@ __global__ void __launch_bounds__(256) k_couple_direct(
 
 // grid: (ceil(klength/64), ncg, n); block 256 (16 x 16 threads, 4 x 4 per thread).
 // STORE: write c3 rows (out[prop][ki][g]); otherwise accumulate Bayes partials.
+// Kdim: columns of T and F that count, of rows of ldT (a multiple of 16).  What the columns past
+// Kdim hold is not used: T's buffer serves other modes in other layouts.
 template <bool STORE>
 __global__ void __launch_bounds__(256) k_angular_plain(
     const float* __restrict__ T, int ldT, int64_t T_stride, const float* __restrict__ F, int Kdim,
@@ -108,7 +110,11 @@ __global__ void __launch_bounds__(256) k_angular_plain(
       const float4 av = *reinterpret_cast<const float4*>(Tp + (int64_t)(r0 + lrow) * ldT + k0 + lk);
       const int gcol = min(c0 + lrow, G - 1);
       const float4 bv = *reinterpret_cast<const float4*>(F + (int64_t)gcol * ldT + k0 + lk);
-      As[lk + 0][lrow] = av.x; As[lk + 1][lrow] = av.y; As[lk + 2][lrow] = av.z; As[lk + 3][lrow] = av.w;
+      const int kv = Kdim - k0 - lk;
+      As[lk + 0][lrow] = kv > 0 ? av.x : 0.f;
+      As[lk + 1][lrow] = kv > 1 ? av.y : 0.f;
+      As[lk + 2][lrow] = kv > 2 ? av.z : 0.f;
+      As[lk + 3][lrow] = kv > 3 ? av.w : 0.f;
       Bs[lk + 0][lrow] = bv.x; Bs[lk + 1][lrow] = bv.y; Bs[lk + 2][lrow] = bv.z; Bs[lk + 3][lrow] = bv.w;
       __syncthreads();
 #pragma unroll
@@ -243,14 +249,14 @@ cudaError_t launch_angular_plain(const DevTables& t, int n, const float* T, cons
   dim3 grid((t.klength + 63) / 64, ncg, n);
   // lambda = 0: A = T [klp][n_ltp] against F; otherwise A = H [klp][nqp] against the cosine table
   const bool hform = t.nqp > 0;
-  const int kd = hform ? t.nqp : t.n_ltp;
+  const int ld = hform ? t.nqp : t.n_ltp, kd = hform ? t.nq : t.n_lt;
   const float* tab = hform ? t.Cq : t.Ffull;
-  const int64_t Ts = (int64_t)t.klp * kd;
+  const int64_t Ts = (int64_t)t.klp * ld;
   if (c3out)
-    k_angular_plain<true><<<grid, 256, 0, s>>>(T, kd, Ts, tab, kd, t.klength, t.G, cpg, nullptr, nullptr, ncg,
+    k_angular_plain<true><<<grid, 256, 0, s>>>(T, ld, Ts, tab, kd, t.klength, t.G, cpg, nullptr, nullptr, ncg,
                                                c3out);
   else
-    k_angular_plain<false><<<grid, 256, 0, s>>>(T, kd, Ts, tab, kd, t.klength, t.G, cpg, q, part, ncg, nullptr);
+    k_angular_plain<false><<<grid, 256, 0, s>>>(T, ld, Ts, tab, kd, t.klength, t.G, cpg, q, part, ncg, nullptr);
   return cudaGetLastError();
 }
 
