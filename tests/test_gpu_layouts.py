@@ -42,3 +42,30 @@ def test_plain_after_a_nonfinite_tf32_batch(bad):
     for got, ref in zip(_results(b, c), want):
         assert np.array_equal(got, ref)
     b.close()
+
+
+FORMS = [(BF16, 9), (BF16, 0), (BF16, 7), (TF32, 9), (TF32, 0), (PLAIN, 0)]
+
+
+@pytest.mark.parametrize("lam", [0.0, 1.7])
+@pytest.mark.parametrize("bad", [1e30, np.inf, np.nan])
+def test_every_form_after_a_nonfinite_batch_of_another(lam, bad):
+    """A batch whose T overflows (or is NaN) in one (mode, form), then clean proposals in another."""
+    b, c = _world(lam)
+
+    def select(mode, form):
+        b.set_mode(mode)
+        b.set_coupling(form)
+
+    want = {}
+    for f in FORMS:
+        select(*f)
+        want[f] = _results(b, c)
+    for dirty in FORMS:
+        for f in FORMS:
+            select(*dirty)
+            b.energy_batch(c * bad)
+            select(*f)
+            for got, ref in zip(_results(b, c), want[f]):
+                assert np.array_equal(got, ref), (dirty, f)
+    b.close()

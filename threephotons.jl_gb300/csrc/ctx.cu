@@ -131,13 +131,14 @@ std::string build_tc_tables(const Basis& b, const tp3::Wigner3jTable& w3j, std::
   return "";
 }
 
-// 2-D tensor map over a [rows][inner] K-major operand; the box is one 64-byte row of K
-// (32 bf16 or 16 tf32 elements) by box_rows rows, 64-byte swizzle.
-cudaError_t encode_2d(tp3_ctx* c, CUtensorMap* m, void* ptr, uint64_t inner, uint64_t rows, uint32_t box_rows,
-                      bool f32) {
+// 2-D tensor map over a K-major operand of rows of ld elements, the first cols of which count
+// (a copy reads zeros past them); the box is one 64-byte row of K (32 bf16 or 16 tf32 elements)
+// by box_rows rows, 64-byte swizzle.
+cudaError_t encode_2d(tp3_ctx* c, CUtensorMap* m, void* ptr, uint64_t cols, uint64_t ld, uint64_t rows,
+                      uint32_t box_rows, bool f32) {
   const uint64_t esz = f32 ? 4 : 2;
-  cuuint64_t dims[2] = {inner, rows};
-  cuuint64_t strides[1] = {inner * esz};
+  cuuint64_t dims[2] = {cols, rows};
+  cuuint64_t strides[1] = {ld * esz};
   cuuint32_t box[2] = {(cuuint32_t)(64 / esz), box_rows};
   cuuint32_t es[2] = {1, 1};
   CUresult r = c->encode(m, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, ptr, dims,
@@ -146,14 +147,15 @@ cudaError_t encode_2d(tp3_ctx* c, CUtensorMap* m, void* ptr, uint64_t inner, uin
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-// 2-D tensor map over the BF16 T operand in the order-major layout [rows][inner] (inner =
-// shell triples): boxes of 64 shell triples (128 bytes) by 32 orders, 128-byte swizzle.
-cudaError_t encode_2d_mn(tp3_ctx* c, CUtensorMap* m, void* ptr, uint64_t inner, uint64_t rows) {
-  cuuint64_t dims[2] = {inner, rows};
-  cuuint64_t strides[1] = {inner * 2};
-  cuuint32_t box[2] = {64, 32};
-  cuuint32_t es[2] = {1, 1};
-  CUresult r = c->encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, ptr, dims, strides, box, es,
+// 3-D tensor map over the BF16 T operand in the order-major layout, per proposal ld orders of
+// inner shell triples, the first orders of which count (a copy reads zeros past them): boxes of
+// 64 shell triples (128 bytes) by 32 orders, 128-byte swizzle.
+cudaError_t encode_mn(tp3_ctx* c, CUtensorMap* m, void* ptr, uint64_t inner, uint64_t orders, uint64_t ld, uint64_t n) {
+  cuuint64_t dims[3] = {inner, orders, n};
+  cuuint64_t strides[2] = {inner * 2, ld * inner * 2};
+  cuuint32_t box[3] = {64, 32, 1};
+  cuuint32_t es[3] = {1, 1, 1};
+  CUresult r = c->encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, ptr, dims, strides, box, es,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
@@ -339,7 +341,7 @@ std::string setup_tc(tp3_ctx* c) {
   tc.n_units_gen = (int)units_gen.size();
   std::vector<int> cmir(b.nc);
   for (int i = 0; i < b.nc; ++i) cmir[i] = b.coff[b.c_l[i] / 2] + b.c_l[i] - b.c_m[i];
-  const int kcols = tc.hform ? (int)c->qpairs.size() : b.n_lt();  // K extent before padding
+  const int kcols = tc.kcols = tc.hform ? (int)c->qpairs.size() : b.n_lt();
   tc.KP = (std::max(kcols, b.n_lt()) + 31) / 32 * 32;
   tc.nhalf = (b.Gu + 255) / 256;
   tc.NP = 256 * tc.nhalf;
@@ -486,10 +488,10 @@ std::string setup_tc(tp3_ctx* c) {
              tp3::couple_split_smem_t(t, tc) <= (size_t)tp3::kCoupleMaxDynSmem &&
              tp3::couple_split_configure(t, tc) == cudaSuccess;
   cudaGetLastError();
-  if ((e = encode_2d(c, &c->maps.b_hi, (void*)tc.Fhi, tc.KP, tc.NP, 128, false)) != cudaSuccess ||
-      (e = encode_2d(c, &c->maps.b_lo, (void*)tc.Flo, tc.KP, tc.NP, 128, false)) != cudaSuccess ||
-      (e = encode_2d(c, &c->maps32.b_hi, (void*)tc.Fhi32, tc.KP, tc.NP, 128, true)) != cudaSuccess ||
-      (e = encode_2d(c, &c->maps32.b_lo, (void*)tc.Flo32, tc.KP, tc.NP, 128, true)) != cudaSuccess)
+  if ((e = encode_2d(c, &c->maps.b_hi, (void*)tc.Fhi, tc.KP, tc.KP, tc.NP, 128, false)) != cudaSuccess ||
+      (e = encode_2d(c, &c->maps.b_lo, (void*)tc.Flo, tc.KP, tc.KP, tc.NP, 128, false)) != cudaSuccess ||
+      (e = encode_2d(c, &c->maps32.b_hi, (void*)tc.Fhi32, tc.KP, tc.KP, tc.NP, 128, true)) != cudaSuccess ||
+      (e = encode_2d(c, &c->maps32.b_lo, (void*)tc.Flo32, tc.KP, tc.KP, tc.NP, 128, true)) != cudaSuccess)
     return "tensor map encoding of F failed";
   cudaGetLastError();
   if (!tc.fused_ok && !tc.split_ok) return "coupling tile exceeds shared memory";
@@ -552,20 +554,22 @@ int ensure_cap(tp3_ctx* c, int n) {
     cudaGetLastError();
     return fail(c, TP3_ERR_ALLOC, std::string("scratch allocation: ") + cudaGetErrorString(e));
   }
-  // padding rows/columns of the coupling outputs stay zero for the lifetime of the buffers
+  // Modes and coupling forms share T, Thi and Tlo in layouts of their own, so what lies past the
+  // columns (orders) that count is whatever another form left: no kernel takes it in, neither the
+  // tensor maps nor the plain kernel.  Rows past klength are read into results that nobody uses.
   if ((e = cudaMemset(c->d_T, 0, tbytes)) != cudaSuccess) return cuda_fail(c, e, "cudaMemset T");
   if (t.nqp > 0 && (e = cudaMemset(c->d_H, 0, (size_t)n * t.klp * t.nqp * sizeof(float))) != cudaSuccess)
     return cuda_fail(c, e, "cudaMemset H");
   if (c->tc_ok) {
     if ((e = cudaMemset(c->d_Thi, 0, tcb)) != cudaSuccess || (e = cudaMemset(c->d_Tlo, 0, tcb)) != cudaSuccess)
       return cuda_fail(c, e, "cudaMemset T hi/lo");
-    if ((e = encode_2d(c, &c->maps.a_hi, c->d_Thi, c->tc.KP, (uint64_t)n * t.klp, 128, false)) != cudaSuccess ||
-        (e = encode_2d(c, &c->maps.a_lo, c->d_Tlo, c->tc.KP, (uint64_t)n * t.klp, 128, false)) != cudaSuccess ||
-        (e = encode_2d_mn(c, &c->maps.a_hi_mn, c->d_Thi, t.klp, (uint64_t)n * c->tc.KP)) != cudaSuccess ||
-        (e = encode_2d_mn(c, &c->maps.a_lo_mn, c->d_Tlo, t.klp, (uint64_t)n * c->tc.KP)) != cudaSuccess ||
-        (elem == 4 &&
-         ((e = encode_2d(c, &c->maps32.a_hi, c->d_Thi, c->tc.KP, (uint64_t)n * t.klp, 128, true)) != cudaSuccess ||
-          (e = encode_2d(c, &c->maps32.a_lo, c->d_Tlo, c->tc.KP, (uint64_t)n * t.klp, 128, true)) != cudaSuccess)))
+    const uint64_t rows = (uint64_t)n * t.klp, KP = c->tc.KP, cols = c->tc.kcols;
+    if ((e = encode_2d(c, &c->maps.a_hi, c->d_Thi, cols, KP, rows, 128, false)) != cudaSuccess ||
+        (e = encode_2d(c, &c->maps.a_lo, c->d_Tlo, cols, KP, rows, 128, false)) != cudaSuccess ||
+        (e = encode_mn(c, &c->maps.a_hi_mn, c->d_Thi, t.klp, cols, KP, n)) != cudaSuccess ||
+        (e = encode_mn(c, &c->maps.a_lo_mn, c->d_Tlo, t.klp, cols, KP, n)) != cudaSuccess ||
+        (elem == 4 && ((e = encode_2d(c, &c->maps32.a_hi, c->d_Thi, cols, KP, rows, 128, true)) != cudaSuccess ||
+                       (e = encode_2d(c, &c->maps32.a_lo, c->d_Tlo, cols, KP, rows, 128, true)) != cudaSuccess)))
       return fail(c, TP3_ERR_CUDA, "tensor map encoding of T failed");
   }
   c->cap = n;

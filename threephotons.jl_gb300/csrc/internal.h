@@ -240,6 +240,7 @@ struct TcTables {
   const int* cm = nullptr;       // [nc] m of each compact coefficient
   const int* cl = nullptr;       // [nc] l of each compact coefficient
   const int* cmir = nullptr;     // [nc] compact index of (l, -m)
+  int kcols = 0;           // columns of the angular operand that count
   int KP = 0;              // K extent of the angular GEMM: l-triples (lambda = 0) or Fourier
                            // pairs (lambda != 0), padded to 32; also the row stride of T hi / lo
   int NP = 0, nhalf = 0;   // unique grid points padded to 256 * nhalf

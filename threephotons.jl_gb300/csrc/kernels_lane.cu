@@ -610,7 +610,7 @@ __global__ void __cluster_dims__(kGatherCtas, 1, 1) __launch_bounds__(256)
 }
 
 // FP32 T [lt][ki] of a proposal -> the TF32 split operand's rows [ki][lt] (hi, lo), 64 x 32
-// tiles through shared memory; a column past n_lt gets 0, as the padding holds.  grid: (klp / 32, lt tiles, n); block (32, 8).
+// tiles through shared memory; the column beside an odd last one gets 0.  grid: (klp / 32, lt tiles, n); block (32, 8).
 // Memory-bound: 6.6 MB read (mostly L2) and 13.6 MB written a proposal at L = 18, K = 26.
 // Writing these rows from the coupling itself costs a sector per value and array.
 __global__ void __launch_bounds__(256) k_split_rows(const float* __restrict__ T, int n_lt, int klp, int KP, int ldT32,

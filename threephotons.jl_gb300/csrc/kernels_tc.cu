@@ -652,11 +652,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_angular_tc(
           const int nb = Gu - h * kBN > kBNh ? 2 : 1;  // boxes of 128 grid points in this half
           mbar_expect_tx(&hd->full[s], 2 * kABytes + nb * kBBytes);
           if (AMN) {
-            const int y = prop * KP + kc * kbk;  // order row of T[lt][ki]
 #pragma unroll
             for (int g = 0; g < 2; ++g) {
-              tma_load_2d(st + g * (kABytes / 2), &tmA_hi, &hd->full[s], mtile * kBM + g * 64, y);
-              tma_load_2d(st + kABytes + g * (kABytes / 2), &tmA_lo, &hd->full[s], mtile * kBM + g * 64, y);
+              tma_load_3d(st + g * (kABytes / 2), &tmA_hi, &hd->full[s], mtile * kBM + g * 64, kc * kbk, prop);
+              tma_load_3d(st + kABytes + g * (kABytes / 2), &tmA_lo, &hd->full[s], mtile * kBM + g * 64, kc * kbk, prop);
             }
           } else {
             tma_load_2d(st, &tmA_hi, &hd->full[s], kc * kbk, row0);
@@ -851,11 +850,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_angular_tp(
           const int nb = Gu - h * kBN > kBNh ? 2 : 1;  // boxes of 128 grid points in this half
           mbar_expect_tx(&hd->full[s], 2 * kABytes + nb * kBBytes);
           if (AMN) {
-            const int y = prop * KP + kc * kbk;
 #pragma unroll
             for (int g = 0; g < 2; ++g) {
-              tma_load_2d(st + g * (kABytes / 2), &tmA_hi, &hd->full[s], mtile * kBM + g * 64, y);
-              tma_load_2d(st + kABytes + g * (kABytes / 2), &tmA_lo, &hd->full[s], mtile * kBM + g * 64, y);
+              tma_load_3d(st + g * (kABytes / 2), &tmA_hi, &hd->full[s], mtile * kBM + g * 64, kc * kbk, prop);
+              tma_load_3d(st + kABytes + g * (kABytes / 2), &tmA_lo, &hd->full[s], mtile * kBM + g * 64, kc * kbk, prop);
             }
           } else {
             tma_load_2d(st, &tmA_hi, &hd->full[s], kc * kbk, row0);
