@@ -1460,7 +1460,7 @@ int tp3_triple_products(tp3_ctx* c, const double* coeff, float* out) {
                              t.klength, cudaMemcpyDeviceToHost, c->stream)) != cudaSuccess ||
       (e = cudaStreamSynchronize(c->stream)) != cudaSuccess)
     return cuda_fail(c, e, "D2H T");
-  return TP3_OK;
+  return check_device_error(c);  // the lane-owned coupling waits for its copies, with a limit
 }
 
 int tp3_energy_batch(tp3_ctx* c, int n, const double* coeffs, double* E) {
