@@ -486,7 +486,7 @@ std::string setup_tc(tp3_ctx* c) {
   // the split coupling is kept for the autotuner and for shapes the fused kernel cannot hold
   tc.split_ok = tp3::couple_split_smem_d(t, tc) <= (size_t)tp3::kCoupleMaxDynSmem &&
              tp3::couple_split_smem_t(t, tc) <= (size_t)tp3::kCoupleMaxDynSmem &&
-             tp3::couple_split_configure(t, tc) == cudaSuccess;
+             tp3::couple_split_configure() == cudaSuccess;
   cudaGetLastError();
   if ((e = encode_2d(c, &c->maps.b_hi, (void*)tc.Fhi, tc.KP, tc.KP, tc.NP, 128, false)) != cudaSuccess ||
       (e = encode_2d(c, &c->maps.b_lo, (void*)tc.Flo, tc.KP, tc.KP, tc.NP, 128, false)) != cudaSuccess ||

@@ -301,7 +301,7 @@ cudaError_t launch_build_H_pairs(const DevTables& t, const TcTables& tc, int n, 
                                  bool tf32, cudaStream_t s);
 size_t couple_split_smem_d(const DevTables& t, const TcTables& tc);
 size_t couple_split_smem_t(const DevTables& t, const TcTables& tc);
-cudaError_t couple_split_configure(const DevTables& t, const TcTables& tc);
+cudaError_t couple_split_configure();
 std::string build_fold_tables(const std::vector<PairBlock>& pbs, const Wigner3jTable& w3j, int drows, std::vector<FoldBlock>& blks,
                               std::vector<FoldRow>& rows, std::vector<float>& w, std::vector<int2>& chunks,
                               int& wmax, int& cmax);

@@ -223,15 +223,17 @@ size_t couple_split_smem_t(const DevTables& t, const TcTables& tc) {
   return (size_t)t.K * (tc.ncp + tc.SDmax) * sizeof(float2);
 }
 
-cudaError_t couple_split_configure(const DevTables& t, const TcTables& tc) {
+// The attribute belongs to the process and not to a context, so it is the limit itself: a context
+// of a smaller shape, made later, must not lower it for the larger ones.
+cudaError_t couple_split_configure() {
   cudaError_t e;
-  const int sd = (int)couple_split_smem_d(t, tc), st = (int)couple_split_smem_t(t, tc);
-  if ((e = cudaFuncSetAttribute(k_couple_d<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, sd)) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(k_couple_d<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, sd)) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(k_couple_d<10>, cudaFuncAttributeMaxDynamicSharedMemorySize, sd)) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(k_couple_d<12>, cudaFuncAttributeMaxDynamicSharedMemorySize, sd)) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(k_couple_d<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, sd)) != cudaSuccess ||
-      (e = cudaFuncSetAttribute(k_couple_t, cudaFuncAttributeMaxDynamicSharedMemorySize, st)) != cudaSuccess)
+  const cudaFuncAttribute ds = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  if ((e = cudaFuncSetAttribute(k_couple_d<4>, ds, kCoupleMaxDynSmem)) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(k_couple_d<8>, ds, kCoupleMaxDynSmem)) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(k_couple_d<10>, ds, kCoupleMaxDynSmem)) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(k_couple_d<12>, ds, kCoupleMaxDynSmem)) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(k_couple_d<16>, ds, kCoupleMaxDynSmem)) != cudaSuccess ||
+      (e = cudaFuncSetAttribute(k_couple_t, ds, kCoupleMaxDynSmem)) != cudaSuccess)
     return e;
   return cudaSuccess;
 }
