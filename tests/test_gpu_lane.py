@@ -155,3 +155,57 @@ def test_gather_takes_the_pair_forms_branch(broken):
     for x, y in zip(got[PAIR], got[LANE]):
         assert np.isfinite(x).all() and np.array_equal(x, y)
     b.close()
+
+
+@pytest.mark.parametrize("L,N,K,n", [(12, 16, 16, 1), (12, 16, 16, 4), (18, 32, 26, 4)])
+@pytest.mark.parametrize("mode", [tp3.TP3_MODE_TC_BF16X3, tp3.TP3_MODE_TC_TF32X3])
+def test_general_coefficients_are_no_slower_than_in_the_pair_form(L, N, K, n, mode):
+    """The default form takes general coefficients in runs of orders; a pass per order was slower than
+    the one-kernel form, which has both signs of m3 in one pass."""
+    import torch
+    b = tp3.calculate_basis(L, L + 1, N, K)
+    rng = np.random.default_rng(1)
+    b.set_histogram(rng.uniform(0.5, 1.5, size=(N, 2 * N, K, K, K)))
+    d_c = torch.from_numpy(_coefficients(L, L + 1, K, n, False, 4).view(np.float64).copy()).cuda()
+    d_E = torch.empty(n, dtype=torch.float64, device="cuda")
+    b.set_mode(mode)
+    stream = torch.cuda.Stream()
+    b.set_stream(stream.cuda_stream)
+    best, E = {PAIR: 1e9, LANE: 1e9}, {}
+    for rep in range(8):  # in turn
+        for form in (PAIR, LANE):
+            b.set_coupling(form)
+            b.energy_batch_device(n, d_c.data_ptr(), d_E.data_ptr())
+            e0, e1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            e0.record(stream)
+            for _ in range(50):
+                b.energy_batch_device(n, d_c.data_ptr(), d_E.data_ptr())
+            e1.record(stream)
+            b.sync()
+            best[form] = min(best[form], e0.elapsed_time(e1))
+            E[form] = d_E.cpu().numpy()
+    assert np.array_equal(E[PAIR], E[LANE])
+    assert best[LANE] <= best[PAIR], best
+    b.set_stream(None)
+    b.close()
+
+
+@pytest.mark.parametrize("L,K", [(6, 12), (16, 17), (18, 26), (22, 9)])
+@pytest.mark.parametrize("n", [1, 2, 40])
+def test_runs_of_orders_equal_the_pair_form(L, K, n):
+    """General coefficients, alone and beside real functions: balanced runs of one to three orders, some
+    blocks in more runs than that (small L), passes spread over a block's CTAs (small n) or taken in
+    turn by one (n = 40)."""
+    LMAX, N = L + 1, 6
+    b = tp3.calculate_basis(L, LMAX, N, K)
+    rng = np.random.default_rng(n)
+    b.set_histogram(rng.uniform(0.5, 1.5, size=(N, 2 * N, K, K, K)))
+    c = _coefficients(L, LMAX, K, n, False, L)
+    c[1::3] = _coefficients(L, LMAX, K, len(c[1::3]), True, K)
+    got = {}
+    for form in (PAIR, LANE):
+        b.set_coupling(form)
+        got[form] = (b.triple_products(c[0]), b.energy_batch(c))
+    for x, y in zip(got[PAIR], got[LANE]):
+        assert np.isfinite(x).all() and np.array_equal(x, y)
+    b.close()

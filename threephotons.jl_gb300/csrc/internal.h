@@ -158,6 +158,7 @@ struct LaneBlock {
   int c1, c2;  // first coefficient rows of l1 and l2
   int q0, nq;  // quads of the real-function path (m3 >= 0, all orders)
   int w0, wn;  // its 3j values (float4)
+  int gp;      // passes of the general path, balanced runs of orders
 };
 struct LaneTables {
   bool ok = false;
@@ -170,7 +171,7 @@ struct LaneTables {
   const int* by_work = nullptr;     // [n_pb] 0, 1, ..
   const int* by_form = nullptr;     // [n_pb] blocks of one loop form (c_k2 stepped, c_k1 stepped) together
   const LaneQuad* quads = nullptr;
-  const int4* gcols = nullptr;  // [n_pb][16] general path, per order: first quad, quads, first 3j float4, count
+  const int4* gcols = nullptr;  // [n_pb][16] general path, per pass: first quad, quads, first 3j float4, count
   const float4* w = nullptr;
   const uint32_t* utab = nullptr;   // units (build_lane_units)
   const uint32_t* slots = nullptr;

@@ -175,9 +175,9 @@ struct LaneOut {
 };
 
 // One task: orders s_lo .. s_lo + w - 1 of the block for the 32 shell pairs of a unit; CR bytes
-// per c_k3 row, slots / nslot: the unit's staging slots (build_lane_units).
-template <int NC, int PS, int CR>
-__device__ __forceinline__ void lane_task(const LaneView& V, bool swap, bool sym, int l3min, int s_lo, int w, int lt_base,
+// per c_k3 row, slots / nslot: the unit's staging slots (build_lane_units).  SYM: real functions.
+template <bool SYM, int NC, int PS, int CR>
+__device__ __forceinline__ void lane_task(const LaneView& V, bool swap, int l3min, int s_lo, int w, int lt_base,
                                           bool wide, int k1, int k2, int len, int off, int nslot, float* stage,
                                           const uint32_t* __restrict__ slots, const LaneOut& o) {
   const int lane = threadIdx.x & 31;
@@ -187,19 +187,19 @@ __device__ __forceinline__ void lane_task(const LaneView& V, bool swap, bool sym
 #pragma unroll
     for (int j = 0; j < 8; ++j) acc[c][j] = make_float2(0.f, 0.f);
   float2 R0[NC], I0[NC], R1[NC], I1[NC];
-  // column c is order s_lo + c - (NC - w); it takes the m3 with (unsigned)(m3 - m_lo) < cnt[c]
+  // column c is order s_lo + c - (NC - w); it takes the m3 with (unsigned)(|m3| - m_lo) < cnt[c]
   // (none for the NC - w columns before the task's orders).  row[c]: address of its c_k3 row of
-  // the quad's first m3: after the rows of the orders below (real functions, m3 = 0 .. l3), or
-  // of the only order staged (general coefficients, m3 = -l3 .. l3)
+  // the quad's first m3, after the rows of the orders staged before it: from order 0 with m3 =
+  // 0 .. l3 (real functions), or from s_lo with m3 = -l3 .. l3 (general coefficients)
   const int s_hi = s_lo + w, s_off = s_lo - (NC - w);
-  int m_lo = sym ? 1 : -(l3min + 2 * s_lo);  // the m3 = 0 term of real functions is added last
+  int m_lo = SYM ? 1 : 0;  // the m3 = 0 term of real functions is added last
   uint32_t row[NC];
   int cnt[NC];
 #pragma unroll
   for (int c = 0; c < NC; ++c) {
-    const int s = s_off + c, l3 = l3min + 2 * s;
+    const int s = s_off + c, l3 = l3min + 2 * s, j = s - s_lo;
     cnt[c] = s < s_lo ? 0 : l3 - m_lo + 1;
-    row[c] = V.C3 + CR * (sym ? s * (l3min + s) : V.quads[0].m3 + l3);
+    row[c] = V.C3 + CR * (SYM ? s * (l3min + s) : j * (2 * l3 - 2 * j - 1) + V.quads[0].m3 + l3);
   }
   const uint32_t xk = V.X + 8 * (swap ? k2 : k1), vk = V.V + 8 * (swap ? k1 : k2);
   float2* D0 = reinterpret_cast<float2*>(stage);  // real functions: D of m3 = 0, [NC][32]
@@ -216,12 +216,12 @@ __device__ __forceinline__ void lane_task(const LaneView& V, bool swap, bool sym
         lane_p1<NC, PS, true>(x, v, q.n, wt, 16 * q.rs, R0, I0, R1, I1);
       else
         lane_p1<NC, PS, false>(x, v, q.n, wt, 16 * q.rs, R0, I0, R1, I1);
-      if (sym && m == 0) {
+      if (SYM && m == 0) {
 #pragma unroll
         for (int c = 0; c < NC; ++c) D0[c * 32 + lane] = make_float2(R0[c].x, I0[c].x);
       }
     } else {
-      if (!sym) break;
+      if (!SYM) break;
       // T = 2 sum_{m3 > 0} Re(D c) + Re(D[0] c[0])
       m_lo = 0;
 #pragma unroll
@@ -242,11 +242,12 @@ __device__ __forceinline__ void lane_task(const LaneView& V, bool swap, bool sym
     // phase 2, two m3 at a time
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const int t = m + 2 * h - m_lo;
+      const int ma = m + 2 * h, mb = ma + 1;
+      const int t0 = (SYM ? ma : abs(ma)) - m_lo, t1 = (SYM ? mb : abs(mb)) - m_lo;
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
-        if ((unsigned)t < (unsigned)cnt[c]) lane_p2(row[c], h ? R1[c].x : R0[c].x, h ? I1[c].x : I0[c].x, wide, acc[c]);
-        if ((unsigned)(t + 1) < (unsigned)cnt[c])
+        if ((unsigned)t0 < (unsigned)cnt[c]) lane_p2(row[c], h ? R1[c].x : R0[c].x, h ? I1[c].x : I0[c].x, wide, acc[c]);
+        if ((unsigned)t1 < (unsigned)cnt[c])
           lane_p2(row[c] + CR, h ? R1[c].y : R0[c].y, h ? I1[c].y : I0[c].y, wide, acc[c]);
         row[c] += 2 * CR;
       }
@@ -325,9 +326,21 @@ __device__ __forceinline__ void lane_task(const LaneView& V, bool swap, bool sym
   }
 }
 
+// Run i of n balanced runs of nl3 orders: first order and orders.
+__host__ __device__ __forceinline__ void lane_run(int nl3, int n, int i, int& s_lo, int& w) {
+  const int lo = nl3 / n, ex = nl3 - lo * n;
+  s_lo = i * lo + (i < ex ? i : ex);
+  w = lo + (i < ex ? 1 : 0);
+}
+
 // grid: (n, Z, n_pb); block 32 x warps; dynamic shared memory lane_smem_bytes.
 // CTA (p, z, b) takes the tasks z, z + Z, .. of block order[b] of proposal p: Z > 1 spreads the
-// tasks of a small batch over the SMs.  Proposals run fastest, so an SM's CTAs are mostly on
+// tasks of a small batch over the SMs.  A real function's c_k3 rows and 3j values (m3 >= 0) are
+// staged for all orders; general coefficients (both signs of m3, twice the rows and values) go in
+// passes of up to kLaneNC orders, one run of orders for all units, and Z > 1 spreads the passes first.
+// A pass per order computes kLaneNC columns for one: 64 general proposals at L = 18, K = 26 took
+// 3.39 ms (the whole scoring) so and 1.85 in runs; four in TF32 mode at L = 12, K = 16 107 and 66 us,
+// where the one-kernel coupling takes 95.  Proposals run fastest, so an SM's CTAs are mostly on
 // one block and their warps in the same code.
 template <int PS>
 __global__ void __launch_bounds__(32 * kLaneMaxWarps, 1) k_couple_lane(
@@ -384,7 +397,10 @@ __global__ void __launch_bounds__(32 * kLaneMaxWarps, 1) k_couple_lane(
   const bool sym = after_wait(symflags)[prop] != 0;
   const int2 ko = kofs[Kp];
   const int nu = ko.y;
-  if ((int)blockIdx.y >= (sym ? nu * fb.nl3 : nu)) return;  // more CTAs than tasks
+  // tasks t = next * tstep + toff; general coefficients: passes pass0, pass0 + pstep, ..
+  const int pstep = sym ? 1 : min((int)gridDim.y, fb.gp), pass0 = sym ? 0 : blockIdx.y % pstep;
+  const int tstep = (gridDim.y - pass0 + pstep - 1) / pstep, toff = blockIdx.y / pstep;
+  if (toff >= (sym ? nu * fb.nl3 : nu)) return;  // more CTAs than tasks
   float2* C1 = reinterpret_cast<float2*>(lane_smem);
   float2* C2 = C1 + (size_t)crows * ps;
   float4* W = reinterpret_cast<float4*>(C2 + (size_t)crows * ps) + 8;  // a rounded-up run may start before its row
@@ -393,7 +409,6 @@ __global__ void __launch_bounds__(32 * kLaneMaxWarps, 1) k_couple_lane(
   const float2* ctp = ct + (size_t)prop * nc * ps;
   const float4* c3g = c3p + (size_t)prop * nc * c3row;
   const int n1r = 2 * fb.l1 + 1, n2r = 2 * fb.l2 + 1;
-  const int passes = sym ? 1 : fb.nl3;  // general coefficients: one order at a time
   // three zero rows at either end of C1 and C2: the union m range of a quad reaches up to
   // three rows past an end, where its 3j value is zero
   for (int i = threadIdx.x; i < 6 * ps; i += blockDim.x) {
@@ -414,66 +429,75 @@ __global__ void __launch_bounds__(32 * kLaneMaxWarps, 1) k_couple_lane(
   V.W = smem_u32(W);
   V.C3 = smem_u32(C3);
   V.quads = s_quads;
-  for (int pass = 0; pass < passes; ++pass) {
-    int4 g = make_int4(fb.q0, fb.nq, fb.w0, fb.wn);
-    if (!sym) g = gcols[blk * 16 + pass];
-    if (pass > 0) {
-      __syncthreads();  // the previous order's reads are done
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    }
-    if (threadIdx.x == 0) {
-      uint32_t bytes = (uint32_t)g.w * 16u;
-      if (pass == 0) bytes += (uint32_t)(n1r + n2r) * ps * 8u;
-      int r = 0;
-      for (int s = sym ? 0 : pass; s < (sym ? fb.nl3 : pass + 1); ++s) {
-        const int l3 = fb.l3min + 2 * s;
-        r += sym ? l3 + 1 : 2 * l3 + 1;
+  // real functions and general coefficients each in code of its own, both without spills: 64 real
+  // proposals at L = 18, K = 26 score in 1.176 ms so and in 1.254 with one task for both
+  auto passes = [&](auto real) {
+    constexpr bool SYM = decltype(real)::value;
+    uint32_t phase = 0;
+    for (int pass = pass0; pass < (SYM ? 1 : fb.gp); pass += pstep, phase ^= 1u) {
+      int4 g = make_int4(fb.q0, fb.nq, fb.w0, fb.wn);
+      int p_lo = 0, p_w = fb.nl3;  // the orders staged
+      if (!SYM) {
+        g = gcols[blk * 16 + pass];
+        lane_run(fb.nl3, fb.gp, pass, p_lo, p_w);
       }
-      bytes += (uint32_t)r * c3row * 16u;
-      mbar_expect_tx(&s_bar, bytes);
-      if (pass == 0) {
-        bulk_load(C1 + 3 * ps, ctp + (size_t)fb.c1 * ps, (uint32_t)n1r * ps * 8u, &s_bar);
-        bulk_load(C2 + 3 * ps, ctp + (size_t)fb.c2 * ps, (uint32_t)n2r * ps * 8u, &s_bar);
+      if (pass > pass0) {
+        __syncthreads();  // the previous orders' reads are done
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       }
-      bulk_load(W, wtab + g.z, (uint32_t)g.w * 16u, &s_bar);
-      r = 0;
-      for (int s = sym ? 0 : pass; s < (sym ? fb.nl3 : pass + 1); ++s) {
-        const int l3 = fb.l3min + 2 * s, cnt = sym ? l3 + 1 : 2 * l3 + 1;
-        const int c0 = coff[l3 >> 1] + (sym ? l3 : 0);
-        bulk_load(C3 + (size_t)r * c3row, c3g + (size_t)c0 * c3row, (uint32_t)cnt * c3row * 16u, &s_bar);
-        r += cnt;
+      if (threadIdx.x == 0) {
+        uint32_t bytes = (uint32_t)g.w * 16u;
+        if (pass == pass0) bytes += (uint32_t)(n1r + n2r) * ps * 8u;
+        int r = 0;
+        for (int s = p_lo; s < p_lo + p_w; ++s) {
+          const int l3 = fb.l3min + 2 * s;
+          r += SYM ? l3 + 1 : 2 * l3 + 1;
+        }
+        bytes += (uint32_t)r * c3row * 16u;
+        mbar_expect_tx(&s_bar, bytes);
+        if (pass == pass0) {
+          bulk_load(C1 + 3 * ps, ctp + (size_t)fb.c1 * ps, (uint32_t)n1r * ps * 8u, &s_bar);
+          bulk_load(C2 + 3 * ps, ctp + (size_t)fb.c2 * ps, (uint32_t)n2r * ps * 8u, &s_bar);
+        }
+        bulk_load(W, wtab + g.z, (uint32_t)g.w * 16u, &s_bar);
+        r = 0;
+        for (int s = p_lo; s < p_lo + p_w; ++s) {
+          const int l3 = fb.l3min + 2 * s, cnt = SYM ? l3 + 1 : 2 * l3 + 1;
+          const int c0 = coff[l3 >> 1] + (SYM ? l3 : 0);
+          bulk_load(C3 + (size_t)r * c3row, c3g + (size_t)c0 * c3row, (uint32_t)cnt * c3row * 16u, &s_bar);
+          r += cnt;
+        }
+      }
+      for (int i = threadIdx.x; i < g.y; i += blockDim.x) s_quads[i] = quads[g.x + i];
+      __syncthreads();
+      V.nq = g.y;
+      if (!mbar_wait(&s_bar, phase, &s_abort, err)) {
+        mbar_wait_limit(&s_bar, phase, kTimeoutCycles, err);  // copies still in flight land before the exit
+        return;
+      }
+      const int nrun = SYM ? (fb.nl3 + kLaneNC - 1) / kLaneNC : 1;
+      for (;;) {
+        int t = 0;
+        if (lane == 0) t = atomicAdd(&s_next[pass], 1);
+        t = __shfl_sync(0xffffffffu, t, 0) * tstep + toff;
+        const int u = t / nrun;
+        if (u >= nu) break;
+        int s_lo = p_lo, w = p_w;
+        if (SYM) lane_run(fb.nl3, nrun, t - u * nrun, s_lo, w);
+        const uint32_t e = utab[ko.x + u * 34 + lane];  // the lane's shell pair, see build_lane_units
+        const uint32_t s0 = utab[ko.x + u * 34 + 32], s1 = utab[ko.x + u * 34 + 33];
+        V.C3 = smem_u32(C3 + 8 * (s1 >> 17));
+        lane_task<SYM, kLaneNC, PS, 8 * PS>(V, fb.swap, fb.l3min, s_lo, w, fb.lt_base, (s1 >> 16) & 1, (int)e & 63,
+                                            (int)(e >> 6) & 63, (int)(e >> 24), (int)(e >> 12) & 0xfff, (int)(s1 & 0xffff),
+                                            stage, slots + s0, out);
+        __syncwarp();
       }
     }
-    for (int i = threadIdx.x; i < g.y; i += blockDim.x) s_quads[i] = quads[g.x + i];
-    __syncthreads();
-    V.nq = g.y;
-    if (!mbar_wait(&s_bar, pass & 1, &s_abort, err)) {
-      mbar_wait_limit(&s_bar, pass & 1, kTimeoutCycles, err);  // copies still in flight land before the exit
-      return;
-    }
-    const int nrun = sym ? (fb.nl3 + kLaneNC - 1) / kLaneNC : 1;
-    for (;;) {
-      int t = 0;
-      if (lane == 0) t = atomicAdd(&s_next[pass], 1);
-      t = __shfl_sync(0xffffffffu, t, 0) * gridDim.y + blockIdx.y;
-      const int u = t / nrun;
-      if (u >= nu) break;
-      int s_lo = pass, w = 1;
-      if (sym) {  // balanced runs of orders
-        const int lo = fb.nl3 / nrun, ex = fb.nl3 - lo * nrun;
-        t -= u * nrun;
-        s_lo = t * lo + min(t, ex);
-        w = lo + (t < ex ? 1 : 0);
-      }
-      const uint32_t e = utab[ko.x + u * 34 + lane];  // the lane's shell pair, see build_lane_units
-      const uint32_t s0 = utab[ko.x + u * 34 + 32], s1 = utab[ko.x + u * 34 + 33];
-      V.C3 = smem_u32(C3 + 8 * (s1 >> 17));
-      lane_task<kLaneNC, PS, 8 * PS>(V, fb.swap, sym, fb.l3min, s_lo, w, fb.lt_base, (s1 >> 16) & 1, (int)e & 63,
-                                     (int)(e >> 6) & 63, (int)(e >> 24), (int)(e >> 12) & 0xfff, (int)(s1 & 0xffff), stage,
-                                     slots + s0, out);
-      __syncwarp();
-    }
-  }
+  };
+  if (sym)
+    passes(std::true_type());
+  else
+    passes(std::false_type());
 }
 
 // (float)x by integer arithmetic: FP64 conversions, like all FP64 arithmetic, run at a few
@@ -653,91 +677,114 @@ std::string build_lane_tables(const std::vector<PairBlock>& pbs, const std::vect
                               std::vector<float4>& w, int& crows, int& wmax, int& c3rows) {
   blks.clear(); quads.clear(); gcols.clear(); w.clear();
   crows = wmax = c3rows = 0;
-  for (const PairBlock& pb : pbs) {
-    const int l1 = pb.l1, l2 = pb.l2;
-    LaneBlock fb{};
-    fb.l1 = l1; fb.l2 = l2; fb.l3min = pb.l3min; fb.nl3 = pb.nl3; fb.lt_base = pb.lt_base;
-    fb.c1 = coff[l1 >> 1]; fb.c2 = coff[l2 >> 1];
-    // steps run over the m of the shorter row, the other row slides with m3
-    fb.swap = l1 > l2;
-    const int a = std::min(l1, l2), b = std::max(l1, l2);
-    // one quad (m3 .. m3 + 3), orders s0 .. nl3 - 1 (or only s0): rows and 3j values
-    auto add = [&](int m3, int s0, int s1) {
-      LaneQuad q{};
-      q.m3 = m3;
-      q.c0 = s0;
-      q.rs = s1 - s0;
-      int lo = std::max(-a, -b - m3 - 3), hi = std::min(a, b - m3);
-      if ((hi - lo) & 1) ++hi;  // an odd number of steps (the form of the loop); the extra one is zero
-      q.n = hi - lo + 1;
-      // without swap: m1 = lo .. hi, window row k holds c_k2[-(m3 + k) - m1]; with swap: m2 =
-      // hi .. lo, window row k holds c_k1[-(m3 + 3 - k) - m2].  Arrays start at row 3.
-      q.x0 = (fb.swap ? hi + l2 : lo + l1) + 3;
-      q.vb = (fb.swap ? -(m3 + 3) - hi + l1 : -m3 - lo + l2) + 3;
-      q.wofs = 0;
-      for (int i = 0; i < q.n; ++i)
-        for (int s = s0; s < s1; ++s) {
-          const int l3 = pb.l3min + 2 * s;
-          float v[4];
-          for (int k = 0; k < 4; ++k) {
-            const int mm3 = m3 + k;
-            const int m1 = fb.swap ? -mm3 - (hi - i) : lo + i, m2 = -mm3 - m1;
-            const bool in = std::abs(mm3) <= l3 && std::abs(m1) <= l1 && std::abs(m2) <= l2;
-            v[k] = in ? (float)w3j(l1, l2, l3, m1, m2, mm3) : 0.f;
-          }
-          w.push_back(make_float4(v[0], v[1], v[2], v[3]));
+  std::string bad;
+  // one quad (m3 .. m3 + 3) of orders s0 .. s1 - 1: its rows and, when put, 3j values; steps run
+  // over the m of the shorter row, the other row slides with m3
+  auto quad_of = [&](const PairBlock& pb, int m3, int s0, int s1, bool put) {
+    const int l1 = pb.l1, l2 = pb.l2, a = std::min(l1, l2), b = std::max(l1, l2);
+    const bool swap = l1 > l2;
+    LaneQuad q{};
+    q.m3 = m3;
+    q.c0 = s0;
+    q.rs = s1 - s0;
+    int lo = std::max(-a, -b - m3 - 3), hi = std::min(a, b - m3);
+    if ((hi - lo) & 1) ++hi;  // an odd number of steps (the form of the loop); the extra one is zero
+    q.n = hi - lo + 1;
+    // without swap: m1 = lo .. hi, window row k holds c_k2[-(m3 + k) - m1]; with swap: m2 =
+    // hi .. lo, window row k holds c_k1[-(m3 + 3 - k) - m2].  Arrays start at row 3.
+    q.x0 = (swap ? hi + l2 : lo + l1) + 3;
+    q.vb = (swap ? -(m3 + 3) - hi + l1 : -m3 - lo + l2) + 3;
+    const int xl = swap ? 2 * l2 + 7 : 2 * l1 + 7, vl = swap ? 2 * l1 + 7 : 2 * l2 + 7;
+    const int sx = swap ? -1 : 1, sv = -sx;
+    const int x1 = q.x0 + sx * (q.n - 1), v1 = q.vb + sv * (q.n + 2);
+    if (q.n < 1 || std::min(q.x0, x1) < 0 || std::max(q.x0, x1) >= xl || std::min(q.vb, v1) < 0 || std::max(q.vb, v1) >= vl)
+      bad = "lane tables: a quad leaves the staged rows";
+    for (int i = 0; put && i < q.n; ++i)
+      for (int s = s0; s < s1; ++s) {
+        const int l3 = pb.l3min + 2 * s;
+        float v[4];
+        for (int k = 0; k < 4; ++k) {
+          const int mm3 = m3 + k;
+          const int m1 = swap ? -mm3 - (hi - i) : lo + i, m2 = -mm3 - m1;
+          const bool in = std::abs(mm3) <= l3 && std::abs(m1) <= l1 && std::abs(m2) <= l2;
+          v[k] = in ? (float)w3j(l1, l2, l3, m1, m2, mm3) : 0.f;
         }
-      quads.push_back(q);
-      return q.n * q.rs;
-    };
-    auto fits = [&](const LaneQuad& q) {
-      const int xl = fb.swap ? 2 * l2 + 7 : 2 * l1 + 7, vl = fb.swap ? 2 * l1 + 7 : 2 * l2 + 7;
-      const int sx = fb.swap ? -1 : 1, sv = -sx;
-      const int x1 = q.x0 + sx * (q.n - 1), v1 = q.vb + sv * (q.n + 2);
-      return q.n >= 1 && std::min(q.x0, x1) >= 0 && std::max(q.x0, x1) < xl && std::min(q.vb, v1) >= 0 &&
-             std::max(q.vb, v1) < vl;
-    };
-    const int l3max = pb.l3min + 2 * (pb.nl3 - 1);
+        w.push_back(make_float4(v[0], v[1], v[2], v[3]));
+      }
+    return q;
+  };
+  // the quads from m3 (a multiple of 4) up of orders sa .. sb - 1, each with the orders that reach
+  // it; returns their 3j values (float4)
+  auto run_of = [&](const PairBlock& pb, int m3, int sa, int sb, bool put) {
+    int len = 0, count = 0;
+    for (; m3 <= pb.l3min + 2 * (sb - 1); m3 += 4, ++count) {
+      const int least = m3 > 0 ? m3 : std::max(0, -(m3 + 3));  // least |m3| of the quad
+      int s0 = sa;
+      while (pb.l3min + 2 * s0 < least) ++s0;
+      LaneQuad q = quad_of(pb, m3, s0, sb, put);
+      q.wofs = len;
+      len += q.n * q.rs;
+      if (put) quads.push_back(q);
+    }
+    if (count > kLaneMaxQuads) bad = "lane tables: more quads than the kernel stages";
+    return len;
+  };
+  // general coefficients: m3 from -l3 of the run's largest order, rows of both signs
+  auto gen_run = [&](const PairBlock& pb, int sa, int sb, bool put) {
+    return run_of(pb, -((pb.l3min + 2 * (sb - 1) + 3) / 4) * 4, sa, sb, put);
+  };
+  auto gen_rows = [&](const PairBlock& pb, int sa, int sb) {
+    int r = 0;
+    for (int s = sa; s < sb; ++s) r += 2 * (pb.l3min + 2 * s) + 1;
+    return r;
+  };
+  for (const PairBlock& pb : pbs) {
+    LaneBlock fb{};
+    fb.l1 = pb.l1; fb.l2 = pb.l2; fb.l3min = pb.l3min; fb.nl3 = pb.nl3; fb.lt_base = pb.lt_base;
+    fb.c1 = coff[pb.l1 >> 1]; fb.c2 = coff[pb.l2 >> 1];
+    fb.swap = pb.l1 > pb.l2;
     fb.q0 = (int)quads.size();
     fb.w0 = (int)w.size();
-    int run = 0, rows = 0;
-    for (int m3 = 0; m3 <= l3max; m3 += 4) {
-      int s0 = 0;
-      while (pb.l3min + 2 * s0 < m3) ++s0;
-      const int len = add(m3, s0, pb.nl3);
-      quads.back().wofs = run;
-      run += len;
-      if (!fits(quads.back())) return "lane tables: a quad leaves the staged rows";
-    }
+    fb.wn = run_of(pb, 0, 0, pb.nl3, true);
     fb.nq = (int)quads.size() - fb.q0;
-    fb.wn = run;
-    wmax = std::max(wmax, run);
-    if (fb.nq > kLaneMaxQuads) return "lane tables: more quads than the kernel stages";
-    for (int s = 0; s < 16; ++s) {
+    blks.push_back(fb);
+    crows = std::max(crows, 2 * std::max(pb.l1, pb.l2) + 7);
+    wmax = std::max(wmax, fb.wn);
+    int rows = 0;
+    for (int s = 0; s < pb.nl3; ++s) {
+      rows += pb.l3min + 2 * s + 1;
+      wmax = std::max(wmax, gen_run(pb, s, s + 1, false));
+      c3rows = std::max(c3rows, gen_rows(pb, s, s + 1));
+    }
+    c3rows = std::max(c3rows, rows);
+  }
+  // general coefficients: as few balanced runs of up to kLaneNC orders as fit the shared memory that
+  // real functions and single orders take, so that the warps of an SM stay as many
+  for (size_t i = 0; i < pbs.size(); ++i) {
+    const PairBlock& pb = pbs[i];
+    int gp = (pb.nl3 + kLaneNC - 1) / kLaneNC;
+    auto fits = [&] {
+      for (int r = 0; r < gp; ++r) {
+        int s0, n;
+        lane_run(pb.nl3, gp, r, s0, n);
+        if (gen_rows(pb, s0, s0 + n) > c3rows || gen_run(pb, s0, s0 + n, false) > wmax) return false;
+      }
+      return true;
+    };
+    while (!fits()) ++gp;
+    blks[i].gp = gp;
+    for (int r = 0; r < 16; ++r) {
       int4 g = make_int4((int)quads.size(), 0, (int)w.size(), 0);
-      if (s < pb.nl3) {
-        const int l3 = pb.l3min + 2 * s;
-        int r = 0;
-        for (int m3 = -((l3 + 3) / 4) * 4; m3 <= l3; m3 += 4) {
-          const int len = add(m3, s, s + 1);
-          quads.back().wofs = r;
-          r += len;
-          if (!fits(quads.back())) return "lane tables: a quad leaves the staged rows";
-          ++g.y;
-        }
-        g.w = r;
-        wmax = std::max(wmax, r);
-        if (g.y > kLaneMaxQuads) return "lane tables: more quads than the kernel stages";
-        rows += l3 + 1;
-        c3rows = std::max(c3rows, 2 * l3 + 1);
+      if (r < gp) {
+        int s0, n;
+        lane_run(pb.nl3, gp, r, s0, n);
+        g.w = gen_run(pb, s0, s0 + n, true);
+        g.y = (int)quads.size() - g.x;
       }
       gcols.push_back(g);
     }
-    c3rows = std::max(c3rows, rows);
-    crows = std::max(crows, 2 * b + 7);
-    blks.push_back(fb);
   }
-  return "";
+  return bad;
 }
 
 // Units of every K' <= K: (offset in utab, units) in kofs[K'], 34 entries a unit: per lane
