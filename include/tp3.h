@@ -483,6 +483,10 @@ int tp3_mlp_train_step(tp3_mlp* net, int rows, const void* d_x, const float* d_v
  * TP3_ERR_TIMEOUT and returns, and the next synchronising call on the context
  * (tp3_sync, tp3_energy*, ...) reports TP3_ERR_TIMEOUT; the context stays usable. */
 int tp3_selftest_timeout(tp3_ctx* ctx, long long cycles);
+/* The scoring kernels' own scalar functions on n host values: op 0 the logarithm of the
+ * energies' sum (double -> double), 1 their float -> double and 2 the gather's double ->
+ * float conversion.  Synchronises. */
+int tp3_selftest_scalar(tp3_ctx* ctx, int op, int n, const void* in, void* out);
 
 /* ---- per-launch timing of the stages ------------------------------------- */
 /* When enabled, CUDA events bracket each launch of the angular + Bayes kernel and

@@ -38,6 +38,7 @@
 
 #include "../../include/tp3.h"
 #include "internal.h"
+#include "scalar.cuh"
 #include "tables.h"
 #include "tc_prims.cuh"
 
@@ -498,20 +499,6 @@ __global__ void __launch_bounds__(32 * kLaneMaxWarps, 1) k_couple_lane(
     passes(std::true_type());
   else
     passes(std::false_type());
-}
-
-// (float)x by integer arithmetic: FP64 conversions, like all FP64 arithmetic, run at a few
-// lanes per clock and SM.  Round to nearest even; subnormal and non-finite results go through
-// the conversion.
-__device__ __forceinline__ float narrow(const double x) {
-  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
-  const int e = (int)((hi >> 20) & 0x7ff) - 1023 + 127;
-  if (e >= 1 && e <= 254) {
-    const uint32_t m = ((hi & 0xfffff) << 3) | (lo >> 29), rem = lo & 0x1fffffff;
-    const uint32_t up = rem > 0x10000000u || (rem == 0x10000000u && (m & 1)) ? 1u : 0u;
-    return __uint_as_float((hi & 0x80000000u) | (((uint32_t)e << 23) + m + up));
-  }
-  return ((hi << 1) | lo) == 0 ? __uint_as_float(hi & 0x80000000u) : (float)x;
 }
 
 __device__ __forceinline__ double flip(const double x, bool neg) {

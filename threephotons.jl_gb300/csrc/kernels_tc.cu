@@ -30,6 +30,7 @@
 
 #include "../../include/tp3.h"
 #include "internal.h"
+#include "scalar.cuh"
 #include "tc_prims.cuh"
 
 namespace tp3 {
@@ -1051,38 +1052,6 @@ __global__ void __launch_bounds__(256) k_finalize_slabs(const double* __restrict
     __syncthreads();
   }
   if (threadIdx.x == 0) E[prop] = ss[0] + sc[0];
-}
-
-// log(x) of a positive normal double, table-driven (P. T. P. Tang, "Table-driven implementation
-// of the logarithm function in IEEE floating-point arithmetic", ACM TOMS 16 (1990)): x = 2^e m
-// with 0.75 <= m < 1.5, c the centre of m's interval (1/128 of its binade), r = m (1/c) - 1 with
-// one rounding, log x = e ln 2 + log c + log1p(r), |r| < 2^-8.  14 FP64 operations, a third of log(): FP64 runs at two lanes per
-// clock and SM here.  tab: 1/c and log c, built in extended precision.
-__device__ __forceinline__ double slab_log(const double x, const SlabLog* __restrict__ tab) {
-  const int hi = __double2hiint(x);
-  const int e = ((hi >> 20) & 0x7ff) - 1023;
-  if (e < -1022 || e > 1023 || hi < 0) return log(x);  // zero, subnormal, infinite, NaN, negative
-  const double m = __hiloint2double((hi & 0xfffff) | 0x3ff00000, __double2loint(x));
-  const int i = (hi >> 13) & 127;
-  const double inv = tab[i].inv, chi = tab[i].hi, clo = tab[i].lo;
-  const double r = fma(m, inv, -1.0), r2 = r * r;
-  double p = fma(r, 1.0 / 7.0, -1.0 / 6.0);
-  p = fma(p, r, 0.2);
-  p = fma(p, r, -0.25);
-  p = fma(p, r, 1.0 / 3.0);
-  p = fma(p, r, -0.5);
-  const double ed = (double)(e + (i >> 6));
-  constexpr double ln2_hi = 0x1.62e42fefa38p-1, ln2_lo = 0x1.ef35793c7673p-45;  // ln 2 to 41 + 53 bits
-  return fma(ed, ln2_hi, chi) + (r + fma(p, r2, fma(ed, ln2_lo, clo)));  // the first sum is exact
-}
-
-// (double)x by integer arithmetic (exact); zeros, subnormals and non-finite values go through
-// the conversion, which runs at FP64 rate.
-__device__ __forceinline__ double widen(const float x) {
-  const uint32_t u = __float_as_uint(x);
-  const uint32_t e = (u >> 23) & 255;
-  if (e == 0 || e == 255) return (double)x;
-  return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + (896u << 20))), (int)(u << 29));
 }
 
 // Energies from the persistent kernel's partial sums [klp][nhalf][2][2] per proposal: slab terms

@@ -116,6 +116,7 @@ SIGNATURES = {
     "tp3_mlp_train_step": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, ctypes.c_float,
                                    P(c_double)]),
     "tp3_selftest_timeout": (c_int, [c_void_p, ctypes.c_longlong]),
+    "tp3_selftest_scalar": (c_int, [c_void_p, c_int, c_int, c_void_p, c_void_p]),
     "tp3_profile_enable": (c_int, [c_void_p, c_int]),
     "tp3_profile_read": (c_int, [c_void_p, P(c_int64), P(c_double)]),
     "tp3_profile_read_stage": (c_int, [c_void_p, c_int, P(c_int64), P(c_double)]),
