@@ -126,6 +126,8 @@ int tp3_get_mode(const tp3_ctx* ctx, int* mode);
 int tp3_autotune(tp3_ctx* ctx, int n, double* report, int* nreport);
 /* Force a coupling form of the tensor-core path (0 to 9 as above). */
 int tp3_set_coupling(tp3_ctx* ctx, int form);
+/* The coupling form that the tensor-core modes of this context use now. */
+int tp3_get_coupling(const tp3_ctx* ctx, int* form);
 /* Angular-stage schedule of the tensor-core path (no reference counterpart).
  * TP3_ANGULAR_PERSISTENT (default): one CTA per SM walks (proposal, 128-triple tile,
  * grid half) units with two TMEM accumulators, so the Bayes epilogue of one unit

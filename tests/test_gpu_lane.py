@@ -209,3 +209,24 @@ def test_runs_of_orders_equal_the_pair_form(L, K, n):
     for x, y in zip(got[PAIR], got[LANE]):
         assert np.isfinite(x).all() and np.array_equal(x, y)
     b.close()
+
+
+def test_form_in_use():
+    """The lane-owned form is what a context starts with unless its shared memory does not fit (more
+    than 64 shells); a forced form is the one reported."""
+    b = tp3.calculate_basis(8, 10, 6, 8)
+    assert b.coupling == LANE
+    b.set_coupling(PAIR)
+    assert b.coupling == PAIR
+    for form in range(1, 10):
+        try:
+            b.set_coupling(form)
+        except tp3.TP3Error:
+            continue
+        assert b.coupling == form
+    b.close()
+    b = tp3.calculate_basis(8, 9, 4, 70)
+    assert b.coupling != LANE
+    with pytest.raises(tp3.TP3Error):
+        b.set_coupling(LANE)
+    b.close()

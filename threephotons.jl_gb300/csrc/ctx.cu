@@ -1258,6 +1258,14 @@ int tp3_set_coupling(tp3_ctx* c, int form) {
   return TP3_OK;
 }
 
+int tp3_get_coupling(const tp3_ctx* c, int* form) {
+  if (!c || !form || !c->tc_ok) return TP3_ERR_ARG;
+  const TcTables& tc = c->tc;  // in the order in which the launches look at them
+  *form = tc.use_lane ? 9 : tc.split ? 1 : tc.use_fold >= 0 ? 5 + tc.use_fold : tc.use_warp2 ? 4 : tc.use_warp ? 3
+          : tc.use_small ? 2 : 0;
+  return TP3_OK;
+}
+
 int tp3_set_angular(tp3_ctx* c, int schedule) {
   if (int r = check_ctx(c)) return r;
   if (schedule != TP3_ANGULAR_TILE && schedule != TP3_ANGULAR_PERSISTENT)

@@ -58,6 +58,7 @@ SIGNATURES = {
     "tp3_reserve": (c_int, [c_void_p, c_int]),
     "tp3_autotune": (c_int, [c_void_p, c_int, c_void_p, P(c_int)]),
     "tp3_set_coupling": (c_int, [c_void_p, c_int]),
+    "tp3_get_coupling": (c_int, [c_void_p, P(c_int)]),
     "tp3_set_angular": (c_int, [c_void_p, c_int]),
     "tp3_set_host_input": (c_int, [c_void_p, c_int]),
     "tp3_retrieve_solution": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_double,

@@ -155,6 +155,13 @@ class BasisTypeGB300:
         default where it fits)."""
         check(self._lib.tp3_set_coupling(self._ctx, form), self._ctx)
 
+    @property
+    def coupling(self) -> int:
+        """The coupling form that the tensor-core modes use now (numbers as for set_coupling)."""
+        f = ctypes.c_int()
+        check(self._lib.tp3_get_coupling(self._ctx, ctypes.byref(f)), self._ctx)
+        return f.value
+
     def autotune(self, n: int = 64) -> list:
         """Time every evaluation variant on n synthetic proposals, keep the fastest (also
         for later TP3_MODE_AUTO contexts of this shape); returns
