@@ -20,3 +20,14 @@ def test_every_included_file_is_a_dependency():
         with open(path) as f:
             todo += [os.path.join(os.path.dirname(path), i) for i in re.findall(r'#include "([^"]+)"', f.read())]
     assert seen <= deps, sorted(seen - deps)
+
+
+def test_debug_build_checks_the_scoring_path():
+    """The kernels of a batch's scoring whose indices come from tables check them in a TP3_DEBUG build."""
+    for file, functions in {"kernels_lane.cu": ("lane_task", "k_couple_lane", "k_gather_lane"),
+                            "kernels_hform.cu": ("k_build_H_pairs",), "kernels_tc.cu": ("k_gather_sym",),
+                            "kernels_fold.cu": ("k_couple_fold",)}.items():
+        with open(os.path.join(PKG, "csrc", file)) as f:
+            bodies = re.split(r"^}", f.read(), flags=re.M)  # functions end at the margin
+        for name in functions:
+            assert any("TP3_DCHECK" in b for b in bodies if re.search(r"\b" + name + r"\([^;{]*\{", b)), name

@@ -12,8 +12,8 @@ namespace tp3 {
 struct Wigner3jTable;  // tables.h
 
 // TP3_DEBUG builds (TP3_DEBUG=1 python threephotons.jl_gb300/build.py --force) check the
-// indices that the gather and folded-row coupling kernels compute before each shared- or
-// global-memory access; a failed check sets TP3_ERR_BOUNDS in the context's error flag
+// indices that the gather kernels, the lane-owned and folded-row couplings and the lambda != 0
+// operand compute before each shared- or global-memory access; a failed check sets TP3_ERR_BOUNDS in the context's error flag
 // (reported by the next synchronising call) and skips the access.  Release builds
 // compile the checks out.
 #ifdef TP3_DEBUG

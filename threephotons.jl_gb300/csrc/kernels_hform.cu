@@ -54,7 +54,8 @@ __global__ void __launch_bounds__(kHfThreads, 1) k_build_H_pairs(
     const float* __restrict__ T32, int klp, int64_t Tstride, int n, int klength, int n_lt,
     const float* __restrict__ Ytab, int nc, int L, const int4* __restrict__ kl, const int2* __restrict__ lists,
     const int2* __restrict__ entries, const float4* __restrict__ wts, const int4* __restrict__ quad_m,
-    const int* __restrict__ quad_q, int nunits, int KP, int tf32, void* __restrict__ Hhi, void* __restrict__ Hlo) {
+    const int* __restrict__ quad_q, int nunits, int KP, int tf32, void* __restrict__ Hhi, void* __restrict__ Hlo,
+    int* __restrict__ err) {
   extern __shared__ __align__(16) float hf_smem[];
   __shared__ int next;
   const int ncp = nc + 2 * L;                   // L zeros on each side: a pair with |m| > l reads them
@@ -102,6 +103,21 @@ __global__ void __launch_bounds__(kHfThreads, 1) k_build_H_pairs(
 #pragma unroll
       for (int p = 0; p < NP / 2; ++p) acc[s][p] = make_float2(0.f, 0.f);
     auto term = [&](const int2 en, const float4 w) {
+#ifdef TP3_DEBUG
+      {  // the l-triple and the quad's three Legendre rows
+        const int4 m = *mq;
+        const uint32_t y = (uint32_t)__cvta_generic_to_shared(Ys), end = 48u * ncp;
+        bool ok = en.x >= 0 && (en.x >> 4) < n_lt;
+        const int ms[4] = {m.x, m.y, m.z, m.w};
+        for (int s = 0; s < 4; ++s) {
+          const int m2 = (short)ms[s], m3 = ms[s] >> 16;
+          ok = ok && Yu + ((en.y & 1023) << 4) - m2 - m3 - y < 16u * ncp &&
+               Yu + 16 * ncp + ((en.y >> 6) & (1023 << 4)) + m2 - y < 32u * ncp &&
+               Yu + 32 * ncp + ((en.y >> 16) & (1023 << 4)) + m3 - y < end;
+        }
+        if (!TP3_DCHECK(ok, err)) return;
+      }
+#endif
       if (en.y < 0) {  // another l2
         const int4 m = *mq;
         const uint32_t b = Yu + 16 * ncp + ((en.y >> 6) & (1023 << 4));
@@ -167,7 +183,7 @@ __global__ void __launch_bounds__(kHfThreads, 1) k_build_H_pairs(
       const float a0 = p & 1 ? acc[0][p >> 1].y : acc[0][p >> 1].x;
       const float b0 = __shfl_down_sync(0xffffffffu, a0, 4);
       if (unit == 0 && pos == 0) v[0] = b0 + a0;
-      if (q < 0 || ki0 + u >= klength || p0 + p >= n) continue;
+      if (q < 0 || ki0 + u >= klength || p0 + p >= n || !TP3_DCHECK(q + 3 < KP, err)) continue;
       const size_t o = ((size_t)(p0 + p) * klp + ki0 + u) * KP + q;
       if (tf32) {
         float h[4], l[4];
@@ -347,7 +363,7 @@ cudaError_t launch_build_H_pairs(const DevTables& t, const TcTables& tc, int n, 
     return launch_after(
         kernel, dim3((t.klength + 3) / 4, (n + np - 1) / np), threads, smem, s, 1, T32, t.klp, (int64_t)t.klp * t.n_ltp, n, t.klength, t.n_lt, t.Ytab, t.nc, h.L, t.kl, h.lists, h.entries,
         reinterpret_cast<const float4*>(h.wts), reinterpret_cast<const int4*>(h.quad_m), h.quad_q, h.nunits, tc.KP,
-        tf32 ? 1 : 0, Hhi, Hlo);
+        tf32 ? 1 : 0, Hhi, Hlo, tc.err);
   };
   switch (np) {
     case 12: return go(k_build_H_pairs<12>);

@@ -83,6 +83,12 @@ struct LaneView {
   uint32_t C3;        // c_k3 rows: (re x 4, im x 4) per quad of shells
   const LaneQuad* quads;
   int nq;
+#ifdef TP3_DEBUG
+  // what is staged: rows of X and V and of C3, 3j values (float4, from 8 before W on); C3 of block 0
+  int xrows, vrows, wlen, c3rows;
+  uint32_t c3first;
+  int* err;
+#endif
 };
 
 // One step of phase 1: the products of x with the window rows of the quad's four m3, each into
@@ -211,6 +217,15 @@ __device__ __forceinline__ void lane_task(const LaneView& V, bool swap, int l3mi
       const LaneQuad q = V.quads[qi];
       if (q.c0 >= s_hi) continue;
       m = q.m3;
+#ifdef TP3_DEBUG
+      {  // the first and last rows of either operand and 3j values
+        const int sx = swap ? -1 : 1, x1 = q.x0 + sx * (q.n - 1), v1 = q.vb - sx * (q.n + 2);
+        const int w0 = q.wofs + s_hi - NC - q.c0;
+        const bool ok = min(q.x0, x1) >= 0 && max(q.x0, x1) < V.xrows && min(q.vb, v1) >= 0 &&
+                        max(q.vb, v1) < V.vrows && w0 >= -8 && w0 + (q.n - 1) * q.rs + NC <= V.wlen && k1 < PS && k2 < PS;
+        if (!TP3_DCHECK(ok, V.err)) continue;
+      }
+#endif
       // all NC columns; those outside the task or below the quad's orders are not used
       const uint32_t x = xk + 8 * PS * q.x0, v = vk + 8 * PS * q.vb, wt = V.W + 16 * (q.wofs + s_hi - NC - q.c0);
       if (swap)
@@ -240,6 +255,17 @@ __device__ __forceinline__ void lane_task(const LaneView& V, bool swap, int l3mi
         }
       }
     }
+#ifdef TP3_DEBUG
+    {  // the c_k3 rows of the m3 that count
+      bool ok = true;
+      for (int k = 0; k < 4; ++k)
+        for (int c = 0; c < NC; ++c) {
+          const int t = (SYM ? m + k : abs(m + k)) - m_lo, at = (int)(row[c] - V.c3first) + k * CR;
+          if ((unsigned)t < (unsigned)cnt[c]) ok = ok && at >= 0 && at + 32 * (wide ? 4 : 2) <= V.c3rows * CR;
+        }
+      if (!TP3_DCHECK(ok, V.err)) break;
+    }
+#endif
     // phase 2, two m3 at a time
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
@@ -290,6 +316,12 @@ __device__ __forceinline__ void lane_task(const LaneView& V, bool swap, int l3mi
           lrow[at + 1] = l.y;
         }
       };
+#ifdef TP3_DEBUG
+      bool rows_ok = lt < o.KP;
+      for (int i = lane; i < nslot; i += 32)
+        rows_ok = rows_ok && ((slots[i] & 3) == 0 || (int)(slots[i] >> 2) * 2 + ((slots[i] & 2) ? 1 : 0) < o.klp);
+      if (!TP3_DCHECK(__all_sync(0xffffffffu, rows_ok), V.err)) break;
+#endif
       const float2* st = reinterpret_cast<const float2*>(stage);
 #pragma unroll 1
       for (int i = lane; i < nslot; i += 64) {
@@ -307,6 +339,7 @@ __device__ __forceinline__ void lane_task(const LaneView& V, bool swap, int l3mi
         if (!((sl >> (i & 1)) & 1)) continue;
         const int ki = 2 * (int)(sl >> 2) + (i & 1);
         const float t = stage[i];
+        if (!TP3_DCHECK(ki < o.klp && lt < (o.T32 && !o.t32maj ? o.ldT32 : o.KP), V.err)) continue;
         if (o.hi && !o.ltmaj) {
           const size_t at = (size_t)ki * o.KP + lt;
           if (o.tf32) {
@@ -424,7 +457,19 @@ __global__ void __launch_bounds__(32 * kLaneMaxWarps, 1) k_couple_lane(
   }
   if (threadIdx.x < 17) s_next[threadIdx.x] = 0;
   __syncthreads();
+#ifdef TP3_DEBUG
+  if (!TP3_DCHECK(n1r + 6 <= crows && n2r + 6 <= crows && fb.c1 + n1r <= nc && fb.c2 + n2r <= nc &&
+                      fb.lt_base + fb.nl3 <= out.KP && fb.gp <= 16 && Kp <= K,
+                  err))
+    return;
+#endif
   LaneView V;
+#ifdef TP3_DEBUG
+  V.xrows = 6 + (fb.swap ? n2r : n1r);
+  V.vrows = 6 + (fb.swap ? n1r : n2r);
+  V.c3first = smem_u32(C3);
+  V.err = err;
+#endif
   V.X = smem_u32(fb.swap ? C2 : C1);
   V.V = smem_u32(fb.swap ? C1 : C2);
   V.W = smem_u32(W);
@@ -442,6 +487,17 @@ __global__ void __launch_bounds__(32 * kLaneMaxWarps, 1) k_couple_lane(
         g = gcols[blk * 16 + pass];
         lane_run(fb.nl3, fb.gp, pass, p_lo, p_w);
       }
+#ifdef TP3_DEBUG
+      V.wlen = g.w;
+      V.c3rows = 0;
+      bool in_layout = g.w <= wmax && g.y <= kLaneMaxQuads;
+      for (int s = p_lo; s < p_lo + p_w; ++s) {
+        const int l3 = fb.l3min + 2 * s;
+        V.c3rows += SYM ? l3 + 1 : 2 * l3 + 1;
+        in_layout = in_layout && coff[l3 >> 1] + 2 * l3 + 1 <= nc;
+      }
+      if (!TP3_DCHECK(in_layout && V.c3rows <= c3rows, err)) return;
+#endif
       if (pass > pass0) {
         __syncthreads();  // the previous orders' reads are done
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -488,6 +544,10 @@ __global__ void __launch_bounds__(32 * kLaneMaxWarps, 1) k_couple_lane(
         const uint32_t e = utab[ko.x + u * 34 + lane];  // the lane's shell pair, see build_lane_units
         const uint32_t s0 = utab[ko.x + u * 34 + 32], s1 = utab[ko.x + u * 34 + 33];
         V.C3 = smem_u32(C3 + 8 * (s1 >> 17));
+        if (!TP3_DCHECK((int)(e >> 24) + ((int)(e >> 12) & 0xfff) <= stage_len && 2 * (int)(s1 & 0xffff) <= stage_len &&
+                            (int)(s1 >> 17) * 8 < c3row,
+                        err))
+          break;
         lane_task<SYM, kLaneNC, PS, 8 * PS>(V, fb.swap, fb.l3min, s_lo, w, fb.lt_base, (s1 >> 16) & 1, (int)e & 63,
                                             (int)(e >> 6) & 63, (int)(e >> 24), (int)(e >> 12) & 0xfff, (int)(s1 & 0xffff),
                                             stage, slots + s0, out);
@@ -520,7 +580,8 @@ template <int ROUNDS>
 __global__ void __cluster_dims__(kGatherCtas, 1, 1) __launch_bounds__(256)
     k_gather_lane(int K, int nc, int ncoef, const int* __restrict__ csean, const int* __restrict__ cm,
                   const int* __restrict__ cmir, const int* __restrict__ cl, const double2* __restrict__ coeff,
-                  float2* __restrict__ ct, float* __restrict__ c3p, int* __restrict__ sym, const RagInfo* __restrict__ rag) {
+                  float2* __restrict__ ct, float* __restrict__ c3p, int* __restrict__ sym, const RagInfo* __restrict__ rag,
+                  int* __restrict__ err) {
   cluster_started_arrive();
   grid_release();
   extern __shared__ __align__(16) double2 gl_smem[];
@@ -530,6 +591,14 @@ __global__ void __cluster_dims__(kGatherCtas, 1, 1) __launch_bounds__(256)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ld = nc | 1;
   const double2* cp = coeff + (size_t)prop * K * ncoef;
+#ifdef TP3_DEBUG
+  {  // the coefficient maps stay inside a shell's coefficients and the compact layout
+    int maps_ok = K <= ps;
+    for (int c = threadIdx.x; c < nc; c += 256)
+      maps_ok &= csean[c] >= 0 && csean[c] < ncoef && cmir[c] >= 0 && cmir[c] < nc;
+    if (!TP3_DCHECK(__syncthreads_and(maps_ok) != 0, err)) K = 0;  // nothing is read, zeros are written
+  }
+#endif
   for (int rd = 0; rd < ROUNDS; ++rd) {
     const int k0 = 4 * (rank + kGatherCtas * rd), nk = min(4, K - k0);
 #pragma unroll 4
@@ -870,7 +939,7 @@ cudaError_t launch_gather_lane(const DevTables& t, const TcTables& tc, int n, co
   const size_t row = (size_t)(t.nc | 1) * sizeof(double2);
   auto go = [&](auto kernel, int rounds) {
     kernel<<<dim3(kGatherCtas, n), 256, 4 * rounds * row, s>>>(t.K, t.nc, lay.stride, lay.map, tc.cm, tc.cmir, tc.cl, coeff,
-                                                               ct, c3p, sym, rag);
+                                                               ct, c3p, sym, rag, tc.err);
   };
   if (tc.lane.ps == 32)
     go(k_gather_lane<1>, 1);
