@@ -893,6 +893,11 @@ int tp3_ctx_create(int L, int LMAX, int N, int K, double lambda, double dq, tp3_
   }
   tp3::fold_grid(b, true);
   // host-side invariants of every table before upload
+  for (int u = 0; u < b.Gu; ++u)
+    if (b.u_to_g[u] != u) {  // the c3 output's index arithmetic
+      delete c;
+      return fail(nullptr, TP3_ERR_TABLE, "unique grid points are not the first ones");
+    }
   for (int t = 0; t < b.n_lt(); ++t) {
     if (b.lt_jstart[t] < 0 || b.lt_jstart[t] + b.lt_jcount[t] > b.basislen()) {
       delete c;
@@ -1002,8 +1007,7 @@ int tp3_ctx_create(int L, int LMAX, int N, int K, double lambda, double dq, tp3_
       (e = upload(c, w32, &t.w)) != cudaSuccess ||
       (e = upload(c, idx, &t.idx)) != cudaSuccess || (e = upload(c, lt, &t.lt)) != cudaSuccess ||
       (e = upload(c, kl, &t.kl)) != cudaSuccess || (e = upload(c, b.tf, &t.tf)) != cudaSuccess ||
-      (e = upload(c, Ffull, &t.Ffull)) != cudaSuccess || (e = upload(c, b.u_to_g, &t.u_to_g)) != cudaSuccess ||
-      (e = upload(c, b.g_to_u, &t.g_to_u)) != cudaSuccess || (e = tp3::plain_configure()) != cudaSuccess ||
+      (e = upload(c, Ffull, &t.Ffull)) != cudaSuccess || (e = tp3::plain_configure()) != cudaSuccess ||
       (e = upload(c, Ytab, &t.Ytab)) != cudaSuccess || (e = upload(c, lt_of_j, &t.lt_of_j)) != cudaSuccess ||
       (e = upload(c, qstart, &t.qstart)) != cudaSuccess || (e = upload(c, qlist, &t.qlist)) != cudaSuccess ||
       (e = upload(c, qent, &t.qent)) != cudaSuccess ||

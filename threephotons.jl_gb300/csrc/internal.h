@@ -40,7 +40,6 @@ struct DevTables {
   const int4* kl;       // [klength] (k1, k2, k3, tf)
   const double* tf;     // [klength]
   const float* Ffull;   // [G][n_ltp]  fp32, full grid (plain path)
-  const int* u_to_g;    // [Gu]
   // lambda != 0 (shell-dependent Legendre factors): Fourier-pair form of the angular stage
   int nq = 0, nqp = 0;       // (m2, m3) pairs up to sign, padded to 16 (0 at lambda = 0)
   const float* Ytab = nullptr;   // [K][nc] sphPlm(l, m, theta_k)
@@ -49,7 +48,6 @@ struct DevTables {
   const int* qlist = nullptr;    // [basislen] basis entries grouped by pair
   const int4* qent = nullptr;    // [basislen] in qlist order: packed indices, w (float bits), l-triple
   const float* Cq = nullptr;     // [G][nqp] cos(m2 alpha + m3 beta)
-  const int* g_to_u;    // [G]
 };
 
 // Plain path launches (kernels_plain.cu).

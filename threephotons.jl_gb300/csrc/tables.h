@@ -65,7 +65,7 @@ struct Basis {
   int G = 0;          // 2 N^2 full grid points, g = a + N*b
   int Gu = 0;         // unique points actually evaluated
   int mult = 1;       // orbit size of each unique point (4 when folded, else 1)
-  std::vector<int> u_to_g;        // [Gu] representative full-grid index
+  std::vector<int> u_to_g;        // [Gu] representative full-grid index: u itself, the c3 output relies on it
   std::vector<int> g_to_u;        // [G]
 };
 
