@@ -71,21 +71,19 @@ DTYPES = {0: "fp32", 1: "bf16x3 (fp32 accumulate)", 2: "tf32x3 (fp32 accumulate)
 STAGE_TRAFFIC = {
     ("tc_bf16x3", "folded_7w", "tile"): {"coupling": (154.2e6 / 32, 0.0), "angular": (230.2e6 / 32, 0.0),
                                  "source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one 32-proposal "
-                                           "launch, scaled in proportion to the proposals "
-                                           "(profiles/traffic_L18K26N32_b32_folded7w.md)"},
+                                           "launch, scaled in proportion to the proposals"},
     ("tc_bf16x3", "folded_13w", "persistent"): {
         "coupling": (155.9e6 / 32, 0.0), "angular": (230.8e6 / 32, 0.0),
         "source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one 32-proposal launch of each stage, "
-                  "scaled in proportion to the proposals (profiles/traffic_L18K26N32_b32_folded13w.md)"},
+                  "scaled in proportion to the proposals"},
     ("tc_bf16x3", "lane", "persistent"): {
         "coupling": (274.6e6 / 32, 0.0), "angular": (229.1e6 / 32, 0.0),
         "source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one 32-proposal launch of each stage, "
-                  "scaled in proportion to the proposals (profiles/traffic_L18K26N32_b32_lane.md)"},
+                  "scaled in proportion to the proposals"},
     ("tc_bf16x3", "folded_7w", "persistent"): {
         "coupling": (154.2e6 / 32, 0.0), "angular": (231.1e6 / 32, 0.0),
         "source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one 32-proposal launch of each stage, "
-                  "scaled in proportion to the proposals (profiles/traffic_L18K26N32_b32_folded7w.md, "
-                  "profiles/k_angular_tp_L18K26N32_b32.md)"},
+                  "scaled in proportion to the proposals"},
 }
 
 
@@ -702,11 +700,23 @@ def main():
             raise SystemExit("l-triple count differs from the basis")
         S = sum(2 * c + 1 for _, _, c in trip)
         W_a = 10.0 * (K * (K + 1) / 2) * basis.basislen + 4.0 * S * klength
+        # what a real function's proposal needs of it (m3 >= 0): a complex product per (m1, m3) of an
+        # (l1, l2) block, its two FMAs per order l3 >= m3, and two per (l-triple, m3) and shell triple
+        prod = sums = third = 0
+        for l1, l2 in sorted({(a, b) for a, b, _ in trip}):
+            orders = [c for a, b, c in trip if (a, b) == (l1, l2)]
+            third += sum(c + 1 for c in orders)
+            for m3 in range(max(orders) + 1):
+                n1 = max(0, min(l1, l2 - m3) - max(-l1, -l2 - m3) + 1)
+                prod += n1
+                sums += n1 * sum(c >= m3 for c in orders)
+        W_r = K * (K + 1) / 2 * (8.0 * prod + 4.0 * sums) + klength * 4.0 * third
         ms_c = ms_prof_c / n_prof_c
         fp32_peak = basis.measure_fp32_peak()
         ach_c = W_a * B / (ms_c / 1e3) / 1e12
         stages = {"coupling": {"bound": "fp32", "kernel": f"coupling ({cform or 'default form'})",
                                "ms_per_launch": ms_c, "algorithmic_flop_per_proposal": W_a, "achieved": ach_c,
+                               "real_function_flop_per_proposal": W_r, "real_function_frac": ach_c / fp32_peak * W_r / W_a,
                                "peak": fp32_peak, "frac": ach_c / fp32_peak, "unit": "TFLOP/s",
                                "peak_source": "measured FFMA (tp3_measure_fp32_peak, this run)",
                                "traffic": traffic_c},
@@ -725,7 +735,9 @@ def main():
                     "algorithmic_flop_per_proposal": st["algorithmic_flop_per_proposal"],
                     "share_of_step": st["ms_per_launch"] / ms_per_step,
                     "note": "the coupling runs on the FP32 FMA pipes (MEASURED_PEAKS.json has no FP32 figure, so "
-                            "its peak is measured in this run); the tensor-core stage is stages.angular"}
+                            "its peak is measured in this run); its count takes no symmetry of the coefficients into "
+                            "account, what these proposals (a real function's) need is stages.coupling."
+                            "real_function_frac of the peak; the tensor-core stage is stages.angular"}
 
     # device-resident annealing chains: 64 chains x 16 speculative candidates per graph replay
     chains_info = None
