@@ -181,7 +181,9 @@ int tp3_energy_batch_device(tp3_ctx* ctx, int n, const void* d_coeffs, void* d_E
  * and K are the largest): orders l > L and shells k > K of a proposal are treated as
  * absent -- exactly the reference's c3 of basis (L, K), whose shell triples are the
  * first K(K+1)(K+2)/6 of the context's -- and each proposal is scored against its own
- * histogram of a set.  Tensor-core modes with the one-kernel coupling only. */
+ * histogram of a set.  Tensor-core modes at lambda = 0, at shapes that the one-kernel
+ * coupling fits or with a folded-row coupling selected; the lane-owned coupling scores
+ * them where it is the form in use. */
 /* Histogram set: nhist histograms (each as for tp3_set_histogram, with K3s[h] >= Ks[h]
  * shells stored and Ks[h] <= the context's K scored). */
 int tp3_set_histograms(tp3_ctx* ctx, int nhist, const double* const* c3refs, const int* K3s, const int* Ks);

@@ -658,7 +658,8 @@ int run_energy(tp3_ctx* c, int n, const double2* d_coeff, double* d_E, bool comp
     if (c->nhist == 0) return fail(c, TP3_ERR_NO_HISTOGRAM, "tp3_set_histograms has not been called");
     if (!is_tc(c->mode) || (!c->tc.fused_ok && c->tc.use_fold < 0) || c->tc.hform)
       return fail(c, TP3_ERR_UNSUPPORTED,
-                  "ragged batches need a tensor-core mode with the one-kernel coupling at lambda = 0");
+                  "ragged batches need a tensor-core mode at lambda = 0 and a shape that the one-kernel coupling "
+                  "fits (or a folded-row coupling selected)");
   } else if (!c->has_hist) {
     return fail(c, TP3_ERR_NO_HISTOGRAM, "tp3_set_histogram has not been called");
   }

@@ -220,7 +220,10 @@ size_t hf_smem_bytes(int np, int n_lt, int nc, int L, int nunits, int threads) {
   return ((size_t)n_lt * 4 * np + 12 * (size_t)(nc + 2 * L) + 32 * (size_t)nunits) * sizeof(float) + threads * 17;
 }
 
-// Proposals a CTA: the most of 12, 8, 4 that are needed and whose T fits.
+// Proposals a CTA: the most of 12, 8, 4 that are needed and whose T fits: the more share w Y1 Y2 Y3, the
+// better, up to a last pass that is mostly empty.  Whole calls at L = 18, K = 26, N = 16 by 12 / 8 / 4:
+// 784 / 958 / 1097 us for 12 proposals, 1424 / 1550 / 2070 for 24, 2003 / 1995 / 2727 for 32 and
+// 3895 / 3917 / 5353 for 64, but 1214 / 1044 / 1403 for 16 (as for 13 to 15), two passes either way.
 int hf_pick(int n_lt, int nc, int L, int nunits, int n) {
   for (int np = n > 8 ? 12 : n > 4 ? 8 : 4; np; np -= 4)
     if (hf_smem_bytes(np, n_lt, nc, L, nunits, kHfThreads) <= (size_t)kHfMaxSmem) return np;

@@ -17,11 +17,12 @@
 //     broadcasts (all lanes read the same four shells).
 // A warp needs no other warp, so warps take tasks from a counter, heaviest first.
 //
-// What bounds it: issue slots and the shared-memory port.  At L = 18, K = 26 a proposal is 11.8 M
-// warp instructions (the folded rows 15.5 M) at 65 % issue, 64 % of the port and 47 % of the FMA
-// pipe; 6.1 us of FMA pipe time on 152
-// SMs (phase 1 4.5, phase 2 1.5) in 14.8 us.  Only coefficients and 3j values are shared, 75 KB
-// a CTA with no D buffer, which lets 16 warps run with no barrier after the staging.
+// What bounds it: issue slots and the shared-memory port.  At L = 18, K = 26 a proposal of a real
+// function is 11.4 M warp instructions (the folded rows 15.5 M) in 14.5 us, 62 % of the issue slots
+// and 60 % of the port; 5.5 M of them go to the FMA pipe, where the operations it cannot do without
+// (m3 >= 0 and the pairs, orders and shells that exist) take 3.2 us on 152 SMs.  Only coefficients
+// and 3j values are shared, 80 KB a CTA with no D buffer, which lets 16 warps run with no barrier
+// after the staging.
 //
 // Every accumulation runs in the order of the one-kernel pair coupling (k_couple_pair), so
 // both give the same bits: m1 upwards in phase 1, m3 = 1 .. l3 then the doubled sum plus the
@@ -42,7 +43,6 @@
 #include "tables.h"
 #include "tc_prims.cuh"
 
-
 namespace tp3 {
 namespace {
 
@@ -50,7 +50,7 @@ namespace {
 // all, so 16 warps per SM.  All kLaneNC columns are always computed (columns outside the task
 // are not used): with a loop per column count, or more instances for more shells k3, the code
 // of an SM's warps left its instruction cache (29 of 34 stall cycles per issue with one
-// instance per width of k3).  64 proposals at L = 18, K = 26: 0.95 ms at 3 orders and 16 warps,
+// instance per width of k3).  64 proposals at L = 18, K = 26: 0.93 ms at 3 orders and 16 warps,
 // 1.02 at 4 and 12, 1.44 at 5 and 12 (spills), 1.30 at 5 with a loop per column count; the
 // one-kernel pair coupling takes 2.51 ms and the folded rows at 13 warps 1.58.
 constexpr int kLaneNC = 3;

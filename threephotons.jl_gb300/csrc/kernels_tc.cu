@@ -1061,7 +1061,8 @@ __global__ void __launch_bounds__(256) k_finalize_slabs(const double* __restrict
 // owns 256 / CTAS consecutive accumulators and their terms, CTA 0 gathers them through
 // distributed shared memory.  Bound by FP64 (two lanes per clock and SM), hence eight SMs for each
 // proposal of a small batch (at K = 26 one proposal took 6.5 + 15 us as a kernel of terms and a
-// kernel of one CTA that summed); a batch that fills the SMs by itself takes one CTA each.
+// kernel of one CTA that summed); a batch that fills the SMs by itself takes one CTA each (the line:
+// launch_finalize_parts).
 constexpr int kFinRows = 16;
 template <int CTAS>
 __global__ void __launch_bounds__(128)
@@ -1308,7 +1309,10 @@ cudaError_t launch_angular_persistent(const DevTables& t, const TcTables& tc, co
 
 cudaError_t launch_finalize_parts(const DevTables& t, const TcTables& tc, int n, const float* part, const double* Qs,
                                   double* E, cudaStream_t s, const RagInfo* rag) {
-  // eight SMs a proposal until the batch has about one proposal per SM
+  // Eight SMs a proposal until the batch holds one for every other SM.  Where the line is best depends
+  // on the terms of a proposal: whole calls by clusters / by single CTAs took 43.5 / 41.7 us for 64
+  // proposals and 45.6 / 42.9 for 76 at K = 8 (120 terms), 67 / 74 for 16 and 170 / 173 for 76 at
+  // K = 16 (816), 349 / 376 for 64, 411 / 435 for 76 and 1290 / 1298 for 256 at K = 26 (3276).
   auto go = [&](auto kernel, unsigned ctas) {
     return launch_after(kernel, dim3(ctas, n), 128, 0, s, ctas, part, t.klp, t.klength, tc.nhalf, Qs, t.tf, t.mult,
                         tc.logtab, E, rag);
